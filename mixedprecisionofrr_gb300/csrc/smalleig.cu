@@ -1,15 +1,411 @@
-// Small dense FP64 (generalized) symmetric eigenproblems on the device, one CTA per pencil.
+// Small dense FP64 (generalized) symmetric eigenproblems on the device.
 //
 // Replaces the host LAPACKE dsyev/dsygv wrappers of the reference (CPP/linalg/blas/mvops.cu:1601-1664)
 // and MATLAB eig(VAV, VV + tau I) inside eig_rr.m:50-54 / svd_rr.m:58-77.
-// Algorithm: Cholesky M = L L' (right-looking), C = L^-1 G L^-T (two forward substitutions, one
-// thread per right-hand side), cyclic Jacobi on C with round-robin parallel ordering (n/2 disjoint
-// rotations per round, Golub & Van Loan sym.Schur2 rotation), eigenvalue sort, U = L^-T W.
-// Everything stays in shared memory when 3 n^2 doubles fit, otherwise in a global workspace.
+// Algorithm: Cholesky M = L L' (right-looking), C = L^-1 G L^-T (two forward substitutions), cyclic
+// Jacobi on C with round-robin parallel ordering (n/2 disjoint rotations per round, Golub & Van Loan
+// sym.Schur2 rotation), eigenvalue sort, U = L^-T W.
 // The eigenvectors are M-orthonormal (U' M U = I), the LAPACK sygv / MATLAB 'chol' normalisation.
+// Orders up to kGeigClusterMaxN (160: what the Cholesky and substitution kernels hold in one CTA's shared
+// memory) run the Jacobi sweeps on a thread-block cluster (k_jacobi_cluster); larger ones run the whole
+// algorithm on one CTA in a global workspace (k_geig_sym).
+#include <atomic>
+
 #include "ofrr_internal.cuh"
 
 namespace ofrr {
+
+// ======================================================================================
+// Jacobi sweeps on a cluster
+// ======================================================================================
+// GB300 runs FP64 at 1/64 of its FP32 rate (a warp instruction occupies an SM sub-partition for about 64
+// cycles), so the sweeps are bound by the FP64 pipe of the SMs they run on and, between two barriers, by
+// the dependent chain that turns (a_pp, a_qq, a_pq) into a rotation (measured on 16 CTAs at n = 64, cycles
+// per round: rotations 3260, C 1100, handing over 100, barrier 1180).  The rotations of a round are
+// independent, so they are spread over a cluster: CTA c owns the seats of PP = ceil(N / 2 / NC) pairs of
+// the round-robin schedule, i.e. 2 PP columns of C and of W.  Rows and columns of a 2 x 2 block only
+// depend on that block, so a round is one pass over the CTA's columns; the new columns go straight to the
+// CTA that holds their seat in the next round (every seat moves by one), into the other of two buffers
+// through distributed shared memory, and the three entries each next rotation needs go to every CTA.  So
+// a round costs one cluster barrier, and every CTA computes all rotations itself (N / 2 threads; the
+// chain's latency does not depend on how many warps run it, up to one per sub-partition).
+constexpr int kJacT = 512;
+constexpr int kGeigClusterMaxN = 160;
+
+// The rotation of sym.Schur2 (t the root of smaller magnitude of t^2 + 2 tau t - 1 = 0, t = 1 for tau = 0).
+// Divisions and square roots are FP64 sequences of about 430 cycles each, so the chain takes ~2000 cycles, the
+// largest part of a round.  Taking the angle in FP32 and normalising (c, s) in FP64 halves it, but on the SVD
+// pencil [[0, K], [K', 0]] of a block U ~ A V the matrix K is triangular up to rounding, equal diagonal entries
+// meet entries of rounding size, and which of the two roots is taken (the sign of the vectors) then hangs on the
+// last bits: the quotients keep every result what the one-CTA form gives, bit for bit.
+__device__ __forceinline__ bool jac_nonzero(double x) {  // an FP64 compare costs ~100 cycles
+  return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) != 0;
+}
+__device__ __forceinline__ void jac_rotation(double app, double aqq, double apq, double* c, double* s) {
+  *c = 1.0;
+  *s = 0.0;
+  if (!jac_nonzero(apq)) return;
+  const double tau = (aqq - app) / (2.0 * apq);
+  const double t = __drcp_rn(fabs(tau) + sqrt(1.0 + tau * tau));
+  *c = __drcp_rn(sqrt(1.0 + t * t));
+  const double sa = t * *c;
+  *s = (__double2hiint(tau) < 0 && jac_nonzero(tau)) ? -sa : sa;
+}
+// c a - s b and s a + c b, one product rounded before the sum (the contraction k_geig_sym's expressions get)
+__device__ __forceinline__ double jac_diff(double c, double a, double s, double b) {
+  return __fma_rn(c, a, -__dmul_rn(s, b));
+}
+__device__ __forceinline__ double jac_sum(double s, double a, double c, double b) {
+  return __fma_rn(s, a, __dmul_rn(c, b));
+}
+
+__device__ __forceinline__ void jac_st(unsigned addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+// The index at a seat in round 0 of a sweep is the seat itself; every round all seats but seat 0 (step 0)
+// advance by one through 1 .. N - 1.
+__device__ __forceinline__ int jac_next(int i, int step, int N) {
+  i += step;
+  return i == N ? 1 : i;
+}
+// the seat a column sits at in the next round
+__device__ __forceinline__ int jac_next_seat(int s, int N) { return (s == 0) ? 0 : (s == 1) ? N - 1 : s - 1; }
+
+// C (n x n, symmetric, ld n) -> eigenvalues w (sorted) and the matching orthonormal eigenvectors Wout
+// (ld n).  Grid = one cluster of NC CTAs.  Every thread owns up to IT items of C (one row pair of one of the
+// CTA's columns; adjacent lanes the two columns of a 2 x 2 block) and IT items of W (one row of one of the
+// CTA's column pairs), and at most one remote entry of the next rotations: their seats never change, so only
+// the indices at the seats are stepped from round to round.  W trails by one round: W <- W J runs beside
+// the next round's rotations, which keep one or a few warps in a dependent FP64 chain.
+template <int IT>
+__global__ void __launch_bounds__(kJacT) k_jacobi_cluster(int n, int NC, int PP, const double* __restrict__ Cin,
+                                                          double* __restrict__ w, double* __restrict__ Wout,
+                                                          int descending, int max_sweeps) {
+  extern __shared__ double jsm[];
+  const int N = n + (n & 1), npair = N / 2, S = 2 * PP;
+  const int rank = (int)cluster_rank();
+  const int tid = threadIdx.x;
+  double* cb = jsm;                          // [2][S][n]
+  double* wb = cb + (size_t)2 * S * n;       // [2][S][n]
+  double* sD = wb + (size_t)2 * S * n;       // [2][npair][3]: a_pp, a_qq, a_pq of every pair
+  double2* s_cs = reinterpret_cast<double2*>(sD + (size_t)2 * npair * 3);  // [2][npair]: c, s of every pair
+  double* s_stage = reinterpret_cast<double*>(s_cs + (size_t)2 * npair);   // [S][2]: the next rotations' entries of this CTA's columns
+  double* s_diag = s_stage + 2 * S;          // n: the final diagonal
+  double* s_part = s_diag + n;               // [NC][2]: off and total sums of squares
+  __shared__ double s_red[2][kJacT / 32];
+  const int k0 = rank * PP;                  // this CTA's first pair
+  // slot 2 l + side holds seat k0 + l (side 0) or N - 1 - (k0 + l) (side 1)
+  auto seat_of = [&](int slot) {
+    const int k = k0 + (slot >> 1);
+    return (slot & 1) ? N - 1 - k : k;
+  };
+  // where the column at slot `slot` goes: CTA, and slot there
+  auto dest = [&](int slot, int* cta) {
+    const int s2 = jac_next_seat(seat_of(slot), N), kk = (s2 < npair) ? s2 : N - 1 - s2;
+    *cta = kk / PP;
+    return 2 * (kk % PP) + (s2 >= npair ? 1 : 0);
+  };
+  auto barrier = [&]() {
+    if (NC > 1) {
+      cluster_arrive();
+      cluster_wait();
+    } else {
+      __syncthreads();
+    }
+  };
+  // items of C: row pair (seats ck, N - 1 - ck), column slot; indices at the seats
+  int c_slot[IT], c_k[IT], c_p[IT], c_q[IT], c_j[IT], c_jp[IT], c_j2[IT];
+  int c_s0[IT], c_s2[IT];  // steps of the column's and of the next partner's seat
+  unsigned c_dst[IT];
+#pragma unroll
+  for (int u = 0; u < IT; ++u) {
+    const int e = tid + u * kJacT, l = (e >> 1) / npair;
+    c_k[u] = (e >> 1) - l * npair;
+    c_slot[u] = (l < PP && k0 + l < npair) ? 2 * l + (e & 1) : -1;
+    c_p[u] = c_k[u];
+    c_q[u] = N - 1 - c_k[u];
+    c_j[u] = c_jp[u] = c_j2[u] = n;
+    c_dst[u] = 0;
+    c_s0[u] = c_s2[u] = 1;
+    if (c_slot[u] >= 0) {
+      int cta;
+      const int ds = dest(c_slot[u], &cta);
+      c_dst[u] = cluster_map(cb + (size_t)ds * n, cta);
+      c_j[u] = seat_of(c_slot[u]);
+      c_jp[u] = seat_of(c_slot[u] ^ 1);
+      c_j2[u] = N - 1 - jac_next_seat(c_j[u], N);  // index at the next partner's seat, this round
+      c_s0[u] = c_j[u] != 0;
+      c_s2[u] = c_j2[u] != 0;
+    }
+  }
+  // what an item does in the coming round, from the indices at its seats: offsets of its rows p < q and a code
+  // (1 active, 2 row q exists, 4 column p of its pair, 8 / 16 its vq / vp is the rotated entry, 32 / 64 vp / vq
+  // is the column's diagonal entry, 128 / 256 vp / vq is the entry (next partner, column)).  Computed between
+  // arriving at the round's barrier and waiting for it.
+  int c_po[IT], c_qo[IT], c_code[IT];
+  auto plan_c = [&]() {
+#pragma unroll
+    for (int u = 0; u < IT; ++u) {
+      const int p = min(c_p[u], c_q[u]), q = max(c_p[u], c_q[u]), j = c_j[u];
+      c_po[u] = p;
+      c_qo[u] = q;
+      int code = 0;
+      if (j < n) {
+        const int j2 = jac_next(c_j2[u], c_s2[u], N);
+        code = 1 | (q < n ? 2 : 0) | (j < c_jp[u] ? 4 : 0);
+        if (c_k[u] == k0 + (c_slot[u] >> 1)) code |= (j == p) ? 8 : 16;
+        code |= (p == j ? 32 : 0) | (q == j ? 64 : 0);
+        if (j2 < j) code |= (p == j2 ? 128 : 0) | (q == j2 ? 256 : 0);
+      }
+      c_code[u] = code;
+    }
+  };
+  auto step_c = [&]() {
+#pragma unroll
+    for (int u = 0; u < IT; ++u) {
+      if (c_slot[u] < 0) continue;
+      // seat 0 is only ever a pair's side 0: the other side's seat always steps
+      c_j[u] = jac_next(c_j[u], c_s0[u], N);
+      c_jp[u] = jac_next(c_jp[u], (c_slot[u] & 1) ? (k0 + (c_slot[u] >> 1)) != 0 : 1, N);
+      c_j2[u] = jac_next(c_j2[u], c_s2[u], N);
+      c_p[u] = jac_next(c_p[u], c_k[u] != 0, N);
+      c_q[u] = jac_next(c_q[u], 1, N);
+    }
+    plan_c();
+  };
+  plan_c();
+  // items of W: the first ones go to the warps that compute no rotations
+  const int rot_warps = (npair + 31) / 32;
+  const int wt = (tid + kJacT - 32 * rot_warps) % kJacT;
+  int w_l[IT], w_i[IT], w_a[IT], w_b[IT];
+  unsigned w_da[IT], w_db[IT];
+#pragma unroll
+  for (int u = 0; u < IT; ++u) {
+    const int e = wt + u * kJacT, l = e / n;
+    w_i[u] = e - l * n;
+    w_l[u] = (l < PP && k0 + l < npair) ? l : -1;
+    w_a[u] = w_b[u] = n;
+    w_da[u] = w_db[u] = 0;
+    if (w_l[u] >= 0) {
+      int cta;
+      int ds = dest(2 * l, &cta);
+      w_da[u] = cluster_map(wb + (size_t)ds * n + w_i[u], cta);
+      ds = dest(2 * l + 1, &cta);
+      w_db[u] = cluster_map(wb + (size_t)ds * n + w_i[u], cta);
+      w_a[u] = k0 + l;
+      w_b[u] = N - 1 - (k0 + l);
+    }
+  }
+  // the remote entry this thread pushes: (slot, diagonal or off-diagonal) to CTA e_cta
+  int e_slot = -1, e_j = n, e_j2 = n, e_s = 1, e_s2 = 1;
+  unsigned e_dst = 0;
+  if (tid < 2 * S * NC) {
+    const int sl = (tid >> 1) % S, cta = (tid >> 1) / S;
+    if (k0 + (sl >> 1) < npair) {
+      const int s2 = jac_next_seat(seat_of(sl), N), k2 = (s2 < npair) ? s2 : N - 1 - s2;
+      e_slot = sl;
+      e_j = seat_of(sl);
+      e_j2 = N - 1 - s2;
+      e_s = e_j != 0;
+      e_s2 = e_j2 != 0;
+      e_dst = cluster_map(sD + (size_t)k2 * 3, cta);
+    }
+  }
+  // byte offset of this thread's entry among its pair's three (-1: nothing to push this round)
+  int e_off = -1;
+  auto plan_e = [&]() {
+    e_off = -1;
+    if (e_slot < 0 || e_j >= n) return;
+    const int j2 = jac_next(e_j2, e_s2, N);
+    if (tid & 1) e_off = (j2 < e_j) ? 16 : -1;
+    else e_off = (e_j < j2) ? 0 : 8;
+  };
+  auto step_e = [&]() {
+    if (e_slot < 0) return;
+    e_j = jac_next(e_j, e_s, N);
+    e_j2 = jac_next(e_j2, e_s2, N);
+    plan_e();
+  };
+  plan_e();
+  int r_x = tid, r_y = N - 1 - tid;  // indices of the pair whose rotation this thread computes (tid < npair)
+
+  for (int e = tid; e < S * n; e += kJacT) {
+    const int sl = e / n, i = e - sl * n;
+    const int j = (k0 + (sl >> 1) < npair) ? seat_of(sl) : n;
+    if (j < n) {
+      cb[e] = Cin[i + (size_t)j * n];
+      wb[e] = (i == j) ? 1.0 : 0.0;
+    }
+  }
+  for (int k = tid; k < npair; k += kJacT) {
+    const int p = k, q = N - 1 - k;
+    sD[3 * k] = Cin[p + (size_t)p * n];
+    sD[3 * k + 1] = (q < n) ? Cin[q + (size_t)q * n] : 0.0;
+    sD[3 * k + 2] = (q < n) ? Cin[p + (size_t)q * n] : 0.0;
+  }
+  __syncthreads();
+  barrier();
+
+  const unsigned bufbytes = (unsigned)((size_t)S * n * sizeof(double));
+  const unsigned dbytes = (unsigned)((size_t)npair * 3 * sizeof(double));
+  int b = 0;
+  bool pending = false;
+  // W <- W J with the rotations of the round before (parity b ^ 1), into buffer b
+  auto update_w = [&]() {
+    const double2* cs = s_cs + (size_t)(b ^ 1) * npair;
+    const unsigned nxt = b ? bufbytes : 0u;
+#pragma unroll
+    for (int u = 0; u < IT; ++u) {
+      if (w_l[u] < 0) continue;
+      const int kg = k0 + w_l[u];
+      const double* W0 = wb + ((size_t)(b ^ 1) * S + 2 * w_l[u]) * n + w_i[u];
+      double wa = W0[0], wv = W0[n];
+      const double c = cs[kg].x, s = cs[kg].y;
+      const bool ab = w_a[u] < w_b[u];
+      if (jac_nonzero(s)) {
+        const double ap = ab ? wa : wv, aq = ab ? wv : wa;
+        const double vp = jac_diff(c, ap, s, aq), vq = jac_sum(s, ap, c, aq);
+        wa = ab ? vp : vq;
+        wv = ab ? vq : vp;
+      }
+      if (w_a[u] < n) jac_st(w_da[u] + nxt, wa);
+      if (w_b[u] < n) jac_st(w_db[u] + nxt, wv);
+      w_a[u] = jac_next(w_a[u], kg != 0, N);
+      w_b[u] = jac_next(w_b[u], 1, N);
+    }
+  };
+  for (int sweep = 0; sweep < max_sweeps && n > 1; ++sweep) {
+    {  // converged when off(C)^2 <= eps^2 ||C||_F^2
+      double off = 0.0, tot = 0.0;
+      for (int e = tid; e < S * n; e += kJacT) {
+        const int sl = e / n, i = e - sl * n;
+        const int j = (k0 + (sl >> 1) < npair) ? seat_of(sl) : n;  // a sweep starts with seat s holding index s
+        if (j < n) {
+          const double x = cb[(size_t)b * S * n + e], v = x * x;
+          tot += v;
+          if (i != j) off += v;
+        }
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        off += __shfl_down_sync(0xffffffffu, off, o);
+        tot += __shfl_down_sync(0xffffffffu, tot, o);
+      }
+      if ((tid & 31) == 0) {
+        s_red[0][tid >> 5] = off;
+        s_red[1][tid >> 5] = tot;
+      }
+      __syncthreads();
+      if (tid < 2 * NC) {
+        double a = 0.0;
+        for (int x = 0; x < kJacT / 32; ++x) a += s_red[tid & 1][x];
+        jac_st(cluster_map(s_part + 2 * rank + (tid & 1), (unsigned)(tid >> 1)), a);
+      }
+      barrier();
+      double so = 0.0, sa = 0.0;
+      for (int c = 0; c < NC; ++c) {
+        so += s_part[2 * c];
+        sa += s_part[2 * c + 1];
+      }
+      if (so <= 1.0e-32 * sa) break;  // every thread of every CTA sees the same sums
+    }
+    for (int r = 0; r < N - 1; ++r) {
+      double2* cs = s_cs + (size_t)b * npair;
+      const double* cur = cb + (size_t)b * S * n;
+      double xp[IT], xq[IT];  // this round's entries, read before the rotations are known
+#pragma unroll
+      for (int u = 0; u < IT; ++u) {
+        const double* col = cur + (size_t)max(c_slot[u], 0) * n;
+        xp[u] = (c_code[u] & 1) ? col[c_po[u]] : 0.0;
+        xq[u] = (c_code[u] & 2) ? col[c_qo[u]] : 0.0;
+      }
+      if (tid < npair) {
+        const double* D = sD + ((size_t)b * npair + tid) * 3;
+        double c = 1.0, s = 0.0;
+        if (max(r_x, r_y) < n) jac_rotation(D[0], D[1], D[2], &c, &s);
+        cs[tid] = make_double2(c, s);
+      }
+      if (pending) update_w();
+      __syncthreads();
+      // C <- J' C J on this CTA's columns
+      const unsigned nxt = b ? 0u : bufbytes;
+#pragma unroll
+      for (int u = 0; u < IT; ++u) {
+        // a warp without items leaves as a whole: a predicated-off FP64 instruction still occupies the pipe
+        const int code = c_code[u];
+        if (!__any_sync(0xffffffffu, code)) continue;
+        const double2 ck = cs[c_k[u]], cg = cs[min(k0 + (max(c_slot[u], 0) >> 1), npair - 1)];
+        double vp = xp[u], vq = xq[u];
+        if ((code & 1) && jac_nonzero(ck.y)) {
+          vp = jac_diff(ck.x, xp[u], ck.y, xq[u]);
+          vq = jac_sum(ck.y, xp[u], ck.x, xq[u]);
+        }
+        const double zp = __shfl_xor_sync(0xffffffffu, vp, 1), zq = __shfl_xor_sync(0xffffffffu, vq, 1);
+        if (code & 1) {
+          if (jac_nonzero(cg.y)) {
+            // column p of its pair: fma(c, a_p, -(s a_q)); column q: fma(s, a_p, c a_q)
+            const bool cp = code & 4;
+            const double m1 = cp ? cg.x : cg.y, m2 = cp ? -cg.y : cg.x;
+            const double ap_ = cp ? vp : zp, aq_ = cp ? zp : vp, bp_ = cp ? vq : zq, bq_ = cp ? zq : vq;
+            vp = __fma_rn(m1, ap_, __dmul_rn(m2, aq_));
+            vq = __fma_rn(m1, bp_, __dmul_rn(m2, bq_));
+            if (code & 8) vq = 0.0;
+            if (code & 16) vp = 0.0;
+          }
+          jac_st(c_dst[u] + nxt + 8u * (unsigned)c_po[u], vp);
+          if (code & 2) jac_st(c_dst[u] + nxt + 8u * (unsigned)c_qo[u], vq);
+          // entries of the next round's rotations
+          if (code & 96) s_stage[2 * c_slot[u]] = (code & 32) ? vp : vq;
+          if (code & 384) s_stage[2 * c_slot[u] + 1] = (code & 128) ? vp : vq;
+        }
+      }
+      __syncthreads();
+      // this CTA's entries of the next rotations, to every CTA
+      if (e_off >= 0) jac_st(e_dst + (b ? 0u : dbytes) + (unsigned)e_off, s_stage[2 * e_slot + (tid & 1)]);
+      if (NC > 1) cluster_arrive();
+      step_c();
+      step_e();
+      if (tid < npair) {
+        r_x = jac_next(r_x, tid != 0, N);
+        r_y = jac_next(r_y, 1, N);
+      }
+      if (NC > 1) cluster_wait();
+      else __syncthreads();
+      b ^= 1;
+      pending = true;
+    }
+  }
+  if (pending) update_w();
+  // the diagonal to every CTA, then each CTA writes its columns at their rank (ties by index)
+  for (int e = tid; e < S * NC; e += kJacT) {
+    const int slot = e % S, c = e / S;
+    const int j = (k0 + (slot >> 1) < npair) ? seat_of(slot) : n;
+    if (j < n) jac_st(cluster_map(s_diag + j, c), cb[((size_t)b * S + slot) * n + j]);
+  }
+  barrier();  // after this barrier no CTA reads or writes another's shared memory
+  for (int slot = tid >> 5; slot < S; slot += kJacT / 32) {
+    const int j = (k0 + (slot >> 1) < npair) ? seat_of(slot) : n;
+    if (j >= n) continue;
+    const double dj = s_diag[j];
+    int rk = 0;
+    for (int i = tid & 31; i < n; i += 32) {
+      const double di = s_diag[i];
+      const bool before = descending ? (di > dj || (di == dj && i < j)) : (di < dj || (di == dj && i < j));
+      rk += before ? 1 : 0;
+    }
+    rk = __reduce_add_sync(0xffffffffu, rk);
+    if ((tid & 31) == 0) w[rk] = dj;
+    for (int i = tid & 31; i < n; i += 32) Wout[i + (size_t)rk * n] = wb[((size_t)b * S + slot) * n + i];
+  }
+}
+
+// C = (G + G') / 2 (or G itself)
+__global__ void k_sym_copy(int n, const double* __restrict__ G, int ldg, int symmetrize, double* __restrict__ C) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
+    const int i = e % n, j = e / n;
+    const double g = G[i + (size_t)j * ldg];
+    C[e] = symmetrize ? 0.5 * (g + G[j + (size_t)i * ldg]) : g;
+  }
+}
 
 struct GeigParams {
   int n;
@@ -22,7 +418,7 @@ struct GeigParams {
   double* w;   // out, n
   double* U;   // out, n x n (ldu)
   int ldu;
-  double* gws;  // global workspace (3 n^2) when shared memory is too small
+  double* gws;  // global workspace (3 n^2)
   int* flag;    // out: 1 if the Cholesky factor needed a clamp (near-singular M)
   int max_sweeps;
 };
@@ -30,10 +426,8 @@ struct GeigParams {
 __device__ __forceinline__ int rr_index(int i, int r, int N) { return i == 0 ? 0 : ((i - 1 + r) % (N - 1)) + 1; }
 
 __global__ void __launch_bounds__(512) k_geig_sym(GeigParams P) {
-  extern __shared__ double sm[];
   const int n = P.n, tid = threadIdx.x, nt = blockDim.x;
-  const bool in_smem = (P.gws == nullptr);
-  double* C = in_smem ? sm : P.gws;
+  double* C = P.gws;
   double* W = C + (size_t)n * n;
   double* L = W + (size_t)n * n;
   __shared__ double s_c[160], s_s[160];
@@ -242,19 +636,124 @@ __global__ void __launch_bounds__(512) k_geig_sym(GeigParams P) {
   }
 }
 
-static int geig_launch(ofrr_ctx* ctx, GeigParams P) {
-  const size_t need = (size_t)3 * P.n * P.n * sizeof(double);
-  int st = OFRR_SUCCESS;
-  size_t smem = 0;
-  if (need <= 200 * 1024) {
-    smem = need;
-    P.gws = nullptr;
-    OFRR_TRY(allow_smem(k_geig_sym));
-  } else {
-    P.gws = ws_get<double>(ctx, (size_t)3 * P.n * P.n, &st);
-    if (!P.gws) return st;
+static size_t jacobi_smem(int n, int NC) {
+  const int N = n + (n & 1), npair = N / 2, PP = (npair + NC - 1) / NC, S = 2 * PP;
+  return sizeof(double) * ((size_t)4 * S * n + 6 * npair + 4 * npair + 2 * S + n + 2 * NC);
+}
+
+// CTAs of the Jacobi cluster.  A round costs the rotation chain and a barrier on any cluster (about 2.6 us
+// on one CTA, 2.9 us on sixteen) plus 6 n^2 FP64 operations shared by the CTAs (one warp instruction per 64
+// cycles and SM sub-partition).  Whole syev calls, random matrices, us for 1 / 4 / 8 / 16 CTAs:
+//   n = 16: 258 / 277 / 289 / 307    n = 32: 1028 / 715 / 716 / 758   n = 48: - / 1279 / 1125 / 1109
+//   n = 64: - / 2148 / 1627 / 1511   n = 96: - / - / 4057 / 3061      n = 128: - / - / 7137 / 5069
+// (the one-CTA kernel below: 363, 1332, 3234, 6146, 23418 and 49327 us).  Sixteen CTAs are beyond the
+// portable cluster size: 0 when the device cannot place them and eight cannot hold the items either.
+static int jacobi_cluster_size(int n) {
+  if (n <= 20) return 1;
+  if (n <= 40) return 4;
+  if (n <= 56) return 8;
+  static std::atomic<int> max_cluster[64];  // per device: 0 not asked yet, else 8 or 16
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return n <= 128 ? 8 : 0;
+  int mc = max_cluster[dev].load(std::memory_order_relaxed);
+  if (mc == 0) {
+    mc = 8;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(kJacT);
+    cfg.dynamicSmemBytes = jacobi_smem(kGeigClusterMaxN, 16);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(k_jacobi_cluster<2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        allow_smem(k_jacobi_cluster<2>) == OFRR_SUCCESS &&
+        cudaOccupancyMaxActiveClusters(&clusters, k_jacobi_cluster<2>, &cfg) == cudaSuccess && clusters >= 1)
+      mc = 16;
+    (void)cudaGetLastError();  // a refused query leaves the portable size
+    max_cluster[dev].store(mc, std::memory_order_relaxed);
   }
-  k_geig_sym<<<1, 512, smem, ctx->stream>>>(P);
+  return mc == 16 ? 16 : n <= 128 ? 8 : 0;
+}
+
+template <int IT>
+static int jacobi_launch(ofrr_ctx* ctx, int n, int NC, const double* C, double* w, double* W, int descending,
+                         int max_sweeps) {
+  OFRR_TRY(allow_smem(k_jacobi_cluster<IT>));
+  if (NC > 8)
+    OFRR_CUDA(cudaFuncSetAttribute(k_jacobi_cluster<IT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)NC;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)NC);
+  cfg.blockDim = dim3(kJacT);
+  cfg.dynamicSmemBytes = jacobi_smem(n, NC);
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const int PP = ((n + 1) / 2 + NC - 1) / NC;
+  OFRR_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi_cluster<IT>, n, NC, PP, C, w, W, descending, max_sweeps));
+  OFRR_LAUNCHED(ctx, "k_jacobi_cluster");
+  return OFRR_SUCCESS;
+}
+
+// The cluster form: Cholesky, two substitutions, the Jacobi sweeps, and the back substitution.
+static int geig_cluster(ofrr_ctx* ctx, const GeigParams& P, int NC) {
+  int st = OFRR_SUCCESS;
+  const int n = P.n;
+  const size_t nn = (size_t)n * n;
+  double *C = ws_get<double>(ctx, nn, &st), *W = ws_get<double>(ctx, nn, &st);
+  if (!C || !W) return st;
+  const unsigned g = (unsigned)std::min<size_t>((nn + 255) / 256, 152);
+  double *L = nullptr, *Y = nullptr;
+  if (P.M) {
+    L = ws_get<double>(ctx, nn, &st);
+    Y = ws_get<double>(ctx, nn, &st);
+    if (!L || !Y) return st;
+    k_sym_copy<<<g, 256, 0, ctx->stream>>>(n, P.G, P.ldg, P.symmetrize, W);
+    OFRR_LAUNCHED(ctx, "k_sym_copy");
+    OFRR_TRY(small_chol(ctx, n, P.M, P.ldm, L));
+    OFRR_TRY(small_trsm(ctx, n, L, W, 0, Y, 0));  // Y = L^-1 G
+    OFRR_TRY(small_trsm(ctx, n, L, Y, 1, W, 0));  // W = L^-1 Y' = L^-1 G L^-T
+    k_sym_copy<<<g, 256, 0, ctx->stream>>>(n, W, n, 1, C);
+    OFRR_LAUNCHED(ctx, "k_sym_copy");
+  } else {
+    k_sym_copy<<<g, 256, 0, ctx->stream>>>(n, P.G, P.ldg, P.symmetrize, C);
+    OFRR_LAUNCHED(ctx, "k_sym_copy");
+  }
+  double* Wj = (!P.M && P.ldu == n) ? P.U : W;
+  // items of C and of W per thread: (N / 2) 2 PP and n PP over kJacT threads
+  const int PP = ((n + 1) / 2 + NC - 1) / NC, items = (n + (n & 1)) * PP;
+  if (items > 2 * kJacT || 4 * PP * NC > kJacT) return OFRR_ERR_INTERNAL;
+  if (items <= kJacT)
+    OFRR_TRY(jacobi_launch<1>(ctx, n, NC, C, P.w, Wj, P.descending, P.max_sweeps));
+  else
+    OFRR_TRY(jacobi_launch<2>(ctx, n, NC, C, P.w, Wj, P.descending, P.max_sweeps));
+  double* Uc = Wj;
+  if (P.M) {
+    Uc = (P.ldu == n) ? P.U : Y;
+    OFRR_TRY(small_trsm(ctx, n, L, W, 0, Uc, 1));  // U = L^-T W
+  }
+  if (Uc != P.U)
+    OFRR_CUDA(cudaMemcpy2DAsync(P.U, P.ldu * sizeof(double), Uc, n * sizeof(double), n * sizeof(double), n,
+                                cudaMemcpyDeviceToDevice, ctx->stream));
+  return OFRR_SUCCESS;
+}
+
+static int geig_launch(ofrr_ctx* ctx, GeigParams P) {
+  const int NC = (P.n <= kGeigClusterMaxN) ? jacobi_cluster_size(P.n) : 0;
+  if (NC > 0) return geig_cluster(ctx, P, NC);
+  int st = OFRR_SUCCESS;
+  P.gws = ws_get<double>(ctx, (size_t)3 * P.n * P.n, &st);
+  if (!P.gws) return st;
+  k_geig_sym<<<1, 512, 0, ctx->stream>>>(P);
   OFRR_LAUNCHED(ctx, "k_geig_sym");
   return OFRR_SUCCESS;
 }

@@ -26,6 +26,9 @@ namespace ofrr {
 // ---- 1. Cholesky (lower) of M + tau I; batched over blockIdx.x ------------------------------------
 // Right-looking; per column one reciprocal square root, the column scaled by it, and the lower
 // triangle of the trailing block updated with one warp per column (no index division).
+// EXACT: square root and divisions instead of the reciprocal square root (the reference-semantics solver,
+// whose results depend on the last bits of its operands: see smalleig.cu).
+template <bool EXACT>
 __global__ void __launch_bounds__(256) k_chol_f64(int n, const double* const* Ms, int ldm, double tau,
                                                   double* const* Ls, int* flag) {
   extern __shared__ double S[];
@@ -69,15 +72,19 @@ __global__ void __launch_bounds__(256) k_chol_f64(int n, const double* const* Ms
       d = floor_d;
       if (flag) *flag = 1;
     }
-    const double r = rsqrt(d);
-    S[k + k * n] = d * r;
-    s_rinv2[k & 1] = r;
+    if constexpr (EXACT) {
+      s_rinv2[k & 1] = S[k + k * n] = sqrt(d);
+    } else {
+      const double r = rsqrt(d);
+      S[k + k * n] = d * r;
+      s_rinv2[k & 1] = r;
+    }
   };
   if (tid == 0 && n > 0) pivot(0);
   __syncthreads();
   for (int k = 0; k < n; ++k) {
     const double rinv = s_rinv2[k & 1];
-    for (int i = k + 1 + tid; i < n; i += nt) S[i + k * n] *= rinv;
+    for (int i = k + 1 + tid; i < n; i += nt) S[i + k * n] = EXACT ? S[i + k * n] / rinv : S[i + k * n] * rinv;
     __syncthreads();
     if (warp == nw - 1) {
       if (lane == 0 && k + 1 < n) {
@@ -106,7 +113,8 @@ __global__ void __launch_bounds__(256) k_chol_f64(int n, const double* const* Ms
 // is 1/64 rate, so a shuffle-reduced dot product per row would cost several times more).
 // TRSM_R: rows per lane (n <= 32 TRSM_R), a template so that no predicated-off FP64 instruction
 // occupies the 1/64-rate pipe.
-template <int TRSM_R>
+// EXACT: x_i = x_i / L_ii correctly rounded (pivot_div).
+template <int TRSM_R, bool EXACT>
 // blockIdx.y selects one of up to two independent systems (L, B, X), (L2, B2, X2) of the same shape
 __global__ void __launch_bounds__(128) k_trsm_f64(int n, int nrhs, const double* __restrict__ L1, int ldl,
                                                   const double* __restrict__ B1, int ldb, int transB,
@@ -154,7 +162,8 @@ __global__ void __launch_bounds__(128) k_trsm_f64(int n, int nrhs, const double*
       for (int il = 0; il < 32; ++il) {
         const int i = 32 * u + il;
         if (i >= n) break;
-        const double xi = __shfl_sync(0xffffffffu, x[u], il) * rd[i];
+        const double xs = __shfl_sync(0xffffffffu, x[u], il);
+        const double xi = EXACT ? pivot_div(xs, Ls[i + i * ld], rd[i], pivot_fast(Ls[i + i * ld])) : xs * rd[i];
         if (lane == il) x[u] = xi;
 #pragma unroll
         for (int v = u; v < TRSM_R; ++v) {
@@ -169,7 +178,8 @@ __global__ void __launch_bounds__(128) k_trsm_f64(int n, int nrhs, const double*
       for (int il = 31; il >= 0; --il) {
         const int i = 32 * u + il;
         if (i >= n) continue;
-        const double xi = __shfl_sync(0xffffffffu, x[u], il) * rd[i];
+        const double xs = __shfl_sync(0xffffffffu, x[u], il);
+        const double xi = EXACT ? pivot_div(xs, Ls[i + i * ld], rd[i], pivot_fast(Ls[i + i * ld])) : xs * rd[i];
         if (lane == il) x[u] = xi;
 #pragma unroll
         for (int v = 0; v <= u; ++v) {
@@ -622,26 +632,29 @@ static int gemm_small2(ofrr_ctx* ctx, const GemmSmall& g0, const GemmSmall& g1) 
   return OFRR_SUCCESS;
 }
 
-template <int R>
+template <int R, bool EXACT>
 static int trsm_r(ofrr_ctx* ctx, int n, int nrhs, const double* L, const double* B, int ldb, int transB, double* X,
                   int upper, const double* L2, const double* B2, double* X2) {
   const size_t smem = ((size_t)n * (n + 1) + (size_t)n) * sizeof(double);
-  OFRR_TRY(allow_smem(k_trsm_f64<R>));
+  OFRR_TRY(allow_smem(k_trsm_f64<R, EXACT>));
   const dim3 grid((unsigned)((nrhs + 3) / 4), L2 ? 2u : 1u);
-  k_trsm_f64<R><<<grid, 128, smem, ctx->stream>>>(n, nrhs, L, n, B, ldb, transB, X, n, upper, L2, B2, X2);
+  k_trsm_f64<R, EXACT><<<grid, 128, smem, ctx->stream>>>(n, nrhs, L, n, B, ldb, transB, X, n, upper, L2, B2, X2);
   OFRR_LAUNCHED(ctx, "k_trsm_f64");
   return OFRR_SUCCESS;
 }
 
 // X = L^-1 B (upper == 0) or L^-T B (upper == 1); with L2 set, X2 = (same op of L2) B2 in the same launch
+template <bool EXACT = false>
 static int trsm(ofrr_ctx* ctx, int n, int nrhs, const double* L, const double* B, int ldb, int transB, double* X,
                 int upper, const double* L2 = nullptr, const double* B2 = nullptr, double* X2 = nullptr) {
-  if (n <= 32) return trsm_r<1>(ctx, n, nrhs, L, B, ldb, transB, X, upper, L2, B2, X2);
-  if (n <= 64) return trsm_r<2>(ctx, n, nrhs, L, B, ldb, transB, X, upper, L2, B2, X2);
-  if (n <= 96) return trsm_r<3>(ctx, n, nrhs, L, B, ldb, transB, X, upper, L2, B2, X2);
-  return trsm_r<4>(ctx, n, nrhs, L, B, ldb, transB, X, upper, L2, B2, X2);
+  if (n <= 32) return trsm_r<1, EXACT>(ctx, n, nrhs, L, B, ldb, transB, X, upper, L2, B2, X2);
+  if (n <= 64) return trsm_r<2, EXACT>(ctx, n, nrhs, L, B, ldb, transB, X, upper, L2, B2, X2);
+  if (n <= 96) return trsm_r<3, EXACT>(ctx, n, nrhs, L, B, ldb, transB, X, upper, L2, B2, X2);
+  if (n > 128) return trsm_r<5, EXACT>(ctx, n, nrhs, L, B, ldb, transB, X, upper, L2, B2, X2);
+  return trsm_r<4, EXACT>(ctx, n, nrhs, L, B, ldb, transB, X, upper, L2, B2, X2);
 }
 
+template <bool EXACT = false>
 static int chol(ofrr_ctx* ctx, int n, int count, const double* const* Ms_host, int ldm, double tau,
                 double* const* Ls_host) {
   int st = OFRR_SUCCESS;
@@ -651,10 +664,19 @@ static int chol(ofrr_ctx* ctx, int n, int count, const double* const* Ms_host, i
   const void* hp[4] = {Ms_host[0], count > 1 ? Ms_host[1] : Ms_host[0], Ls_host[0], count > 1 ? Ls_host[1] : Ls_host[0]};
   OFRR_CUDA(cudaMemcpyAsync(Md, hp, sizeof(hp), cudaMemcpyHostToDevice, ctx->stream));
   const size_t smem = (size_t)n * n * sizeof(double);
-  OFRR_TRY(allow_smem(k_chol_f64));
-  k_chol_f64<<<count, 256, smem, ctx->stream>>>(n, Md, ldm, tau, Ld, ctx->dev_flags + 1);
+  OFRR_TRY(allow_smem(k_chol_f64<EXACT>));
+  k_chol_f64<EXACT><<<count, 256, smem, ctx->stream>>>(n, Md, ldm, tau, Ld, ctx->dev_flags + 1);
   OFRR_LAUNCHED(ctx, "k_chol_f64");
   return OFRR_SUCCESS;
+}
+
+int small_chol(ofrr_ctx* ctx, int n, const double* M, int ldm, double* L) {
+  if (n > 160) return OFRR_ERR_BLAS_INVALID_SIZE;
+  return chol<true>(ctx, n, 1, &M, ldm, 0.0, &L);
+}
+int small_trsm(ofrr_ctx* ctx, int n, const double* L, const double* B, int transB, double* X, int upper) {
+  if (n > 160) return OFRR_ERR_BLAS_INVALID_SIZE;
+  return trsm<true>(ctx, n, n, L, B, n, transB, X, upper);
 }
 
 // Ogita-Aishima refinement of approximate eigenvectors W0 (n x n, overwritten) of a symmetric C
