@@ -9,15 +9,17 @@
 //   t = norm2(v); while t >= orth_tol and t < reorth_tol normv: normv = t, another pass with
 //   R(j,i) = po(pc(R(j,i)) + pc(r_j)), t = norm2(v)
 //   t < select_tol -> dropped; else q_i = po(pc(v) / pc(t)), R(i,i) = t.
-// Dots and norms are grid reductions in the compute type (per-CTA partial sums, the last CTA adds
-// them in a fixed order: deterministic); the updates are row-parallel and apply the j terms in order
-// with one rounding to the output type per term, as the MATLAB code does.  The while-loop decisions
-// need t on the host: one synchronisation per column and pass (the comparison path, not the hot one).
+// Bases in FP64 throughout are built in one cooperative launch (k_gs_coop).  With a narrower storage type the
+// column loop runs: dots and norms are grid reductions in the compute type (per-CTA partial sums, the last CTA
+// adds them in a fixed order: deterministic); the updates are row-parallel and apply the j terms in order with
+// one rounding to the output type per term, as the MATLAB code does; the while-loop decisions need t on the
+// host, one synchronisation per column and pass.
 // Q keeps the input's column positions (dropped columns zero) with select flags, like the Hessenberg
 // basis, so the solvers compact both the same way.
 #include <cmath>
 #include <vector>
 
+#include "grid_barrier.cuh"
 #include "ofrr_internal.cuh"
 
 namespace ofrr {
@@ -107,6 +109,369 @@ __global__ void __launch_bounds__(GS_T) k_gs_scale(int64_t m, const TO* __restri
   for (int64_t i = blockIdx.x * (int64_t)GS_T + threadIdx.x; i < m; i += (int64_t)gridDim.x * GS_T)
     q[i] = from_c<TO, TC>(div_rn(to_c<TC, TO>(v[i]), tc));
   if (blockIdx.x == 0 && threadIdx.x == 0) *Rii = (double)to_c<TC, TO>(*t);
+}
+
+// ---- FP64 bases in one cooperative launch ------------------------------------------------------------
+// The column loop above costs two launches per projection and a host synchronisation per column and pass:
+// 80.8 ms for 64 correlated columns of 8192 rows (4000 dependent dots).  Here one launch does the whole basis.
+//  * The rows are split over the CTAs of a resident grid; all of a column's decisions are taken by every CTA
+//    from the same reduced sums, so nothing returns to the host.
+//  * MGS's dots of one pass depend on each other only through Q'Q: r_j = q_j'v - sum_{l<j} (q_j'q_l) r_l, that is
+//    r = T Q'v with T = (I + strict lower(Q'Q))^-1, the inverse compact form of MGS (K. Swirydowicz, J. Langou,
+//    S. Ananthan, U. Yang, S. Thomas, "Low synchronization Gram-Schmidt and generalized minimal residual
+//    algorithms", Numer. Linear Algebra Appl. 28, 2021), which has MGS's error bounds.  T grows by one row per
+//    column.  So a pass needs one reduction instead of one per earlier column; CGS has r = Q'v.
+//  * One reduction after a pass gives v'v (the norm), Q'v (the next pass's dots, or the new row of Q'Q) and
+//    v'a_c for the columns still to come (their first dots, once divided by the norm): a column costs as many
+//    reductions as it takes passes.
+// Sums are in a fixed order (rows of a CTA, then CTAs), so results do not depend on the schedule.  The terms of
+// an update are summed by FMA before they are subtracted: fewer roundings than one per term.
+// A reduction takes two rounds through L2: every CTA writes its partial sums, value k is summed by one warp of
+// CTA k mod G, and all CTAs read the totals.
+// What bounds it: for 8192 x 64 (122 passes) a pass takes about 21,000 cycles: the dots, the update and T's
+// product 3,000 to 3,400 each (every FP64 warp instruction takes its sub-partition 64 cycles), the two rounds of
+// the reduction 7,000, and norm, scaling and the new row of T the rest.
+// Measured, call included, correlated columns: 8192 x 64 MGS 80.8 -> 1.43 ms, CGS -> 1.17 ms; 100000 x 80 MGS 5.7 ms
+// (its dots, read from L2, then take two thirds); 300 x 20 0.49 ms.
+constexpr int GC_T = 512;
+constexpr int GC_W = GC_T / 32;
+constexpr int GC_MAXN = 128;
+constexpr int GC_MAXG = 160;  // CTAs at most (152 SMs, rounded up to whole warps)
+
+struct GsCoop {
+  int64_t m, lda, ldq;
+  int n, classical, rows;  // rows per CTA
+  const double* A;
+  double* Q;
+  double* R;
+  int* sel;
+  double stol, otol, rtol;
+  double* partial;  // [G][n + 1]
+  double* total;    // [n + 1]
+  unsigned* ctr;    // two counters
+  int* err;
+};
+
+// XS: this CTA's rows of [Q(:, < i), A(:, >= i)] stay in shared memory (row-major); otherwise they are read
+// from global memory
+template <bool XS>
+__global__ void __launch_bounds__(GC_T) k_gs_coop(GsCoop P) {
+  extern __shared__ double gsm[];
+  const int n = P.n, K = n + 1, LD = n | 1, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int G = gridDim.x;
+  const int64_t row0 = (int64_t)blockIdx.x * P.rows;
+  const int nr = (int)max((int64_t)0, min((int64_t)P.rows, P.m - row0));
+  double* TH = gsm;                        // lower triangle: T; strict upper (l, c): q_l'a_c
+  double* s_v = TH + (size_t)n * LD;       // the CTA's rows of v
+  double* s_r = s_v + P.rows;              // projection coefficients
+  double* s_h = s_r + n;                   // dots of the pass
+  double* s_tot = s_h + n;                 // totals of the reduction
+  double* s_norm = s_tot + K;              // norms of the original columns
+  double* s_red = s_norm + n;              // scratch: max(16 n, 1024)
+  double* X = s_red + max(GC_W * n, 1024);  // XS: nr x n, row-major, leading dimension LD
+  __shared__ int s_sel[GC_MAXN];
+  __shared__ int s_ok;
+  __shared__ double s_vv, s_t;
+  // decisions are taken by one thread: an FP64 square root or compare on every warp would queue on the pipe
+  __shared__ int s_skip[GC_MAXN], s_dec;
+  const double* A = P.A + row0;
+  double* Q = P.Q + row0;
+
+  for (int e = tid; e < n * LD; e += GC_T) TH[e] = 0.0;
+  for (int c = tid; c < n; c += GC_T) s_sel[c] = 0;
+  if (XS)
+    for (int c = wid; c < n; c += GC_W)
+      for (int r = lane; r < nr; r += 32) X[(size_t)r * LD + c] = A[r + (int64_t)c * P.lda];
+  __syncthreads();
+
+  unsigned step = 0;
+  const int owners = min(K, G);
+  // s_red[0 .. K) -> s_tot[0 .. K), summed over the CTAs
+  auto reduce = [&]() -> bool {
+    ++step;
+    for (int k = tid; k < K; k += GC_T) __stcg(P.partial + (size_t)blockIdx.x * K + k, s_red[k]);
+    grid_arrive(P.ctr);
+    if ((int)blockIdx.x < owners) {
+      if (!grid_wait(P.ctr, (unsigned)G * step, &s_ok, P.err, 51)) return false;
+      for (int k = blockIdx.x + G * wid; k < K; k += G * GC_W) {
+        double v[GC_MAXG / 32], s = 0.0;  // all loads in flight together: one L2 latency
+#pragma unroll
+        for (int u = 0; u < GC_MAXG / 32; ++u)
+          v[u] = (lane + 32 * u < G) ? __ldcg(P.partial + (size_t)(lane + 32 * u) * K + k) : 0.0;
+#pragma unroll
+        for (int u = 0; u < GC_MAXG / 32; ++u) s += v[u];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) __stcg(P.total + k, s);
+      }
+      grid_arrive(P.ctr + 1);
+    }
+    if (!grid_wait(P.ctr + 1, (unsigned)owners * step, &s_ok, P.err, 52)) return false;
+    for (int k = tid; k < K; k += GC_T) s_tot[k] = __ldcg(P.total + k);
+    __syncthreads();
+    return true;
+  };
+  // s_red[c] = this CTA's part of x_c'v (x_c'x_c with self) for every column c, x_c = q_c for c < i and a_c
+  // otherwise; s_red[n] = v'v
+  auto dots = [&](int i, bool self) {
+    if (XS) {
+      // lanes over columns, row groups over warps; the last warp takes v'v
+      const int cg = (n + 31) / 32, rg = (GC_W - 1) / cg, g = wid / cg, c = (wid % cg) * 32 + lane;
+      double acc = 0.0;
+      if (wid < rg * cg) {
+        const int per = (nr + rg - 1) / rg, ra = g * per, rb = min(nr, ra + per);
+        if (c < n)
+          for (int r = ra; r < rb; ++r) {
+            const double x = X[(size_t)r * LD + c];
+            acc = fma(x, self ? x : s_v[r], acc);
+          }
+      } else if (wid == GC_W - 1 && !self) {
+        for (int r = lane; r < nr; r += 32) acc = fma(s_v[r], s_v[r], acc);
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+        if (lane == 0) s_vv = acc;
+      }
+      __syncthreads();  // the scratch may still hold an update's partial sums
+      if (wid < rg * cg && c < n) s_red[g * n + c] = acc;
+      __syncthreads();
+      double s = 0.0;
+      if (tid < n)
+        for (int x = 0; x < rg; ++x) s += s_red[x * n + tid];
+      __syncthreads();
+      if (tid < n) s_red[tid] = s;
+      if (tid == 0) s_red[n] = self ? 0.0 : s_vv;
+    } else {
+      __syncthreads();
+      for (int c = wid; c < K; c += GC_W) {
+        double acc = 0.0;
+        if (c == n) {
+          if (!self)
+            for (int r = lane; r < nr; r += 32) acc = fma(s_v[r], s_v[r], acc);
+        } else if (self || c > i || s_sel[c]) {
+          const double* x = (c < i) ? Q + (int64_t)c * P.ldq : A + (int64_t)c * P.lda;
+          double a1 = 0.0;
+          int r = lane;
+          for (; r + 96 < nr; r += 128) {
+            const double x0 = x[r], x1 = x[r + 32], x2 = x[r + 64], x3 = x[r + 96];
+            acc = fma(x0, self ? x0 : s_v[r], acc);
+            a1 = fma(x1, self ? x1 : s_v[r + 32], a1);
+            acc = fma(x2, self ? x2 : s_v[r + 64], acc);
+            a1 = fma(x3, self ? x3 : s_v[r + 96], a1);
+          }
+          for (; r < nr; r += 32) {
+            const double x0 = x[r];
+            acc = fma(x0, self ? x0 : s_v[r], acc);
+          }
+          acc += a1;
+        }
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+        if (lane == 0) s_red[c] = acc;
+      }
+    }
+    __syncthreads();
+  };
+  // out[j] = sum over k of rows j0 .. of TH, j < i: columns of the lower triangle (mode 0: s_r = T s_h) or
+  // its rows (mode 1: s_r(l) = sum_k s_h(k) T(k, l))
+  auto apply_t = [&](int i, int mode) {
+    const int jg = (i + 31) / 32, lg = GC_W / jg, g = wid / jg, j = (wid % jg) * 32 + lane;
+    double acc = 0.0;
+    if (wid < lg * jg) {
+      const int per = (i + lg - 1) / lg, la = g * per, lb = min(i, la + per);
+      if (j < i)
+        for (int l = la; l < lb; ++l) {
+          if (mode == 0 ? l <= j : l >= j) acc = fma(TH[mode == 0 ? j * LD + l : l * LD + j], s_h[l], acc);
+        }
+      if (j < i) s_red[g * i + j] = acc;
+    }
+    __syncthreads();
+    for (int x = tid; x < i; x += GC_T) {
+      double s = 0.0;
+      for (int y = 0; y < lg; ++y) s += s_red[y * i + x];
+      s_r[x] = s_sel[x] ? s : 0.0;
+    }
+    __syncthreads();
+  };
+  // v -= sum_{j < i} r_j q_j
+  auto update = [&](int i) {
+    if (XS) {
+      const int rgs = (nr + 31) / 32, jgs = max(1, GC_W / max(rgs, 1));
+      for (int item = wid; item < rgs * jgs; item += GC_W) {
+        const int g = item / max(rgs, 1), r = (item % max(rgs, 1)) * 32 + lane;
+        const int per = (i + jgs - 1) / jgs, ja = g * per, jb = min(i, ja + per);
+        double acc = 0.0;
+        if (r < nr)
+          for (int j = ja; j < jb; ++j) acc = fma(s_r[j], X[(size_t)r * LD + j], acc);
+        if (jgs == 1) {
+          if (r < nr) s_v[r] -= acc;
+        } else if (r < nr) {
+          s_red[g * nr + r] = acc;
+        }
+      }
+      __syncthreads();
+      if (jgs > 1) {
+        for (int r = tid; r < nr; r += GC_T) {
+          double s = 0.0;
+          for (int g = 0; g < jgs; ++g) s += s_red[g * nr + r];
+          s_v[r] -= s;
+        }
+        __syncthreads();
+      }
+    } else {
+      for (int r = tid; r < nr; r += GC_T) {
+        double acc = 0.0;
+        int j = 0;
+        for (; j + 8 <= i; j += 8) {
+          double q[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) q[u] = s_sel[j + u] ? Q[r + (int64_t)(j + u) * P.ldq] : 0.0;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) acc = fma(s_r[j + u], q[u], acc);
+        }
+        for (; j < i; ++j) acc = fma(s_r[j], s_sel[j] ? Q[r + (int64_t)j * P.ldq] : 0.0, acc);
+        s_v[r] -= acc;
+      }
+      __syncthreads();
+    }
+  };
+  auto drop = [&](int i) {  // column i leaves the basis
+    for (int r = tid; r < nr; r += GC_T) {
+      Q[r + (int64_t)i * P.ldq] = 0.0;
+      if (XS) X[(size_t)r * LD + i] = 0.0;
+    }
+    if (blockIdx.x == 0 && tid == 0) P.sel[i] = 0;
+    __syncthreads();
+  };
+
+  dots(0, true);
+  if (!reduce()) return;
+  for (int c = tid; c < n; c += GC_T) {
+    s_norm[c] = sqrt(s_tot[c]);
+    s_skip[c] = s_norm[c] < P.stol;
+  }
+  __syncthreads();
+  int nsel = 0;
+  for (int i = 0; i < n; ++i) {
+    double normv = s_norm[i];  // thread 0's copy decides
+    if (s_skip[i]) {
+      drop(i);
+      continue;
+    }
+    for (int r = tid; r < nr; r += GC_T) s_v[r] = XS ? X[(size_t)r * LD + i] : A[r + (int64_t)i * P.lda];
+    for (int l = tid; l < i; l += GC_T) s_h[l] = TH[l * LD + i];  // q_l'a_i (0 for dropped columns)
+    __syncthreads();
+    // (at most 64 further passes: the reference loops until the norm stops dropping, which takes 1-2)
+    for (int pass = 0; pass <= 64; ++pass) {
+      if (nsel > 0) {
+        if (P.classical) {
+          for (int l = tid; l < i; l += GC_T) s_r[l] = s_h[l];
+          __syncthreads();
+        } else {
+          apply_t(i, 0);
+        }
+        update(i);
+        if (blockIdx.x == 0)
+          for (int j = tid; j < i; j += GC_T)
+            if (s_sel[j]) P.R[j + (int64_t)i * n] = pass ? P.R[j + (int64_t)i * n] + s_r[j] : s_r[j];
+      }
+      dots(i, false);
+      if (!reduce()) return;
+      if (tid == 0) {
+        const double t = sqrt(s_tot[n]);
+        const bool again = pass < 64 && P.rtol >= 0 && t >= P.otol && t < P.rtol * normv;
+        s_dec = again ? 2 : (t < P.stol ? 1 : 0);
+        s_t = t;
+        normv = t;
+      }
+      for (int l = tid; l < i; l += GC_T) s_h[l] = s_sel[l] ? s_tot[l] : 0.0;
+      __syncthreads();
+      if (s_dec != 2) break;
+    }
+    const double t = s_t;
+    if (s_dec == 1) {
+      drop(i);
+      continue;
+    }
+    for (int r = tid; r < nr; r += GC_T) {
+      const double q = s_v[r] / t;
+      Q[r + (int64_t)i * P.ldq] = q;
+      if (XS) X[(size_t)r * LD + i] = q;
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+      P.sel[i] = 1;
+      P.R[i + (int64_t)i * n] = t;
+    }
+    // the first dots of the columns to come, and the new row of T: T(i, l) = -sum_k (q_i'q_k) T(k, l)
+    for (int c = tid; c < n; c += GC_T) {
+      if (c > i) TH[i * LD + c] = s_tot[c] / t;
+      if (c < i) s_h[c] /= t;
+    }
+    __syncthreads();
+    if (!P.classical && nsel > 0) {
+      apply_t(i, 1);
+      for (int l = tid; l < i; l += GC_T) TH[i * LD + l] = -s_r[l];
+    }
+    if (tid == 0) {
+      TH[i * LD + i] = 1.0;
+      s_sel[i] = 1;
+    }
+    ++nsel;
+    __syncthreads();
+  }
+}
+
+// shared memory of k_gs_coop
+size_t gs_coop_smem(int n, int rows, bool xs) {
+  const int LD = n | 1;
+  return sizeof(double) * ((size_t)n * LD + rows + 4 * (size_t)n + 1 + std::max(GC_W * n, 1024) +
+                           (xs ? (size_t)rows * LD : 0));
+}
+
+// *done = false: the shape does not fit (or the grid cannot be resident at once), the column loop takes it
+int gs_coop(ofrr_ctx* ctx, bool classical, int64_t m, int64_t n, const double* A, int64_t lda, double* Q, int64_t ldq,
+            double stol, double otol, double rtol, double* R, int* select_dev, bool* done) {
+  *done = false;
+  if (n > GC_MAXN) return OFRR_SUCCESS;
+  // 32 rows or more per CTA; one CTA per SM
+  const int G = (int)std::min<int64_t>(152, (m + 31) / 32);
+  const int64_t rows = (m + G - 1) / G;
+  constexpr size_t kMax = 220 * 1024;
+  if (rows > 16384) return OFRR_SUCCESS;
+  const bool xs = gs_coop_smem((int)n, (int)rows, true) <= kMax;
+  const size_t smem = gs_coop_smem((int)n, (int)rows, xs);
+  if (smem > kMax) return OFRR_SUCCESS;
+  WsScope scope(ctx);
+  int st = OFRR_SUCCESS;
+  GsCoop P{};
+  P.partial = ws_get<double>(ctx, (size_t)G * (n + 1), &st);
+  P.total = ws_get<double>(ctx, (size_t)n + 1, &st);
+  P.ctr = ws_get<unsigned>(ctx, 2, &st);
+  if (!P.partial || !P.total || !P.ctr) return st;
+  P.m = m;
+  P.n = (int)n;
+  P.lda = lda;
+  P.ldq = ldq;
+  P.classical = classical ? 1 : 0;
+  P.rows = (int)rows;
+  P.A = A;
+  P.Q = Q;
+  P.R = R;
+  P.sel = select_dev;
+  P.stol = stol;
+  P.otol = otol;
+  P.rtol = rtol;
+  P.err = ctx->dev_flags + kFlagHessWait;
+  OFRR_CUDA(cudaMemsetAsync(P.ctr, 0, 2 * sizeof(unsigned), ctx->stream));
+  OFRR_CUDA(cudaMemsetAsync(R, 0, sizeof(double) * n * n, ctx->stream));
+  void* args[] = {&P};
+  const void* f = xs ? (const void*)k_gs_coop<true> : (const void*)k_gs_coop<false>;
+  OFRR_TRY(allow_dynamic_smem(f));
+  const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3((unsigned)G), dim3(GC_T), args, smem, ctx->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    (void)cudaGetLastError();
+    return OFRR_SUCCESS;
+  }
+  OFRR_CUDA(e);
+  OFRR_LAUNCHED(ctx, "k_gs_coop");
+  *done = true;
+  return OFRR_SUCCESS;
 }
 
 template <class TO, class TC>
@@ -215,6 +580,14 @@ int gs_basis_impl(ofrr_ctx* ctx, bool classical, ofrr_dtype tin, ofrr_dtype tout
   // the tolerances are compared in the output precision, as mgs.m:141-152 casts them
   const double s_t = round_to(tout, stol), o_t = round_to(tout, std::isnan(orth_tol) ? e : orth_tol),
                r_t = round_to(tout, std::isnan(reorth_tol) ? 1.0 / std::sqrt(2.0) : reorth_tol);
+  // FP64 throughout: one cooperative launch.  With a narrower storage type every term of an update is rounded
+  // to it and the next dot sees that rounding, so those bases keep the column loop's order of operations.
+  if (tout == OFRR_F64 && tc == OFRR_F64) {
+    bool done = false;
+    OFRR_TRY(gs_coop(ctx, classical, m, n, (const double*)Ain, ldin, (double*)Q, ldq, s_t, o_t, r_t, R_dev,
+                     select_dev, &done));
+    if (done) return OFRR_SUCCESS;
+  }
   OFRR_DISPATCH_STORAGE(tout, TO, OFRR_DISPATCH_COMPUTE(tc, TC, {
     OFRR_TRY((gs_run<TO, TC>(ctx, classical, m, n, (const TO*)Ain, ldin, (TO*)Q, ldq, s_t, o_t, r_t, R_dev,
                              select_dev)));
