@@ -462,9 +462,9 @@ int quant_e4m3(ofrr_ctx* ctx, ofrr_dtype tin, int64_t K, int64_t M, const void* 
                int64_t ld8, float* scale);
 int gemm_e4m3_tn(ofrr_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A8, int64_t lda8, const float* sa,
                  const void* B8, int64_t ldb8, const float* sb, float* C, int64_t ldc);
-// A' as CSR (row pointers, rows sorted within each column, every value copy present in A), in ctx's
-// current workspace scope; deterministic
-int csr_transpose_impl(ofrr_ctx* ctx, const ofrr_csr* A, ofrr_csr* At);
+// A' as CSR (row pointers, rows sorted within each column, the value copies of the mask `want` present in A:
+// 1 FP64, 2 FP32, 4 FP16), in ctx's current workspace scope; deterministic
+int csr_transpose_impl(ofrr_ctx* ctx, const ofrr_csr* A, ofrr_csr* At, int want = 7);
 int cast_transpose_impl(ofrr_ctx* ctx, ofrr_dtype tin, ofrr_dtype tout, int64_t m, int64_t n, const void* in,
                         int64_t ldin, void* out, int64_t ldout);
 int cast_impl(ofrr_ctx* ctx, ofrr_dtype tin, ofrr_dtype tout, int64_t m, int64_t n, const void* in,

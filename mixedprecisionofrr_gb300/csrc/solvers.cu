@@ -633,7 +633,6 @@ extern "C" int ofrr_rr_eig(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_opt
   const Precisions P = precisions_of(opt);
   WsScope scope(ctx);
   Op op{A};
-  OFRR_TRY(op.prepare_csr_t(ctx));
   double* d;
   OFRR_TRY(dmalloc(ctx, &d, (size_t)ncols));
   // eig_rr on V (type p_output): pmc = p_rr_compute, pmo = p_rr_output, A-matvec in (p_compute, p_output)
@@ -977,7 +976,6 @@ extern "C" int ofrr_rr_svd(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_opt
   const Precisions P = precisions_of(opt);
   WsScope scope(ctx);
   Op op{A};
-  OFRR_TRY(op.prepare_csr_t(ctx));
   double* d;
   OFRR_TRY(dmalloc(ctx, &d, (size_t)ncols));
   const int b = (int)ncols;
@@ -1817,7 +1815,6 @@ static int si_eig_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_options
   WsScope scope(ctx);
   int st = OFRR_SUCCESS;
   Op op{A};
-  OFRR_TRY(op.prepare_csr_t(ctx));
   const int nev = std::min(opt->nev > 0 ? opt->nev : b0, b0);
   PhaseState S;
   S.b = b0;
