@@ -30,22 +30,60 @@ template <> struct CsrVals<float> {
 constexpr int kSpmmRows = 256;
 constexpr int kSpmmCap = 2048;  // staged nonzeros per CTA (8 per row on average)
 
-template <class TX, class TC, class TY, int RC>
-__global__ void __launch_bounds__(kSpmmRows) k_csrmm_n(int64_t nrows, const int32_t* __restrict__ indptr,
+// Products of one row with RC columns of X, nonzeros in order.  U nonzeros' entries of X are loaded ahead of the
+// dependent sums, so that U RC loads of a thread are in flight.  Offsets of up to 32 bits (OFF32) leave the columns'
+// bases in uniform registers: one instruction per load instead of three.
+template <class TX, class TC, int RC, int U, bool OFF32, bool FULL, class IDX, class VAL>
+__device__ __forceinline__ void csrmm_row(int32_t p0, int32_t p1, IDX idx, VAL val, const TX* __restrict__ Xc,
+                                          int64_t ldx, int nr, TC (&acc)[RC]) {
+  for (int32_t p = p0; __any_sync(0xffffffffu, p < p1); p += U) {
+    TX x[U][RC];
+    TC a[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool ok = p + u < p1;
+      const int32_t col = ok ? idx(p + u) : 0;  // past the row: column 0, read and not used
+      a[u] = ok ? val(p + u) : TC(0);
+#pragma unroll
+      for (int r = 0; r < RC; ++r) {
+        const TX* base = Xc + r * ldx;
+        const TX* at = OFF32 ? reinterpret_cast<const TX*>(reinterpret_cast<const char*>(base) +
+                                                           (uint32_t)col * (uint32_t)sizeof(TX))
+                             : base + col;
+        x[u][r] = (FULL || r < nr) ? __ldg(at) : TX(0);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      // an FP64 FMA occupies its 1/64-rate pipe even where it is predicated off: leave with the whole warp
+      if (u > 0 && !__any_sync(0xffffffffu, p + u < p1)) break;
+      if (p + u < p1) {
+#pragma unroll
+        for (int r = 0; r < RC; ++r) acc[r] = fma(a[u], to_c<TC, TX>(x[u][r]), acc[r]);
+      }
+    }
+  }
+}
+
+template <class TX, class TC, class TY, int RC, int U, int MB, bool OFF32>
+__global__ void __launch_bounds__(kSpmmRows, MB) k_csrmm_n(int64_t nrows, const int32_t* __restrict__ indptr,
                                                        const int32_t* __restrict__ indices,
                                                        const TC* __restrict__ vals, int64_t nrhs,
                                                        const TX* __restrict__ X, int64_t ldx, TY* __restrict__ Y,
-                                                       int64_t ldy, int nchunks) {
+                                                       int64_t ldy, int nsplit, int64_t per) {
   __shared__ TC s_val[kSpmmCap];
   __shared__ int32_t s_idx[kSpmmCap];
-  // CTA b: row block b / nchunks, right-hand sides [RC (b % nchunks), ...) -- the CTAs of one row block are
+  // CTA b: row block b / nsplit, right-hand sides [per (b % nsplit), ...) -- the CTAs of one row block are
   // adjacent, so the block's nonzeros are read from HBM once and from L2 by the others
-  const int64_t r0 = (int64_t)(blockIdx.x / nchunks) * kSpmmRows;
-  const int64_t cbeg = (nchunks > 1) ? (int64_t)(blockIdx.x % nchunks) * RC : 0;
-  const int64_t cend = (nchunks > 1) ? min(nrhs, cbeg + RC) : nrhs;
+  const int64_t r0 = (int64_t)(blockIdx.x / nsplit) * kSpmmRows;
+  const int64_t cbeg = (int64_t)(blockIdx.x % nsplit) * per;
+  const int64_t cend = min(nrhs, cbeg + per);
   if (r0 >= nrows) return;
   const int64_t rend = min(nrows, r0 + kSpmmRows);
+  const int64_t row = r0 + threadIdx.x;
+  const bool have = row < rend;
   const int32_t pbase = __ldg(indptr + r0), pend = __ldg(indptr + rend);
+  const int32_t p0 = have ? __ldg(indptr + row) : 0, p1 = have ? __ldg(indptr + row + 1) : 0;
   const bool staged = (pend - pbase) <= kSpmmCap;
   if (staged) {
     for (int32_t e = threadIdx.x; e < pend - pbase; e += kSpmmRows) {
@@ -54,24 +92,24 @@ __global__ void __launch_bounds__(kSpmmRows) k_csrmm_n(int64_t nrows, const int3
     }
   }
   __syncthreads();
-  const int64_t row = r0 + threadIdx.x;
-  if (row >= rend) return;
-  const int32_t p0 = __ldg(indptr + row), p1 = __ldg(indptr + row + 1);
   for (int64_t c0 = cbeg; c0 < cend; c0 += RC) {
     TC acc[RC];
 #pragma unroll
     for (int r = 0; r < RC; ++r) acc[r] = TC(0);
-    for (int32_t p = p0; p < p1; ++p) {
-      const int64_t col = staged ? s_idx[p - pbase] : __ldg(indices + p);
-      const TC a = staged ? s_val[p - pbase] : __ldg(vals + p);
+    const int nr = (int)min((int64_t)RC, cend - c0);
+    const TX* Xc = X + c0 * ldx;
+    auto si = [&](int32_t p) { return s_idx[p - pbase]; };
+    auto sv = [&](int32_t p) { return s_val[p - pbase]; };
+    auto gi = [&](int32_t p) { return __ldg(indices + p); };
+    auto gv = [&](int32_t p) { return __ldg(vals + p); };
+    if (staged && nr == RC) csrmm_row<TX, TC, RC, U, OFF32, true>(p0, p1, si, sv, Xc, ldx, nr, acc);
+    else if (staged) csrmm_row<TX, TC, RC, U, OFF32, false>(p0, p1, si, sv, Xc, ldx, nr, acc);
+    else csrmm_row<TX, TC, RC, 1, OFF32, false>(p0, p1, gi, gv, Xc, ldx, nr, acc);
+    if (have) {
 #pragma unroll
-      for (int r = 0; r < RC; ++r) {
-        if (c0 + r < cend) acc[r] = fma(a, to_c<TC, TX>(X[col + (c0 + r) * ldx]), acc[r]);
-      }
+      for (int r = 0; r < RC; ++r)
+        if (r < nr) Y[row + (c0 + r) * ldy] = from_c<TY, TC>(acc[r]);
     }
-#pragma unroll
-    for (int r = 0; r < RC; ++r)
-      if (c0 + r < cend) Y[row + (c0 + r) * ldy] = from_c<TY, TC>(acc[r]);
   }
 }
 
@@ -242,24 +280,27 @@ int csr_transpose_impl(ofrr_ctx* ctx, const ofrr_csr* A, ofrr_csr* At, int want)
 static int csrmm_n(ofrr_ctx* ctx, const ofrr_csr* A, ofrr_dtype tx, ofrr_dtype tc, ofrr_dtype ty, int64_t nrhs,
                    const void* X, int64_t ldx, void* Y, int64_t ldy) {
   const int64_t blocks = (A->nrows + kSpmmRows - 1) / kSpmmRows;
-  // many right-hand sides: one CTA per (row block, 8-column chunk), for more loads in flight per SM
-  const int nchunks = (nrhs > 8) ? (int)((nrhs + 7) / 8) : 1;
-  if (blocks * nchunks > 0x7fffffffLL) return OFRR_ERR_BLAS_INVALID_SIZE;
-  const unsigned grid = (unsigned)(blocks * nchunks);
+  const bool off32 = A->ncols * (int64_t)dtype_size(tx) <= 0xffffffffLL;
+  const int rc = !off32 ? 8 : nrhs == 1 ? 1 : nrhs <= 4 ? 4 : 8;
+  // a CTA takes as many column chunks as leave the device about 16 CTAs per SM
+  const int64_t nchunks = (nrhs + rc - 1) / rc;
+  const int64_t split = std::min<int64_t>(nchunks, std::max<int64_t>(1, (152 * 16 + blocks - 1) / blocks));
+  const int64_t per = (nchunks + split - 1) / split * rc;
+  const int nsplit = (int)((nrhs + per - 1) / per);
+  if (blocks * nsplit > 0x7fffffffLL) return OFRR_ERR_BLAS_INVALID_SIZE;
+  const unsigned grid = (unsigned)(blocks * nsplit);
   OFRR_DISPATCH_COMPUTE(tc, TC, {
     const TC* vals = CsrVals<TC>::get(A);
     if (!vals) return OFRR_ERR_INVALID_ARGUMENT;
+    // CTAs per SM the registers are kept to: FP64 is bound by its pipe and keeps more of a row in registers
+    constexpr int MB = sizeof(TC) == 8 ? 6 : 8;
     OFRR_DISPATCH_STORAGE(tx, TX, OFRR_DISPATCH_STORAGE(ty, TY, {
-      if (nrhs == 1) {
-        k_csrmm_n<TX, TC, TY, 1><<<grid, kSpmmRows, 0, ctx->stream>>>(A->nrows, A->indptr, A->indices, vals, nrhs,
-                                                                      (const TX*)X, ldx, (TY*)Y, ldy, nchunks);
-      } else if (nrhs <= 4) {
-        k_csrmm_n<TX, TC, TY, 4><<<grid, kSpmmRows, 0, ctx->stream>>>(A->nrows, A->indptr, A->indices, vals, nrhs,
-                                                                      (const TX*)X, ldx, (TY*)Y, ldy, nchunks);
-      } else {
-        k_csrmm_n<TX, TC, TY, 8><<<grid, kSpmmRows, 0, ctx->stream>>>(A->nrows, A->indptr, A->indices, vals, nrhs,
-                                                                      (const TX*)X, ldx, (TY*)Y, ldy, nchunks);
-      }
+      auto k = off32 ? (rc == 1   ? k_csrmm_n<TX, TC, TY, 1, 4, 8, true>
+                        : rc == 4 ? k_csrmm_n<TX, TC, TY, 4, 1, MB, true>
+                                  : k_csrmm_n<TX, TC, TY, 8, 1, MB, true>)
+                     : k_csrmm_n<TX, TC, TY, 8, 1, MB, false>;
+      k<<<grid, kSpmmRows, 0, ctx->stream>>>(A->nrows, A->indptr, A->indices, vals, nrhs, (const TX*)X, ldx, (TY*)Y, ldy,
+                                             nsplit, per);
       OFRR_LAUNCHED(ctx, "k_csrmm_n");
     }));
   });
