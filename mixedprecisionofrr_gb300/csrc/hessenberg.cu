@@ -27,9 +27,10 @@ __global__ void __launch_bounds__(256) k_hess_col(int64_t m, int n, int i, TO* _
                                                    unsigned int* __restrict__ counter, double select_tol,
                                                    int scale_prev, int* __restrict__ stop, int stage_L,
                                                    TO* __restrict__ snap = nullptr) {
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   TC* s_r = reinterpret_cast<TC*>(smem_raw);                       // n entries
-  TO* s_x = reinterpret_cast<TO*>(s_r + n);                        // n entries
+  // n entries (aligned: FP32 arithmetic with FP64 storage leaves an odd n at a multiple of four bytes)
+  TO* s_x = reinterpret_cast<TO*>(((uintptr_t)(s_r + n) + 15) & ~(uintptr_t)15);
   int* s_sel = reinterpret_cast<int*>(((uintptr_t)(s_x + n) + 15) & ~(uintptr_t)15);  // n entries
   __shared__ ArgMax red[32];
   __shared__ bool s_last;
@@ -196,7 +197,7 @@ static int hess_run(ofrr_ctx* ctx, int64_t m, int n, TO* Q, int64_t ldq, double 
   OFRR_TRY(fill_zero(ctx, R, sizeof(double) * (size_t)n * n));
   OFRR_TRY(fill_zero(ctx, pivrows, sizeof(TO) * (size_t)n * n));
   const int stage = ((size_t)n * n * sizeof(TO) <= 96 * 1024) ? 1 : 0;
-  size_t smem = (size_t)n * (sizeof(TC) + sizeof(TO)) + 16 + (size_t)n * sizeof(int);
+  size_t smem = (size_t)n * (sizeof(TC) + sizeof(TO)) + 32 + (size_t)n * sizeof(int);
   if (stage) smem += 16 + (size_t)n * n * sizeof(TO);
   if (smem > 48 * 1024) {
     OFRR_TRY(allow_smem(k_hess_col<TO, TC>));
@@ -245,7 +246,7 @@ static int kry_col(ofrr_ctx* ctx, int64_t m, int nb, int i, TO* V, int64_t ldv, 
   ArgMax* partial = ws_get<ArgMax>(ctx, grid, &st);
   if (!partial) return st;
   const int stage = ((size_t)nb * nb * sizeof(TO) <= 96 * 1024) ? 1 : 0;
-  size_t smem = (size_t)nb * (sizeof(TC) + sizeof(TO)) + 16 + (size_t)nb * sizeof(int);
+  size_t smem = (size_t)nb * (sizeof(TC) + sizeof(TO)) + 32 + (size_t)nb * sizeof(int);
   if (stage) smem += 16 + (size_t)nb * nb * sizeof(TO);
   if (smem > 48 * 1024) {
     OFRR_TRY(allow_smem(k_hess_col<TO, TC>));
@@ -372,7 +373,7 @@ int hess_run_noalloc(ofrr_ctx* sctx, unsigned char* scratch, int64_t m, int n, T
   OFRR_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned int), sctx->stream));
   OFRR_TRY(fill_zero(sctx, R, sizeof(double) * (size_t)n * n));
   OFRR_TRY(fill_zero(sctx, pivrows, sizeof(TO) * (size_t)n * n));
-  const size_t smem = (size_t)n * (sizeof(TC) + sizeof(TO)) + 16 + (size_t)n * sizeof(int);
+  const size_t smem = (size_t)n * (sizeof(TC) + sizeof(TO)) + 32 + (size_t)n * sizeof(int);
   if (smem > 48 * 1024) return OFRR_ERR_BLAS_INVALID_SIZE;
   for (int i = 0; i < n; ++i) {
     k_hess_col<TO, TC><<<grid, block, smem, sctx->stream>>>(m, n, i, Q, ldq, select, perm, pivrows, pvals, R, partial,

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(HB_B * 32) k_hess_blockcoef(int n, int c0, int
                                                               int64_t ldq, const int* __restrict__ select,
                                                               const int* __restrict__ perm, TC* __restrict__ rcoef,
                                                               double* __restrict__ R) {
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nb = c1 - c0;
   TO* s_L = reinterpret_cast<TO*>(smem_raw);                                               // c0 x c0
   TO* s_x = s_L + (size_t)c0 * c0;                                                          // HB_B x c0
@@ -179,7 +179,7 @@ template <class TO, class TC, bool FAST>
 __global__ void __launch_bounds__(HB_UT) k_hess_blockupd(int64_t m, int c0, int c1, TO* __restrict__ Q, int64_t ldq,
                                                          const int* __restrict__ select,
                                                          const TC* __restrict__ rcoef) {
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   TC* s_r = reinterpret_cast<TC*>(smem_raw);                // HB_CG x c0
   int* s_sel = reinterpret_cast<int*>(s_r + HB_CG * c0);   // c0
   const int tid = threadIdx.x;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(HB_T) k_hess_inblock(int64_t m, int n, int c0,
   constexpr uint32_t CB = sizeof(HbCand<TO>);
   constexpr int NCH = (int)(CB / 16);  // 16-byte chunks per candidate
   static_assert(CB % 16 == 0, "candidates move in 16-byte stores");
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   TO* s_blk = reinterpret_cast<TO*>(smem_raw);  // HB_B columns x RR rows (column t at t * RR)
   __shared__ HbCand<TO> s_recv[2][HB_CL_MAX];   // candidates of column t in [t & 1][source rank]
   __shared__ HbCand<TO> s_send;                 // this CTA's candidate, staged for the stores

@@ -749,7 +749,7 @@ constexpr int kSignMaxN = 96;
 template <class T>
 __global__ void __launch_bounds__(256) k_sign_newton(int n, double* __restrict__ Xg, int maxit, double tol,
                                                      int* __restrict__ flag) {
-  extern __shared__ unsigned char sgn_raw[];
+  extern __shared__ __align__(16) unsigned char sgn_raw[];
   T* X = reinterpret_cast<T*>(sgn_raw);  // n x n, column-major
   T* Y = X + (size_t)n * n;              // its inverse (Gauss-Jordan in place)
   __shared__ int piv[kSignMaxN];

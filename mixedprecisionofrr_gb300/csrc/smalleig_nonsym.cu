@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(32) k_nonsym_eig(int nn, const double* __restr
                                                        double* __restrict__ wr, double* __restrict__ wi,
                                                        double* __restrict__ X, int* __restrict__ flag,
                                                        int pair_imag) {
-  extern __shared__ unsigned char sm_raw[];
+  extern __shared__ __align__(16) unsigned char sm_raw[];
   T* sm = reinterpret_cast<T*>(sm_raw);
   const int ld = nn + 1;
   T* H = sm;             // n x n (row i, column j at i + j * ld)
