@@ -212,6 +212,8 @@ static int hess_run(ofrr_ctx* ctx, int64_t m, int n, TO* Q, int64_t ldq, double 
   return OFRR_SUCCESS;
 }
 
+int hess_run_coop(ofrr_ctx* ctx, ofrr_dtype tout, ofrr_dtype tc, int64_t m, int64_t n, void* Q, int64_t ldq,
+                  double select_tol, double* R, int* select, int* perm, bool fast, bool* done);
 int hess_run_blocked(ofrr_ctx* ctx, ofrr_dtype tout, ofrr_dtype tc, int64_t m, int64_t n, void* Q, int64_t ldq,
                      double select_tol, double* R, int* select, int* perm, bool fast, bool* done);
 
@@ -225,8 +227,11 @@ int hessenberg_impl(ofrr_ctx* ctx, ofrr_dtype tin, ofrr_dtype tout, ofrr_dtype t
   if (A == Q && (tin != tout || lda != ldq)) return OFRR_ERR_INVALID_ARGUMENT;
   if (A != Q) OFRR_TRY(cast_impl(ctx, tin, tout, m, n, A, lda, Q, ldq));
   WsScope scope(ctx);
-  // blocked cluster schedule (hessenberg_blocked.cu) when the block fits on chip, else per column
+  // one cooperative launch (hessenberg_coop.cu) when the whole basis fits the SMs' shared memory, the blocked
+  // cluster schedule (hessenberg_blocked.cu) when a block of columns does, else per column
   bool done = false;
+  OFRR_TRY(hess_run_coop(ctx, tout, tc, m, n, Q, ldq, select_tol, R_dev, select_dev, perm_dev, fast, &done));
+  if (done) return OFRR_SUCCESS;
   OFRR_TRY(hess_run_blocked(ctx, tout, tc, m, n, Q, ldq, select_tol, R_dev, select_dev, perm_dev, fast, &done));
   if (done) return OFRR_SUCCESS;
   OFRR_DISPATCH_STORAGE(tout, TO, OFRR_DISPATCH_COMPUTE(tc, TC, {

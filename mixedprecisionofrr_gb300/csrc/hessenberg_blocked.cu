@@ -53,7 +53,7 @@ __device__ __forceinline__ float mul_recip(float x, float y) { return __fmul_rn(
 // shuffle from its owner, then every later entry is updated; the same roundings as the shared-memory
 // form (each update rounded to the storage type).
 template <int NR, class TO, class TC, bool FAST>
-__device__ __forceinline__ void blockcoef_subst(int c0, int n, int warp, int lane, const TO* x, const TO* s_L,
+__device__ __forceinline__ void blockcoef_subst(int c0, int t0, int n, int warp, int lane, const TO* x, const TO* s_L,
                                                 const int* s_sel, TC* r, double* R) {
   TC xv[NR];
   bool sv[NR];
@@ -72,7 +72,7 @@ __device__ __forceinline__ void blockcoef_subst(int c0, int n, int warp, int lan
       const TC rc = __shfl_sync(0xffffffffu, xv[q], jl);
       if (lane == 0) {
         r[j] = selj ? rc : TC(0);
-        R[j + (int64_t)(c0 + warp) * n] = selj ? to_c<double, TC>(rc) : 0.0;
+        R[j + (int64_t)(t0 + warp) * n] = selj ? to_c<double, TC>(rc) : 0.0;
       }
       if (!selj) continue;
 #pragma unroll
@@ -85,14 +85,16 @@ __device__ __forceinline__ void blockcoef_subst(int c0, int n, int warp, int lan
   }
 }
 
-// ---- step 0: coefficients of the block columns against the final columns [0, c0) -----------------
+// ---- step 0: coefficients of the block columns [c0, c1) against the final columns [0, c0), HB_B columns per CTA ----
 template <class TO, class TC, bool FAST>
 __global__ void __launch_bounds__(HB_B * 32) k_hess_blockcoef(int n, int c0, int c1, const TO* __restrict__ Q,
                                                               int64_t ldq, const int* __restrict__ select,
                                                               const int* __restrict__ perm, TC* __restrict__ rcoef,
                                                               double* __restrict__ R) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int nb = c1 - c0;
+  const int t0 = c0 + (int)blockIdx.x * HB_B;  // this CTA's first column
+  const int nb = min(HB_B, c1 - t0);
+  rcoef += (size_t)(t0 - c0) * c0;
   TO* s_L = reinterpret_cast<TO*>(smem_raw);                                               // c0 x c0
   TO* s_x = s_L + (size_t)c0 * c0;                                                          // HB_B x c0
   int* s_sel = reinterpret_cast<int*>(((uintptr_t)(s_x + (size_t)HB_B * c0) + 15) & ~(uintptr_t)15);  // c0
@@ -125,7 +127,7 @@ __global__ void __launch_bounds__(HB_B * 32) k_hess_blockcoef(int n, int c0, int
     for (int u = 0; u < 8; ++u) {
       const int e = e0 + u * blockDim.x;
       const int t = e / c0, j = e - t * c0;
-      v[u] = (e < nb * c0 && s_sel[j]) ? Q[(int64_t)s_perm[j] + (int64_t)(c0 + t) * ldq] : TO(0);
+      v[u] = (e < nb * c0 && s_sel[j]) ? Q[(int64_t)s_perm[j] + (int64_t)(t0 + t) * ldq] : TO(0);
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -141,14 +143,14 @@ __global__ void __launch_bounds__(HB_B * 32) k_hess_blockcoef(int n, int c0, int
     TO* x = s_x + warp * c0;
     TC* r = rcoef + (size_t)warp * c0;
     switch (nr) {
-      case 1: blockcoef_subst<1, TO, TC, FAST>(c0, n, warp, lane, x, s_L, s_sel, r, R); break;
-      case 2: blockcoef_subst<2, TO, TC, FAST>(c0, n, warp, lane, x, s_L, s_sel, r, R); break;
-      case 3: blockcoef_subst<3, TO, TC, FAST>(c0, n, warp, lane, x, s_L, s_sel, r, R); break;
-      case 4: blockcoef_subst<4, TO, TC, FAST>(c0, n, warp, lane, x, s_L, s_sel, r, R); break;
-      case 5: blockcoef_subst<5, TO, TC, FAST>(c0, n, warp, lane, x, s_L, s_sel, r, R); break;
-      case 6: blockcoef_subst<6, TO, TC, FAST>(c0, n, warp, lane, x, s_L, s_sel, r, R); break;
-      case 7: blockcoef_subst<7, TO, TC, FAST>(c0, n, warp, lane, x, s_L, s_sel, r, R); break;
-      default: blockcoef_subst<8, TO, TC, FAST>(c0, n, warp, lane, x, s_L, s_sel, r, R); break;
+      case 1: blockcoef_subst<1, TO, TC, FAST>(c0, t0, n, warp, lane, x, s_L, s_sel, r, R); break;
+      case 2: blockcoef_subst<2, TO, TC, FAST>(c0, t0, n, warp, lane, x, s_L, s_sel, r, R); break;
+      case 3: blockcoef_subst<3, TO, TC, FAST>(c0, t0, n, warp, lane, x, s_L, s_sel, r, R); break;
+      case 4: blockcoef_subst<4, TO, TC, FAST>(c0, t0, n, warp, lane, x, s_L, s_sel, r, R); break;
+      case 5: blockcoef_subst<5, TO, TC, FAST>(c0, t0, n, warp, lane, x, s_L, s_sel, r, R); break;
+      case 6: blockcoef_subst<6, TO, TC, FAST>(c0, t0, n, warp, lane, x, s_L, s_sel, r, R); break;
+      case 7: blockcoef_subst<7, TO, TC, FAST>(c0, t0, n, warp, lane, x, s_L, s_sel, r, R); break;
+      default: blockcoef_subst<8, TO, TC, FAST>(c0, t0, n, warp, lane, x, s_L, s_sel, r, R); break;
     }
   } else if (warp < nb) {
     TO* x = s_x + warp * c0;
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(HB_B * 32) k_hess_blockcoef(int n, int c0, int
       if (!s_sel[j]) {
         if (lane == 0) {
           r[j] = TC(0);
-          R[j + (int64_t)(c0 + warp) * n] = 0.0;
+          R[j + (int64_t)(t0 + warp) * n] = 0.0;
         }
         continue;
       }
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(HB_B * 32) k_hess_blockcoef(int n, int c0, int
       }
       if (lane == 0) {
         r[j] = rc;
-        R[j + (int64_t)(c0 + warp) * n] = to_c<double, TC>(rc);
+        R[j + (int64_t)(t0 + warp) * n] = to_c<double, TC>(rc);
       }
     }
   }
@@ -410,6 +412,174 @@ __global__ void __launch_bounds__(HB_T) k_hess_inblock(int64_t m, int n, int c0,
   cluster.sync();  // every push into this CTA has landed before any CTA leaves
 }
 
+// ---- panels of FP32-compute bases: one row per thread in registers ---------------------------------
+// For at most HR_T rows per CTA (8192 rows on sixteen) and FP32 arithmetic a thread keeps its row's values of up to
+// NV = 16 or 32 panel columns in registers.  The values shift down by one with every column (column t is always v[0]; the shift is part of the
+// elimination), so the loop over columns stays rolled with constant register indices, and a finished column goes
+// straight to Q.  The exchange is k_hess_inblock's: candidates pushed by st.async into every CTA's receive slots, two
+// buffers, completing on the receiver's mbarrier; the warp that owns the CTA's candidate sends it.
+// What bounds it: the chain of a column, about 3,200 cycles at 8192 rows and 32 columns (waiting for the candidates
+// 940, choosing 330, dividing 440, eliminating 860, argmax and sending 600).  The shared-memory form above takes 3,500
+// with blocks of 16 columns, each with two further launches.  Measured, half storage, 8192 rows: 16 columns 31 -> 25
+// us, 64 columns (two panels, one block update) 190 -> 123 us.  Panels of 64 columns (4,700 cycles a column: the
+// eliminations, and the registers spill) take 164 us.
+constexpr int HR_T = 512;
+
+template <class TO> __device__ __forceinline__ void hr_round2(float& a, float& b);
+template <> __device__ __forceinline__ void hr_round2<float>(float&, float&) {}
+template <> __device__ __forceinline__ void hr_round2<__half>(float& a, float& b) {
+  const float2 f = __half22float2(__floats2half2_rn(a, b));
+  a = f.x;
+  b = f.y;
+}
+template <> __device__ __forceinline__ void hr_round2<__nv_bfloat16>(float& a, float& b) {
+  const float2 f = __bfloat1622float2(__floats2bfloat162_rn(a, b));
+  a = f.x;
+  b = f.y;
+}
+
+template <class TO, int NV>
+struct __align__(16) HrCand {
+  unsigned key;  // 0: the CTA has no rows, 1: NaN, else the bits of |value| + 2
+  int row;       // its row within the CTA
+  int pad[2];
+  TO vals[NV];   // the row's values of the columns still to come, the current one first
+};
+
+template <class TO, int NV>
+__global__ void __launch_bounds__(HR_T) k_hess_reg(int64_t m, int n, int c0, int c1, int rows, TO* __restrict__ Q,
+                                                   int64_t ldq, int* __restrict__ select, int* __restrict__ perm,
+                                                   double* __restrict__ R, double select_tol, int* __restrict__ err) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), ncl = (int)cluster.num_blocks();
+  const int nb = c1 - c0, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int64_t r0 = (int64_t)rank * rows;
+  const int nr = (int)max((int64_t)0, min((int64_t)rows, m - r0));
+  using Cand = HrCand<TO, NV>;
+  constexpr int EPC = 16 / (int)sizeof(TO);  // values per 16-byte chunk
+  __shared__ Cand s_recv[2][HB_CL_MAX];
+  __shared__ Cand s_send;
+  __shared__ __align__(8) uint64_t s_bar[2];
+  __shared__ uint2 s_red[HR_T / 32];  // per warp: key, thread
+  __shared__ int s_abort;
+  const bool have = tid < nr;
+  const int nwarps = (nr + 31) / 32;  // warps with rows (warp 0 always takes part)
+
+  // bytes of a candidate when nrem columns are left
+  auto cand_bytes = [&](int nrem) { return (uint32_t)(16 + (nrem + EPC - 1) / EPC * 16); };
+  if (tid == 0) {
+    tc::mbar_init(&s_bar[0], 1);
+    tc::mbar_init(&s_bar[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tc::mbar_expect_tx(&s_bar[0], ncl * cand_bytes(nb));
+    if (nb > 1) tc::mbar_expect_tx(&s_bar[1], ncl * cand_bytes(nb - 1));
+    s_abort = 0;
+  }
+  float v[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+    v[j] = (have && j < nb) ? to_c<float, TO>(Q[r0 + tid + (int64_t)(c0 + j) * ldq]) : 0.f;
+  // this lane's destination CTA of a send (two lanes per CTA share the chunks)
+  const int dst = lane & (HB_CL_MAX - 1);
+  const uint32_t d_recv = cluster_addr(&s_recv[0][rank], dst < ncl ? dst : 0);
+  const uint32_t d_bar = cluster_addr(&s_bar[0], dst < ncl ? dst : 0);
+  cluster.sync();  // every CTA's barriers are armed before the first push
+
+  // the CTA's candidate for column t (v[0]) to every CTA
+  auto publish = [&](int t, int nrem) {
+    const unsigned bits = __float_as_uint(v[0]) & 0x7fffffffu;
+    const unsigned key = !have ? 0u : bits > 0x7f800000u ? 1u : bits + 2u;
+    const unsigned mk = __reduce_max_sync(0xffffffffu, key);
+    const unsigned who = __ballot_sync(0xffffffffu, key == mk);
+    if (lane == 0) s_red[wid] = make_uint2(mk, wid * 32 + __ffs(who) - 1);  // lowest row of the warp's maxima
+    __syncthreads();
+    const uint2 e = (lane < HR_T / 32) ? s_red[lane] : make_uint2(0u, 0u);
+    const unsigned bk = __reduce_max_sync(0xffffffffu, e.x);
+    const unsigned bw = __ballot_sync(0xffffffffu, lane < HR_T / 32 && e.x == bk);
+    const int win = __shfl_sync(0xffffffffu, (int)e.y, __ffs(bw) - 1);  // the lowest warp's
+    if (wid != (win >> 5)) return;
+    if (lane == (win & 31)) {
+      s_send.key = bk;
+      s_send.row = win;
+#pragma unroll
+      for (int j = 0; j < NV; j += EPC) {
+        if (j < nrem) {
+          __align__(16) TO x[EPC];
+#pragma unroll
+          for (int u = 0; u < EPC; ++u) x[u] = from_c<TO, float>(v[j + u]);
+          *reinterpret_cast<uint4*>(&s_send.vals[j]) = *reinterpret_cast<const uint4*>(x);
+        }
+      }
+    }
+    __syncwarp();
+    if (dst < ncl) {
+      const uint64_t* src = reinterpret_cast<const uint64_t*>(&s_send);
+      const int nch = (int)(cand_bytes(nrem) / 16);
+      const uint32_t to = d_recv + (uint32_t)((t & 1) * HB_CL_MAX * sizeof(Cand));
+      for (int c = lane / HB_CL_MAX; c < nch; c += 32 / HB_CL_MAX)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(to + 16u * c),
+                     "l"(src[2 * c]), "l"(src[2 * c + 1]), "r"(d_bar + 8u * (t & 1))
+                     : "memory");
+    }
+  };
+
+  const double tol_o = to_c<double, TO>(from_c<TO, double>(select_tol));
+  publish(0, nb);
+  for (int t = 0; t < nb; ++t) {
+    const int b = t & 1, nrem = nb - t;
+    if (!tc::mbar_wait(&s_bar[b], (uint32_t)((t >> 1) & 1), err, 43)) s_abort = 1;
+    if (tid == 0 && t + 2 < nb) tc::mbar_expect_tx(&s_bar[b], ncl * cand_bytes(nb - t - 2));  // re-arm for column t + 2
+    // the winner: the largest key, the lowest CTA (hence row) among equal ones
+    const unsigned ck = (lane < ncl) ? s_recv[b][lane].key : 0u;
+    const unsigned mk = __reduce_max_sync(0xffffffffu, ck);
+    const int w = __ffs(__ballot_sync(0xffffffffu, lane < ncl && ck == mk)) - 1;
+    const Cand* pc = &s_recv[b][w];
+    const TO pv = pc->vals[0];
+    const float pf = to_c<float, TO>(pv);
+    const bool keep = !(fabs((double)pf) < tol_o);  // a NaN pivot keeps the column (hessenberg.m)
+    if (rank == 0) {
+      const int i = c0 + t;
+      if (tid == 0) {
+        select[i] = keep ? 1 : 0;
+        perm[i] = keep ? (int)((int64_t)w * rows + pc->row) : -1;
+      }
+      for (int u = tid; u < nrem; u += HR_T)
+        R[i + (int64_t)(i + u) * n] = (u == 0 || keep) ? (double)to_c<float, TO>(pc->vals[u]) : 0.0;
+    }
+    // scale (or zero) column t, shift and eliminate the others
+    float so = keep ? __fdiv_rn(v[0], pf) : 0.f, dummy = 0.f;
+    hr_round2<TO>(so, dummy);
+    if (have) Q[r0 + tid + (int64_t)(c0 + t) * ldq] = from_c<TO, float>(so);
+    if (wid < nwarps) {
+#pragma unroll
+      for (int g = 0; g < NV; g += 8) {  // v[g .. g + 7] from v[g + 1 .. g + 8]
+        if (g + 1 < nrem) {
+          float r[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) r[u] = (g + 1 + u < NV) ? to_c<float, TO>(pc->vals[(g + 1 + u) % NV]) : 0.f;
+          if (keep) {
+#pragma unroll
+            for (int u = 0; u < 8; u += 2) {
+              float x = __fsub_rn(v[(g + u + 1) % NV], __fmul_rn(r[u], so));
+              float y = __fsub_rn(v[(g + u + 2) % NV], __fmul_rn(r[u + 1], so));
+              hr_round2<TO>(x, y);
+              v[g + u] = x;
+              v[g + u + 1] = y;
+            }
+          } else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[g + u] = v[(g + u + 1) % NV];
+          }
+        }
+      }
+    }
+    if (nrem == 1) break;
+    publish(t + 1, nrem - 1);  // its barrier also makes s_abort visible to every thread
+    if (s_abort) break;        // a peer stopped answering: leave (the status word is set)
+  }
+  cluster.sync();  // every push into this CTA has landed before any CTA leaves
+}
+
 // shared memory the in-block kernel needs for m rows on ncl CTAs (0 if it does not fit)
 size_t hess_blocked_smem(int64_t m, size_t es, int ncl) {
   const int64_t RR = (m + ncl - 1) / ncl;
@@ -451,6 +621,59 @@ static int inblock_cluster(int64_t m, size_t smem16) {
   return ncl;
 }
 
+template <class TO, int NV>
+static int hess_reg_launch(ofrr_ctx* ctx, int ncl, int64_t m, int n, int c0, int c1, TO* Q, int64_t ldq,
+                           double select_tol, double* R, int* select, int* perm) {
+  if (ncl > 8)
+    OFRR_CUDA(cudaFuncSetAttribute(k_hess_reg<TO, NV>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ncl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ncl);
+  cfg.blockDim = dim3(HR_T);
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  OFRR_CUDA(cudaLaunchKernelEx(&cfg, k_hess_reg<TO, NV>, m, n, c0, c1, (int)((m + ncl - 1) / ncl), Q, ldq, select, perm,
+                               R, select_tol, ctx->dev_flags + kFlagHessWait));
+  OFRR_LAUNCHED(ctx, "k_hess_reg");
+  return OFRR_SUCCESS;
+}
+
+// FP32-compute bases of at most HR_T rows per CTA of the cluster: panels of up to 64 columns
+template <class TO>
+static int hess_run_reg(ofrr_ctx* ctx, int ncl, int64_t m, int n, TO* Q, int64_t ldq, double select_tol, double* R,
+                        int* select, int* perm) {
+  int st = OFRR_SUCCESS;
+  WsScope scope(ctx);
+  constexpr int P = 32;
+  float* rcoef = ws_get<float>(ctx, (size_t)P * n, &st);
+  if (!rcoef) return st;
+  OFRR_TRY(fill_zero(ctx, R, sizeof(double) * (size_t)n * n));
+  for (int c0 = 0; c0 < n; c0 += P) {
+    const int c1 = std::min(c0 + P, n), nb = c1 - c0;
+    if (c0 > 0) {
+      const size_t smem0 = (size_t)c0 * c0 * sizeof(TO) + (size_t)HB_B * c0 * sizeof(TO) + 16 + 2 * (size_t)c0 * 4;
+      if (smem0 > 48 * 1024) OFRR_TRY(allow_smem(k_hess_blockcoef<TO, float, false>));
+      k_hess_blockcoef<TO, float, false><<<(nb + HB_B - 1) / HB_B, HB_B * 32, smem0, ctx->stream>>>(
+          n, c0, c1, Q, ldq, select, perm, rcoef, R);
+      OFRR_LAUNCHED(ctx, "k_hess_blockcoef");
+      const size_t smem1 = (size_t)HB_CG * c0 * sizeof(float) + (size_t)c0 * sizeof(int);
+      const dim3 grid1((unsigned)((m + HB_UT - 1) / HB_UT), (unsigned)((nb + HB_CG - 1) / HB_CG));
+      k_hess_blockupd<TO, float, false><<<grid1, HB_UT, smem1, ctx->stream>>>(m, c0, c1, Q, ldq, select, rcoef);
+      OFRR_LAUNCHED(ctx, "k_hess_blockupd");
+    }
+    if (nb <= 16)
+      OFRR_TRY((hess_reg_launch<TO, 16>(ctx, ncl, m, n, c0, c1, Q, ldq, select_tol, R, select, perm)));
+    else
+      OFRR_TRY((hess_reg_launch<TO, 32>(ctx, ncl, m, n, c0, c1, Q, ldq, select_tol, R, select, perm)));
+  }
+  return OFRR_SUCCESS;
+}
+
 template <class TO, class TC, bool FAST>
 int hess_run_blocked_t(ofrr_ctx* ctx, int64_t m, int n, TO* Q, int64_t ldq, double select_tol, double* R, int* select,
                        int* perm, bool* done) {
@@ -460,6 +683,10 @@ int hess_run_blocked_t(ofrr_ctx* ctx, int64_t m, int n, TO* Q, int64_t ldq, doub
   const size_t smem2 = hess_blocked_smem(m, sizeof(TO), ncl);
   if (!smem2) return OFRR_SUCCESS;  // needs 16 CTAs, and the device cannot co-schedule them
   *done = true;
+  if constexpr (std::is_same<TC, float>::value && !std::is_same<TO, double>::value) {
+    if (m <= (int64_t)ncl * HR_T)
+      return hess_run_reg<TO>(ctx, ncl, m, n, Q, ldq, select_tol, R, select, perm);
+  }
   int st = OFRR_SUCCESS;
   WsScope scope(ctx);
   TC* rcoef = ws_get<TC>(ctx, (size_t)HB_B * n, &st);
@@ -502,18 +729,22 @@ int hess_run_blocked_t(ofrr_ctx* ctx, int64_t m, int n, TO* Q, int64_t ldq, doub
   return OFRR_SUCCESS;
 }
 
+// whether the blocked schedule holds an m x n basis: the block's rows in the shared memory of sixteen CTAs, and the
+// coefficients' step at the last block (the c0 x c0 pivot block and the block's pivot-row values)
+bool hess_blocked_fits(int64_t m, int64_t n, size_t es) {
+  if (n > 256 || m < 2 * 8) return false;
+  const int64_t c0max = ((n - 1) / HB_B) * HB_B;
+  return (size_t)c0max * c0max * es + (size_t)HB_B * c0max * es + 16 + 2 * (size_t)c0max * 4 <= HB_SMEM_MAX &&
+         hess_blocked_smem(m, es, 16) != 0;
+}
+
 // Blocked build when it fits (m rows of the block in the cluster's shared memory, n <= 256);
 // *done = false leaves the call to the per-column path.  fast selects the FMA / reciprocal arithmetic
 // for an FP64 compute type (the production refinement phases); the exact arithmetic otherwise.
 int hess_run_blocked(ofrr_ctx* ctx, ofrr_dtype tout, ofrr_dtype tc, int64_t m, int64_t n, void* Q, int64_t ldq,
                      double select_tol, double* R, int* select, int* perm, bool fast, bool* done) {
   *done = false;
-  if (n > 256 || m < 2 * 8 || getenv("OFRR_HESS_PER_COLUMN")) return OFRR_SUCCESS;
-  // step-0 shared memory at the last block: the c0 x c0 pivot block and the block's pivot-row values
-  const int64_t c0max = ((n - 1) / HB_B) * HB_B;
-  const size_t es = dtype_size(tout);
-  if ((size_t)c0max * c0max * es + (size_t)HB_B * c0max * es + 16 + 2 * (size_t)c0max * 4 > HB_SMEM_MAX)
-    return OFRR_SUCCESS;
+  if (!hess_blocked_fits(m, n, dtype_size(tout)) || getenv("OFRR_HESS_PER_COLUMN")) return OFRR_SUCCESS;
   if (fast && tc == OFRR_F64) {
     OFRR_DISPATCH_STORAGE(tout, TO, {
       OFRR_TRY((hess_run_blocked_t<TO, double, true>(ctx, m, (int)n, (TO*)Q, ldq, select_tol, R, select, perm, done)));
