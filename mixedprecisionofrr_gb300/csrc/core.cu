@@ -134,6 +134,28 @@ int sync_and_check(ofrr_ctx* ctx) {
   return OFRR_SUCCESS;
 }
 
+int fetch_parts(ofrr_ctx* ctx, const void* src, std::initializer_list<HostPart> parts) {
+  size_t total = 0;
+  for (const HostPart& x : parts) total += x.bytes;
+  if (total == 0) return sync_and_check(ctx);
+  if (total <= ctx->pinned_size) {
+    OFRR_CUDA(cudaMemcpyAsync(ctx->pinned, src, total, cudaMemcpyDeviceToHost, ctx->stream));
+    OFRR_TRY(sync_and_check(ctx));
+    const char* p = (const char*)ctx->pinned;
+    for (const HostPart& x : parts) {
+      if (x.dst && x.bytes) memcpy(x.dst, p, x.bytes);
+      p += x.bytes;
+    }
+    return OFRR_SUCCESS;
+  }
+  const char* p = (const char*)src;
+  for (const HostPart& x : parts) {
+    if (x.dst && x.bytes) OFRR_CUDA(cudaMemcpyAsync(x.dst, p, x.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    p += x.bytes;
+  }
+  return sync_and_check(ctx);
+}
+
 int fill_zero(ofrr_ctx* ctx, void* p, size_t bytes) {
   if (bytes == 0) return OFRR_SUCCESS;
   OFRR_CUDA(cudaMemsetAsync(p, 0, bytes, ctx->stream));

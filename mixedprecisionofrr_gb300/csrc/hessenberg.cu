@@ -308,18 +308,15 @@ extern "C" int ofrr_hessenberg(ofrr_ctx* ctx, ofrr_dtype tin, ofrr_dtype tout, o
   if (!A || !Q || lda < m || ldq < m) return OFRR_ERR_INVALID_ARGUMENT;
   WsScope scope(ctx);
   int st = OFRR_SUCCESS;
-  double* R = ws_get<double>(ctx, (size_t)n * n, &st);
+  // R, then the flags, then the pivot rows: adjacent, for one copy to the host
+  double* R = (double*)ws_alloc(ctx, sizeof(double) * n * n + 2 * sizeof(int) * n, &st);
   if (!R) return st;
-  int* sel = ws_get<int>(ctx, (size_t)n, &st);
-  if (!sel) return st;
-  int* perm = ws_get<int>(ctx, (size_t)n, &st);
-  if (!perm) return st;
+  int* sel = (int*)(R + n * n);
+  int* perm = sel + n;
   OFRR_TRY(hessenberg_impl(ctx, tin, tout, tcompute, m, n, A, lda, Q, ldq, select_tol, R, sel, perm));
   std::vector<int> hsel(n), hperm(n);
-  OFRR_CUDA(cudaMemcpyAsync(hsel.data(), sel, n * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_CUDA(cudaMemcpyAsync(hperm.data(), perm, n * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  if (R_host) OFRR_CUDA(cudaMemcpyAsync(R_host, R, sizeof(double) * n * n, cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch_parts(
+      ctx, R, {{R_host, sizeof(double) * n * n}, {hsel.data(), n * sizeof(int)}, {hperm.data(), n * sizeof(int)}}));
   for (int64_t j = 0; j < n; ++j) {
     if (skip_host) skip_host[j] = hsel[j] ? 0 : 1;
     if (perm_host) perm_host[j] = hperm[j];

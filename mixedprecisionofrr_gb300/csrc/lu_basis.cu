@@ -142,14 +142,13 @@ extern "C" int ofrr_lu_basis(ofrr_ctx* ctx, ofrr_dtype tin, ofrr_dtype tout, ofr
   if (!A || !Q || lda < m || ldq < m) return OFRR_ERR_INVALID_ARGUMENT;
   WsScope scope(ctx);
   int st = OFRR_SUCCESS;
-  double* R = ws_get<double>(ctx, (size_t)n * n, &st);
-  int* sel = ws_get<int>(ctx, (size_t)n, &st);
-  if (!R || !sel) return st;
+  // U, then the flags: adjacent, for one copy to the host
+  double* R = (double*)ws_alloc(ctx, sizeof(double) * n * n + sizeof(int) * n, &st);
+  if (!R) return st;
+  int* sel = (int*)(R + n * n);
   OFRR_TRY(lu_basis_impl(ctx, tin, tout, tcompute, m, n, A, lda, Q, ldq, select_tol, R, sel));
   std::vector<int> hsel((size_t)n);
-  OFRR_CUDA(cudaMemcpyAsync(hsel.data(), sel, sizeof(int) * n, cudaMemcpyDeviceToHost, ctx->stream));
-  if (U_host) OFRR_CUDA(cudaMemcpyAsync(U_host, R, sizeof(double) * n * n, cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch_parts(ctx, R, {{U_host, sizeof(double) * n * n}, {hsel.data(), sizeof(int) * n}}));
   if (skip_host)
     for (int64_t j = 0; j < n; ++j) skip_host[j] = hsel[(size_t)j] ? 0 : 1;
   return OFRR_SUCCESS;

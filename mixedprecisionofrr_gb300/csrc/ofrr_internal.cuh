@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <cstddef>
 #include <cstdio>
+#include <initializer_list>
 #include <vector>
 #include <algorithm>
 
@@ -121,6 +122,19 @@ constexpr int kFlagHessWait = 4;
 // Synchronise ctx's stream; OFRR_ERR_DEVICE_TIMEOUT when a bounded device wait gave up since the
 // last check (the words are cleared again).
 int sync_and_check(ofrr_ctx* ctx);
+
+// Small results to the host: one asynchronous copy into the context's pinned buffer, one synchronisation
+// (sync_and_check), then plain host copies.  (A copy to pageable memory waits for the stream by itself, about 8 us,
+// and the synchronisation after it comes on top.)  Parts: {destination or null, bytes}, adjacent in `src`; more than
+// the pinned buffer holds goes straight to the destinations.
+struct HostPart {
+  void* dst;
+  size_t bytes;
+};
+int fetch_parts(ofrr_ctx* ctx, const void* src, std::initializer_list<HostPart> parts);
+inline int fetch(ofrr_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  return fetch_parts(ctx, src, {HostPart{dst, bytes}});
+}
 
 // Concurrency inside one solve: aux_begin() returns the context's auxiliary context (created on
 // first use: same device, its own stream, cuBLAS handle and workspace) after ordering its stream

@@ -499,8 +499,7 @@ int gs_run(ofrr_ctx* ctx, bool classical, int64_t m, int64_t n, const TO* A, int
   // the norms of the original columns (column i is untouched until its turn)
   for (int64_t i = 0; i < n; ++i) OFRR_TRY(norm_of(A + i * lda, norms + i));
   std::vector<TO> hn((size_t)n);
-  OFRR_CUDA(cudaMemcpyAsync(hn.data(), norms, sizeof(TO) * n, cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch(ctx, hn.data(), norms, sizeof(TO) * n));
   std::vector<int> sel((size_t)n, 0), hcols;
   // one projection pass of v against the selected columns hcols (R column i; acc: accumulate)
   auto pass = [&](int64_t i, int acc) -> int {
@@ -529,16 +528,14 @@ int gs_run(ofrr_ctx* ctx, bool classical, int64_t m, int64_t n, const TO* A, int
     OFRR_TRY(pass(i, 0));
     TO ht;
     OFRR_TRY(norm_of(v, rr + n));
-    OFRR_CUDA(cudaMemcpyAsync(&ht, rr + n, sizeof(TO), cudaMemcpyDeviceToHost, ctx->stream));
-    OFRR_TRY(sync_and_check(ctx));
+    OFRR_TRY(fetch(ctx, &ht, rr + n, sizeof(TO)));
     double t = host_double(ht);
     // (at most 64 passes: the reference loops until the norm stops dropping, which takes 1-2)
     for (int guard = 0; rtol >= 0 && t >= otol && t < rtol * normv && guard < 64; ++guard) {
       normv = t;
       OFRR_TRY(pass(i, 1));
       OFRR_TRY(norm_of(v, rr + n));
-      OFRR_CUDA(cudaMemcpyAsync(&ht, rr + n, sizeof(TO), cudaMemcpyDeviceToHost, ctx->stream));
-      OFRR_TRY(sync_and_check(ctx));
+      OFRR_TRY(fetch(ctx, &ht, rr + n, sizeof(TO)));
       t = host_double(ht);
     }
     if (t < stol) continue;
@@ -609,16 +606,14 @@ extern "C" int ofrr_gs_basis(ofrr_ctx* ctx, int classical, ofrr_dtype tin, ofrr_
   if (!A || !Q || lda < m || ldq < m) return OFRR_ERR_INVALID_ARGUMENT;
   WsScope scope(ctx);
   int st = OFRR_SUCCESS;
-  double* R = ws_get<double>(ctx, (size_t)n * n, &st);
+  // R, then the flags: adjacent, for one copy to the host
+  double* R = (double*)ws_alloc(ctx, sizeof(double) * n * n + sizeof(int) * n, &st);
   if (!R) return st;
-  int* sel = ws_get<int>(ctx, (size_t)n, &st);
-  if (!sel) return st;
+  int* sel = (int*)(R + n * n);
   OFRR_TRY(gs_basis_impl(ctx, classical != 0, tin, tout, tcompute, m, n, A, lda, Q, ldq, select_tol, R, sel,
                          orth_tol, reorth_tol));
   std::vector<int> hsel((size_t)n);
-  OFRR_CUDA(cudaMemcpyAsync(hsel.data(), sel, n * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  if (R_host) OFRR_CUDA(cudaMemcpyAsync(R_host, R, sizeof(double) * n * n, cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch_parts(ctx, R, {{R_host, sizeof(double) * n * n}, {hsel.data(), sizeof(int) * n}}));
   if (skip_host)
     for (int64_t j = 0; j < n; ++j) skip_host[j] = hsel[(size_t)j] ? 0 : 1;
   return OFRR_SUCCESS;

@@ -951,8 +951,7 @@ int invariant_subspace_nonsym(ofrr_ctx* ctx, int n, const double* G, const doubl
   OFRR_LAUNCHED(ctx, "k_proj_basis");
   OFRR_TRY(trsm(ctx, n, p, L, Q, n, 0, Y, 1));  // Y = L^-T Q
   int hf = 0;
-  OFRR_CUDA(cudaMemcpyAsync(&hf, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch(ctx, &hf, flag, sizeof(int)));
   return hf ? OFRR_ERR_SINGULAR_MATRIX : OFRR_SUCCESS;
 }
 

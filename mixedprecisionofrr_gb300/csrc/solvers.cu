@@ -568,8 +568,7 @@ int residuals_dev(ofrr_ctx* ctx, Op& op, ofrr_dtype tx, const void* X, int64_t l
   OFRR_TRY(residual_columns(ctx, n, k, AX, n, X64, n, lam, res));
   OFRR_TRY(column_norms(ctx, OFRR_F64, n, k, X64, n, nrm));
   std::vector<double> h(3 * k, 0.0);
-  OFRR_CUDA(cudaMemcpyAsync(h.data(), res, sizeof(double) * 2 * k, cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch(ctx, h.data(), res, sizeof(double) * 2 * k));
   if (normA <= 0) {
     normA = 0;
     for (int j = 0; j < k; ++j) normA = std::max(normA, std::fabs(lam_host[j]));
@@ -583,8 +582,7 @@ int residuals_dev(ofrr_ctx* ctx, Op& op, ofrr_dtype tx, const void* X, int64_t l
     k_normalize_cols<<<grid_cols(n, k), 256, 0, ctx->stream>>>(n, k, X64, nrm);
     OFRR_LAUNCHED(ctx, "k_normalize_cols");
     OFRR_TRY(emulation_bounds(ctx, op, 0, (ofrr_dtype)certify16, X64, n, k, bnd));
-    OFRR_CUDA(cudaMemcpyAsync(h.data() + 2 * k, bnd, sizeof(double) * k, cudaMemcpyDeviceToHost, ctx->stream));
-    OFRR_TRY(sync_and_check(ctx));
+    OFRR_TRY(fetch(ctx, h.data() + 2 * k, bnd, sizeof(double) * k));
   }
   for (int j = 0; j < k; ++j) {
     out_host[j] = (h[k + j] > 0) ? h[j] / (normA * h[k + j]) + kEmulBound * h[2 * k + j] / normA : INFINITY;
@@ -638,8 +636,7 @@ extern "C" int ofrr_rr_eig(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_opt
   // eig_rr on V (type p_output): pmc = p_rr_compute, pmo = p_rr_output, A-matvec in (p_compute, p_output)
   OFRR_TRY(rr_eig_dev(ctx, op, P.po, V, P.po, ldv, (int)ncols, P.prc, P.pro, P.pc, P.po, opt->use_generalized != 0,
                       opt->generalized_tol, A->symmetric != 0, V, ldv, d));
-  OFRR_CUDA(cudaMemcpyAsync(evals, d, sizeof(double) * ncols, cudaMemcpyDeviceToHost, ctx->stream));
-  return sync_and_check(ctx);
+  return fetch(ctx, evals, d, sizeof(double) * ncols);
 }
 
 extern "C" int ofrr_ofrr_eig(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_operator* B, const ofrr_options* opt,
@@ -680,8 +677,7 @@ extern "C" int ofrr_ofrr_eig(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_o
   OFRR_TRY(geig_dev(ctx, b, G, b, M, b, 1, d, U, b));
   OFRR_TRY(gemm_impl(ctx, 0, 0, P.po, OFRR_F64, P.prc, P.pro, n, b, b, 1.0, V, ldv, U, b, 0.0, Vn, n));
   OFRR_TRY(cast_impl(ctx, P.pro, P.po, n, b, Vn, n, V, ldv));
-  OFRR_CUDA(cudaMemcpyAsync(evals, d, sizeof(double) * b, cudaMemcpyDeviceToHost, ctx->stream));
-  return sync_and_check(ctx);
+  return fetch(ctx, evals, d, sizeof(double) * b);
 }
 
 extern "C" int ofrr_residual_norms(ofrr_ctx* ctx, const ofrr_operator* A, ofrr_dtype tx, int64_t ncols, const void* X,
@@ -886,8 +882,7 @@ int svd_residuals_dev(ofrr_ctx* ctx, Op& op, ofrr_dtype tx, const void* U, int64
     OFRR_LAUNCHED(ctx, "k_rescol2");
   }
   std::vector<double> h(4 * k, 0.0);
-  OFRR_CUDA(cudaMemcpyAsync(h.data(), nr + 2 * k, sizeof(double) * 2 * k, cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch(ctx, h.data(), nr + 2 * k, sizeof(double) * 2 * k));
   if (normA <= 0) {
     normA = 0;
     for (int j = 0; j < k; ++j) normA = std::max(normA, std::fabs(s_host[j]));
@@ -900,8 +895,7 @@ int svd_residuals_dev(ofrr_ctx* ctx, Op& op, ofrr_dtype tx, const void* U, int64
     OFRR_TRY(dmalloc(ctx, &bnd, (size_t)2 * k));
     OFRR_TRY(emulation_bounds(ctx, op, 0, (ofrr_dtype)certify16, V64, n, k, bnd));
     OFRR_TRY(emulation_bounds(ctx, op, 1, (ofrr_dtype)certify16, U64, m, k, bnd + k));
-    OFRR_CUDA(cudaMemcpyAsync(h.data() + 2 * k, bnd, sizeof(double) * 2 * k, cudaMemcpyDeviceToHost, ctx->stream));
-    OFRR_TRY(sync_and_check(ctx));
+    OFRR_TRY(fetch(ctx, h.data() + 2 * k, bnd, sizeof(double) * 2 * k));
   }
   for (int j = 0; j < k; ++j) {
     out_host[j] = std::max(h[j] + kEmulBound * h[2 * k + j], h[k + j] + kEmulBound * h[3 * k + j]) / normA;
@@ -989,8 +983,7 @@ extern "C" int ofrr_rr_svd(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_opt
                               cudaMemcpyDeviceToDevice, ctx->stream));
   OFRR_CUDA(cudaMemcpy2DAsync(V, ldv * dtype_size(P.po), Vt, n * dtype_size(P.po), n * dtype_size(P.po), b,
                               cudaMemcpyDeviceToDevice, ctx->stream));
-  OFRR_CUDA(cudaMemcpyAsync(s, d, sizeof(double) * b, cudaMemcpyDeviceToHost, ctx->stream));
-  return sync_and_check(ctx);
+  return fetch(ctx, s, d, sizeof(double) * b);
 }
 
 // ======================================================================================
@@ -1053,8 +1046,8 @@ static int arnoldi_thick_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_
   OFRR_TRY(dmalloc(ctx, &d, (size_t)nb));
   OFRR_TRY(dmalloc(ctx, &xg, (size_t)nb));
   OFRR_TRY(dmalloc(ctx, &nrm, (size_t)nb));
-  OFRR_TRY(dmalloc(ctx, &sel, (size_t)nb));
-  OFRR_TRY(dmalloc(ctx, &perm, (size_t)nb));
+  OFRR_TRY(dmalloc(ctx, &sel, (size_t)2 * nb));
+  perm = sel + nb;
   // the start vector (FP64) as the first block
   if (opt->use_start_block) {
     OFRR_CUDA(cudaMemcpyAsync(Wb, v0, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -1087,9 +1080,7 @@ static int arnoldi_thick_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_
       OFRR_TRY(scalecols_impl(ctx, tw, tw, n, q0, blk, ld, nullptr, tw == OFRR_F64));
       const double stol_blk = (t == OFRR_F64) ? 1e-12 : 4.0 * dtype_eps(t);
       OFRR_TRY(hessenberg_impl(ctx, tw, t, ta, n, q0, blk, ld, S.V, S.ldv, stol_blk, R, sel, perm, true));
-      OFRR_CUDA(cudaMemcpyAsync(hsel.data(), sel, sizeof(int) * q0, cudaMemcpyDeviceToHost, ctx->stream));
-      OFRR_CUDA(cudaMemcpyAsync(hperm.data(), perm, sizeof(int) * q0, cudaMemcpyDeviceToHost, ctx->stream));
-      OFRR_TRY(sync_and_check(ctx));
+      OFRR_TRY(fetch_parts(ctx, sel, {{hsel.data(), sizeof(int) * nb}, {hperm.data(), sizeof(int) * nb}}));
       std::vector<int> s0(hsel.begin(), hsel.begin() + q0);
       for (int j = 0; j < q0; ++j)
         if (s0[j]) cperm[q++] = hperm[j];
@@ -1102,8 +1093,7 @@ static int arnoldi_thick_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_
     ts.next("krylov.steps");
     OFRR_TRY(kry_cycle_steps(ctx, S, q));
     int hstop = -1;
-    OFRR_CUDA(cudaMemcpyAsync(&hstop, S.stop, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    OFRR_TRY(sync_and_check(ctx));
+    OFRR_TRY(fetch(ctx, &hstop, S.stop, sizeof(int)));
     ncols = (hstop >= 0) ? hstop : nb;
     steps += ncols - q;
     // (3) generalized Rayleigh-Ritz on the ncols columns, the Ritz vectors, the kept block and the
@@ -1145,8 +1135,7 @@ static int arnoldi_thick_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_
       const bool restricted = !symmetric && t == OFRR_F64 && ncols <= 96;
       if (symmetric) OFRR_TRY(geig_fast(ctx, ncols, G, M, 0.0, d, U, t == OFRR_F64 ? 2 : 1));
       else OFRR_TRY(geig_nonsym(ctx, ncols, G, M, d, U, t == OFRR_F64 && !restricted, true, restricted));
-      OFRR_CUDA(cudaMemcpyAsync(hd.data(), d, sizeof(double) * ncols, cudaMemcpyDeviceToHost, ctx->stream));
-      OFRR_TRY(sync_and_check(ctx));
+      OFRR_TRY(fetch(ctx, hd.data(), d, sizeof(double) * ncols));
       k = std::min(nev, ncols);
       // the kept block ends at the widest gap of the real parts near `keep` (never inside a complex pair)
       pp = std::min(keep, ncols - 1);
@@ -1366,8 +1355,7 @@ static int arnoldi_eig_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_op
     } else {
       OFRR_TRY(hess_krylov_first(ctx, po, pc, n, nb, V, n, stol, sel, perm, pivrows, pvals, R, stop));
     }
-    OFRR_CUDA(cudaMemcpyAsync(hstop, stop, sizeof(int) * 2, cudaMemcpyDeviceToHost, ctx->stream));
-    OFRR_TRY(sync_and_check(ctx));
+    OFRR_TRY(fetch(ctx, hstop, stop, sizeof(int) * 2));
     if (hstop[0] >= 0) break;  // start vector below select_tol
     int ncols = nb;
     for (int i = 1; i <= kdim; ++i) {
@@ -1381,8 +1369,7 @@ static int arnoldi_eig_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_op
         OFRR_TRY(hess_scale_col(ctx, po, pc, n, i, V, n, sel, pvals, stop));
       }
     }
-    OFRR_CUDA(cudaMemcpyAsync(hstop, stop, sizeof(int) * 2, cudaMemcpyDeviceToHost, ctx->stream));
-    OFRR_TRY(sync_and_check(ctx));
+    OFRR_TRY(fetch(ctx, hstop, stop, sizeof(int) * 2));
     int steps = kdim;
     if (hstop[0] >= 0) {  // breakdown at step hstop[0]: invariant subspace found
       steps = hstop[0] - 1;
@@ -1405,8 +1392,7 @@ static int arnoldi_eig_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_op
     if (tits < opt->maxiter) {
       OFRR_CUDA(cudaMemcpyAsync(V, Vr, (size_t)n * dtype_size(po), cudaMemcpyDeviceToDevice, ctx->stream));
       if (opt->tol > 0) {  // convergence check on the current Ritz pairs (new behaviour)
-        OFRR_CUDA(cudaMemcpyAsync(hd.data(), d, sizeof(double) * ncols, cudaMemcpyDeviceToHost, ctx->stream));
-        OFRR_TRY(sync_and_check(ctx));
+        OFRR_TRY(fetch(ctx, hd.data(), d, sizeof(double) * ncols));
         const int k = std::min(nev, ncols);
         OFRR_TRY(residuals_dev(ctx, op, po, Vr, n, k, hd.data(), -1.0, hres.data()));
         bool ok = true;
@@ -1419,8 +1405,7 @@ static int arnoldi_eig_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_op
   const int k = std::min(nev, ncols_final);
   OFRR_CUDA(cudaMemcpy2DAsync(X, ldx * dtype_size(po), Vr, n * dtype_size(po), n * dtype_size(po), k,
                               cudaMemcpyDeviceToDevice, ctx->stream));
-  OFRR_CUDA(cudaMemcpyAsync(hd.data(), d, sizeof(double) * ncols_final, cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch(ctx, hd.data(), d, sizeof(double) * ncols_final));
   for (int j = 0; j < nev; ++j) evals[j] = (j < k) ? hd[j] : NAN;
   OFRR_TRY(residuals_dev(ctx, op, po, X, ldx, k, hd.data(), -1.0, hres.data()));
   if (resid)
@@ -1545,8 +1530,7 @@ int eig_phase(ofrr_ctx* ctx, Op& op, const Precisions& P, const ofrr_options* op
     // [Q,~] = hessenberg(V): the economic form drops deselected columns
     OFRR_TRY(basis_impl(ctx, opt->orth, P.po, P.pho, P.phc, n, b, cur, ldcur, Q, n, opt->select_tol, R, sel, perm,
                         P.fast));
-    OFRR_CUDA(cudaMemcpyAsync(hsel.data(), sel, sizeof(int) * b, cudaMemcpyDeviceToHost, ctx->stream));
-    OFRR_TRY(sync_and_check(ctx));
+    OFRR_TRY(fetch(ctx, hsel.data(), sel, sizeof(int) * b));
     int w = b;
     OFRR_TRY(compact_columns(ctx, P.pho, n, Q, n, std::vector<int>(hsel.begin(), hsel.begin() + b), &w));
     if (w == 0) return OFRR_ERR_SOLVER_DIVERGENCE;
@@ -1574,8 +1558,7 @@ int eig_phase(ofrr_ctx* ctx, Op& op, const Precisions& P, const ofrr_options* op
     const bool last = (k + 1 == maxit);
     const bool check = tol > 0 && ((S.it % check_every) == 0 || last);
     if (check || stag_tol > 0) {
-      OFRR_CUDA(cudaMemcpyAsync(S.d.data(), d_dev, sizeof(double) * b, cudaMemcpyDeviceToHost, ctx->stream));
-      OFRR_TRY(sync_and_check(ctx));
+      OFRR_TRY(fetch(ctx, S.d.data(), d_dev, sizeof(double) * b));
     }
     if (check && certify16 >= 0) {
       // certified check (emulated products), as in svd_phase
@@ -1693,8 +1676,7 @@ int svd_phase(ofrr_ctx* ctx, Op& op, const Precisions& P, const ofrr_options* op
       OFRR_TRY(basis_impl(ctx, opt->orth, P.po, P.pho, P.phc, m, b, U, ldu, P1, m, opt->select_tol, R, sel, perm,
                           P.fast));
       OFRR_TRY(aux_end(ctx));
-      OFRR_CUDA(cudaMemcpyAsync(hsel.data(), sel, sizeof(int) * 2 * b0, cudaMemcpyDeviceToHost, ctx->stream));
-      OFRR_TRY(sync_and_check(ctx));
+      OFRR_TRY(fetch(ctx, hsel.data(), sel, sizeof(int) * 2 * b0));
     }
     {
       TraceScope ts(ctx, f64 ? "rr.f64" : "rr.16bit");
@@ -1722,8 +1704,7 @@ int svd_phase(ofrr_ctx* ctx, Op& op, const Precisions& P, const ofrr_options* op
     const bool check = tol > 0 && ((S.it % check_every) == 0 || last);
     TraceScope ts(ctx, f64 ? "check.f64" : "check.16bit");
     if (check || stag_tol > 0) {
-      OFRR_CUDA(cudaMemcpyAsync(S.d.data(), d_dev, sizeof(double) * b, cudaMemcpyDeviceToHost, ctx->stream));
-      OFRR_TRY(sync_and_check(ctx));
+      OFRR_TRY(fetch(ctx, S.d.data(), d_dev, sizeof(double) * b));
     }
     if (check && certify16 >= 0) {
       // certified check (emulated products): the emulated residuals plus the bounds on the emulation
@@ -1874,8 +1855,7 @@ static int si_eig_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_options
     OFRR_TRY(scalecols_impl(ctx, P.po, P.pc, n, b0, V, ldv, nullptr));
     OFRR_TRY(eig_phase(ctx, op, P, opt, V, ldv, opt->maxiter, opt->tol, nev, 0.0, S, d));
   }
-  OFRR_CUDA(cudaMemcpyAsync(S.d.data(), d, sizeof(double) * S.b, cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch(ctx, S.d.data(), d, sizeof(double) * S.b));
   for (int j = 0; j < b0; ++j) evals[j] = (j < S.b) ? S.d[j] : NAN;
   if (resid) {
     if (opt->tol <= 0) OFRR_TRY(residuals_dev(ctx, op, tV, V, ldv, S.b, S.d.data(), -1.0, S.res.data()));
@@ -1985,8 +1965,7 @@ static int si_svd_body(ofrr_ctx* ctx, const ofrr_operator* A, const ofrr_options
     OFRR_TRY(scalecols_impl(ctx, P.po, P.pc, n, b0, V, ldv, nullptr));
     OFRR_TRY(svd_phase(ctx, op, P, opt, U, ldu, V, ldv, opt->maxiter, opt->tol, nev, 0.0, S, d));
   }
-  OFRR_CUDA(cudaMemcpyAsync(S.d.data(), d, sizeof(double) * S.b, cudaMemcpyDeviceToHost, ctx->stream));
-  OFRR_TRY(sync_and_check(ctx));
+  OFRR_TRY(fetch(ctx, S.d.data(), d, sizeof(double) * S.b));
   for (int j = 0; j < b0; ++j) s[j] = (j < S.b) ? S.d[j] : NAN;
   if (resid) {
     if (opt->tol <= 0) OFRR_TRY(svd_residuals_dev(ctx, op, tV, U, ldu, V, ldv, S.b, S.d.data(), -1.0, S.res.data()));
