@@ -513,9 +513,9 @@ int geig_dev(ofrr_ctx* ctx, int n, const double* G, int ldg, const double* M, in
              double* w, double* U, int ldu);
 
 // the FP64 pieces of the small solvers, n <= 160 (ld n): Cholesky factor L of M (lower, near-zero pivots
-// clamped), and X = L^-1 B (upper = 0) or L^-T B (upper = 1), B read transposed for transB (n x n)
+// clamped), and X = L^-1 B, B read transposed for transB (n x n); correctly rounded quotients and square roots
 int small_chol(ofrr_ctx* ctx, int n, const double* M, int ldm, double* L);
-int small_trsm(ofrr_ctx* ctx, int n, const double* L, const double* B, int transB, double* X, int upper);
+int small_trsm(ofrr_ctx* ctx, int n, const double* L, const double* B, int transB, double* X);
 
 // production small solvers (FP32 Jacobi + FP64 refinement, multi-CTA FP64 products), n <= 128:
 // eig(G, M + tau I) (M may be null) and the svd_rr pencil of B with Gram matrices UU, VV

@@ -6,7 +6,7 @@
 // Jacobi on C with round-robin parallel ordering (n/2 disjoint rotations per round, Golub & Van Loan
 // sym.Schur2 rotation), eigenvalue sort, U = L^-T W.
 // The eigenvectors are M-orthonormal (U' M U = I), the LAPACK sygv / MATLAB 'chol' normalisation.
-// Orders up to kGeigClusterMaxN (160: what the Cholesky and substitution kernels hold in one CTA's shared
+// Orders up to kGeigClusterMaxN (144: what the Cholesky and substitution kernels hold in one CTA's shared
 // memory) run the Jacobi sweeps on a thread-block cluster (k_jacobi_cluster); larger ones run the whole
 // algorithm on one CTA in a global workspace (k_geig_sym).
 #include <atomic>
@@ -30,7 +30,7 @@ namespace ofrr {
 // a round costs one cluster barrier, and every CTA computes all rotations itself (N / 2 threads; the
 // chain's latency does not depend on how many warps run it, up to one per sub-partition).
 constexpr int kJacT = 512;
-constexpr int kGeigClusterMaxN = 160;
+constexpr int kGeigClusterMaxN = 144;  // Cholesky, substitutions and L beside 32 columns in one CTA's 227 KB
 
 // The rotation of sym.Schur2 (t the root of smaller magnitude of t^2 + 2 tau t - 1 = 0, t = 1 for tau = 0).
 // Divisions and square roots are FP64 sequences of about 430 cycles each, so the chain takes ~2000 cycles, the
@@ -72,7 +72,8 @@ __device__ __forceinline__ int jac_next(int i, int step, int N) {
 __device__ __forceinline__ int jac_next_seat(int s, int N) { return (s == 0) ? 0 : (s == 1) ? N - 1 : s - 1; }
 
 // C (n x n, symmetric, ld n) -> eigenvalues w (sorted) and the matching orthonormal eigenvectors Wout
-// (ld n).  Grid = one cluster of NC CTAs.  Every thread owns up to IT items of C (one row pair of one of the
+// (ld n); hit[r] = 1 for the ranks that were written (all of them, but for eigenvalues that are NaN).
+// Grid = one cluster of NC CTAs.  Every thread owns up to IT items of C (one row pair of one of the
 // CTA's columns; adjacent lanes the two columns of a 2 x 2 block) and IT items of W (one row of one of the
 // CTA's column pairs), and at most one remote entry of the next rotations: their seats never change, so only
 // the indices at the seats are stepped from round to round.  W trails by one round: W <- W J runs beside
@@ -80,7 +81,7 @@ __device__ __forceinline__ int jac_next_seat(int s, int N) { return (s == 0) ? 0
 template <int IT>
 __global__ void __launch_bounds__(kJacT) k_jacobi_cluster(int n, int NC, int PP, const double* __restrict__ Cin,
                                                           double* __restrict__ w, double* __restrict__ Wout,
-                                                          int descending, int max_sweeps) {
+                                                          int* __restrict__ hit, int descending, int max_sweeps) {
   extern __shared__ double jsm[];
   const int N = n + (n & 1), npair = N / 2, S = 2 * PP;
   const int rank = (int)cluster_rank();
@@ -227,6 +228,8 @@ __global__ void __launch_bounds__(kJacT) k_jacobi_cluster(int n, int NC, int PP,
     plan_e();
   };
   plan_e();
+  if (rank == 0)
+    for (int i = tid; i < n; i += kJacT) hit[i] = 0;
   int r_x = tid, r_y = N - 1 - tid;  // indices of the pair whose rotation this thread computes (tid < npair)
 
   for (int e = tid; e < S * n; e += kJacT) {
@@ -393,8 +396,46 @@ __global__ void __launch_bounds__(kJacT) k_jacobi_cluster(int n, int NC, int PP,
       rk += before ? 1 : 0;
     }
     rk = __reduce_add_sync(0xffffffffu, rk);
-    if ((tid & 31) == 0) w[rk] = dj;
+    if ((tid & 31) == 0) {
+      w[rk] = dj;
+      hit[rk] = 1;
+    }
     for (int i = tid & 31; i < n; i += 32) Wout[i + (size_t)rk * n] = wb[((size_t)b * S + slot) * n + i];
+  }
+}
+
+// U = L^-T W (n x n, ld n; U with ld ldu): u_r = (w_r - sum_{k > r} L(k, r) u_k) / L(r, r), the sum in ascending k, so
+// that the bits are the one-CTA form's -- where M is nearly singular (pivots clamped) another order of the sum gives
+// other vectors altogether.  The first term of a row is the value found last, so a column is a chain of n^2 / 2
+// dependent FMAs whatever the schedule (n = 64: 62 us); one lane per column, one warp per CTA, L in shared memory
+// where it fits.
+__global__ void __launch_bounds__(32) k_back_subst(int n, const double* __restrict__ L, const double* __restrict__ W,
+                                                   const int* __restrict__ hit, double* __restrict__ U, int ldu) {
+  extern __shared__ double bsm[];  // L (column-major), then the CTA's 32 columns of U (row-major)
+  double* sL = bsm;
+  double* sU = bsm + (size_t)n * n;
+  const int lane = threadIdx.x, j = blockIdx.x * 32 + lane;
+  for (int e = lane; e < n * n; e += 32) sL[e] = L[e];
+  __syncwarp();
+  const bool store = j < n && hit[j];
+  for (int r = n - 1; r >= 0; --r) {
+    double s = (j < n) ? W[r + (size_t)j * n] : 0.0;
+    const double* l = sL + (size_t)r * n;
+    int k = r + 1;
+    for (; k + 8 <= n; k += 8) {
+      double a[8], b[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        a[u] = l[k + u];
+        b[u] = sU[(k + u) * 32 + lane];
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s = __fma_rn(-a[u], b[u], s);
+    }
+    for (; k < n; ++k) s = __fma_rn(-l[k], sU[k * 32 + lane], s);
+    s = s / l[r];
+    sU[r * 32 + lane] = s;
+    if (store) U[r + (size_t)j * ldu] = s;
   }
 }
 
@@ -681,7 +722,7 @@ static int jacobi_cluster_size(int n) {
 }
 
 template <int IT>
-static int jacobi_launch(ofrr_ctx* ctx, int n, int NC, const double* C, double* w, double* W, int descending,
+static int jacobi_launch(ofrr_ctx* ctx, int n, int NC, const double* C, double* w, double* W, int* hit, int descending,
                          int max_sweeps) {
   OFRR_TRY(allow_smem(k_jacobi_cluster<IT>));
   if (NC > 8)
@@ -699,7 +740,7 @@ static int jacobi_launch(ofrr_ctx* ctx, int n, int NC, const double* C, double* 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const int PP = ((n + 1) / 2 + NC - 1) / NC;
-  OFRR_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi_cluster<IT>, n, NC, PP, C, w, W, descending, max_sweeps));
+  OFRR_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi_cluster<IT>, n, NC, PP, C, w, W, hit, descending, max_sweeps));
   OFRR_LAUNCHED(ctx, "k_jacobi_cluster");
   return OFRR_SUCCESS;
 }
@@ -710,7 +751,8 @@ static int geig_cluster(ofrr_ctx* ctx, const GeigParams& P, int NC) {
   const int n = P.n;
   const size_t nn = (size_t)n * n;
   double *C = ws_get<double>(ctx, nn, &st), *W = ws_get<double>(ctx, nn, &st);
-  if (!C || !W) return st;
+  int* hit = ws_get<int>(ctx, (size_t)n, &st);
+  if (!C || !W || !hit) return st;
   const unsigned g = (unsigned)std::min<size_t>((nn + 255) / 256, 152);
   double *L = nullptr, *Y = nullptr;
   if (P.M) {
@@ -720,8 +762,8 @@ static int geig_cluster(ofrr_ctx* ctx, const GeigParams& P, int NC) {
     k_sym_copy<<<g, 256, 0, ctx->stream>>>(n, P.G, P.ldg, P.symmetrize, W);
     OFRR_LAUNCHED(ctx, "k_sym_copy");
     OFRR_TRY(small_chol(ctx, n, P.M, P.ldm, L));
-    OFRR_TRY(small_trsm(ctx, n, L, W, 0, Y, 0));  // Y = L^-1 G
-    OFRR_TRY(small_trsm(ctx, n, L, Y, 1, W, 0));  // W = L^-1 Y' = L^-1 G L^-T
+    OFRR_TRY(small_trsm(ctx, n, L, W, 0, Y));  // Y = L^-1 G
+    OFRR_TRY(small_trsm(ctx, n, L, Y, 1, W));  // W = L^-1 Y' = L^-1 G L^-T
     k_sym_copy<<<g, 256, 0, ctx->stream>>>(n, W, n, 1, C);
     OFRR_LAUNCHED(ctx, "k_sym_copy");
   } else {
@@ -733,17 +775,18 @@ static int geig_cluster(ofrr_ctx* ctx, const GeigParams& P, int NC) {
   const int PP = ((n + 1) / 2 + NC - 1) / NC, items = (n + (n & 1)) * PP;
   if (items > 2 * kJacT || 4 * PP * NC > kJacT) return OFRR_ERR_INTERNAL;
   if (items <= kJacT)
-    OFRR_TRY(jacobi_launch<1>(ctx, n, NC, C, P.w, Wj, P.descending, P.max_sweeps));
+    OFRR_TRY(jacobi_launch<1>(ctx, n, NC, C, P.w, Wj, hit, P.descending, P.max_sweeps));
   else
-    OFRR_TRY(jacobi_launch<2>(ctx, n, NC, C, P.w, Wj, P.descending, P.max_sweeps));
-  double* Uc = Wj;
+    OFRR_TRY(jacobi_launch<2>(ctx, n, NC, C, P.w, Wj, hit, P.descending, P.max_sweeps));
   if (P.M) {
-    Uc = (P.ldu == n) ? P.U : Y;
-    OFRR_TRY(small_trsm(ctx, n, L, W, 0, Uc, 1));  // U = L^-T W
-  }
-  if (Uc != P.U)
-    OFRR_CUDA(cudaMemcpy2DAsync(P.U, P.ldu * sizeof(double), Uc, n * sizeof(double), n * sizeof(double), n,
+    const size_t smem = sizeof(double) * (nn + (size_t)32 * n);
+    OFRR_TRY(allow_smem(k_back_subst));
+    k_back_subst<<<(unsigned)((n + 31) / 32), 32, smem, ctx->stream>>>(n, L, W, hit, P.U, P.ldu);  // U = L^-T W
+    OFRR_LAUNCHED(ctx, "k_back_subst");
+  } else if (Wj != P.U) {
+    OFRR_CUDA(cudaMemcpy2DAsync(P.U, P.ldu * sizeof(double), Wj, n * sizeof(double), n * sizeof(double), n,
                                 cudaMemcpyDeviceToDevice, ctx->stream));
+  }
   return OFRR_SUCCESS;
 }
 

@@ -674,9 +674,9 @@ int small_chol(ofrr_ctx* ctx, int n, const double* M, int ldm, double* L) {
   if (n > 160) return OFRR_ERR_BLAS_INVALID_SIZE;
   return chol<true>(ctx, n, 1, &M, ldm, 0.0, &L);
 }
-int small_trsm(ofrr_ctx* ctx, int n, const double* L, const double* B, int transB, double* X, int upper) {
+int small_trsm(ofrr_ctx* ctx, int n, const double* L, const double* B, int transB, double* X) {
   if (n > 160) return OFRR_ERR_BLAS_INVALID_SIZE;
-  return trsm<true>(ctx, n, n, L, B, n, transB, X, upper);
+  return trsm<true>(ctx, n, n, L, B, n, transB, X, 0);
 }
 
 // Ogita-Aishima refinement of approximate eigenvectors W0 (n x n, overwritten) of a symmetric C
