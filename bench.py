@@ -282,7 +282,7 @@ def sliced_roofline(api, reps=20):
     """Live CUDA-event timing of the dominant kernel of the solve, the fused exact-slice product
     k_sliced_tn, on the solver's A V shape (C 8192 x 64 = A_op' V, A_op the 5-digit stack of A',
     K = 2048): the library slices both operands once and times reps launches of the kernel alone
-    on its stream.  The A digit stack (168 MB) is larger than L2, so every launch streams it."""
+    on its stream.  The A digit stack is 84 MB (one byte per digit)."""
     import torch
     import ctypes as C
     from mixedprecisionofrr_gb300 import _lib as L
@@ -932,11 +932,14 @@ def main():
         src = "measured" if "hbm_gbs" in peaks else "fallback"
         dt_s, bytes_s = sliced_roofline(api)
         bb = CFG["mixed"][0]
-        roof = {"kernel": f"k_sliced_tn: exact-slice FP64 A.V, 8192x{bb} = (5-digit A' 2048x8192)' V", "bound": "hbm",
-                "achieved": bytes_s / dt_s / 1e9, "peak": hbm_peak, "unit": "GB/s",
-                "frac": bytes_s / dt_s / 1e9 / hbm_peak, "traffic": profiled_traffic() if bb == 64 else None,
+        # 15 BF16 digit pairs per FP64 product: bound by the tensor pipe, with the bytes it moves beside it
+        tc_peak = peaks.get("bf16_tflops", 1900.0)
+        tflops = 15 * 2.0 * M_ROWS * N_COLS * bb / dt_s / 1e12
+        roof = {"kernel": f"k_sliced_tn: exact-slice FP64 A.V, 8192x{bb} = (5-digit A' 2048x8192)' V", "bound": "tensor",
+                "achieved": tflops, "peak": tc_peak, "unit": "TFLOP/s", "frac": tflops / tc_peak,
+                "hbm_frac": bytes_s / dt_s / 1e9 / hbm_peak, "traffic": profiled_traffic() if bb == 64 else None,
                 "algorithmic_bytes": bytes_s, "peak_source": src, "us_per_launch": dt_s * 1e6}
-        # the same launch against the FP64 operands it stands for (A 8 B per element instead of its 10 B digit
+        # the same launch against the FP64 operands it stands for (A 8 B per element instead of its 5 B digit
         # stack, V and the FP64 result C once)
         fp64_bytes = 8.0 * (M_ROWS * N_COLS + N_COLS * bb + M_ROWS * bb)
         roof["frac_fp64_operand"] = fp64_bytes / dt_s / 1e9 / hbm_peak

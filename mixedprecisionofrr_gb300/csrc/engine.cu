@@ -47,7 +47,8 @@ size_t request_charge(const ofrr_request& r) {
   const size_t b = (size_t)(r.opt.block > 0 ? r.opt.block : 1);
   size_t bytes = (size_t)64 << 20;  // small matrices, flags, first workspace chunk
   if (A.kind == OFRR_OP_DENSE) {
-    // 16-bit copies of A and A', exact-slice digit stacks of both orientations, an FP64 A' transient
+    // 16-bit copies of A and A', exact-slice digit stacks of both orientations (5 bytes an element, padded to 64 x 128
+    // blocks: at most 10), an FP64 A' transient
     bytes += m * n * (2 + 2 + 10 + 10 + 8);
   } else {
     bytes += (size_t)A.csr.nnz * 8;

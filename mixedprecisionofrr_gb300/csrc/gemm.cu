@@ -205,7 +205,7 @@ int gemm_impl(ofrr_ctx* ctx, int transA, int transB, ofrr_dtype ta, ofrr_dtype t
       }
       return OFRR_SUCCESS;
     }
-    SlicedOperand As;
+    SlicedLeft As;
     if (transA == 1) {
       OFRR_TRY(sliced_prepare(ctx, K, M, (const double*)A, lda, &As));
     } else {

@@ -551,25 +551,37 @@ int residual_columns2(ofrr_ctx* ctx, int64_t m, int64_t n, const double* AV, con
 int column_norms(ofrr_ctx* ctx, ofrr_dtype t, int64_t m, int64_t n, const void* X, int64_t ldx,
                  double* out_dev);
 // exact-slice FP64 emulation (sliced.cu): digit stacks of a fixed K x M FP64 operand and the
-// product C (M x N) = X' B with X the prepared operand and B (K x N) FP64
-struct SlicedOperand {
+// product C (M x N) = X' B with X the prepared left operand and B (K x N) FP64.  The left operand (the large one) keeps
+// its digits in one byte each, the right one in BF16.
+template <class TD>
+struct SlicedDigits {
   int64_t K = 0, Kp = 0, M = 0;
-  __nv_bfloat16* stack = nullptr;
+  TD* stack = nullptr;
   int* expo = nullptr;
 };
+using SlicedOperand = SlicedDigits<__nv_bfloat16>;
+using SlicedLeft = SlicedDigits<uint8_t>;
 constexpr int kSliceDigits = 5;
-int sliced_prepare(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, int64_t ldx, SlicedOperand* out);
-int sliced_prepare_into(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, int64_t ldx, __nv_bfloat16* stack,
-                        int* expo, SlicedOperand* out);
+// elements of a digit stack of M columns of Kp entries (the packed one is laid out in blocks of 128 columns)
+template <class TD>
+inline size_t sliced_digits(int64_t M, int64_t Kp) {
+  const int64_t cols = (sizeof(TD) == 1 && M > 128) ? (M + 127) / 128 * 128 : M;
+  return (size_t)cols * kSliceDigits * Kp;
+}
+template <class TD>
+int sliced_prepare(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, int64_t ldx, SlicedDigits<TD>* out);
+template <class TD>
+int sliced_prepare_into(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, int64_t ldx, TD* stack, int* expo,
+                        SlicedDigits<TD>* out);
 // scalecols (FAST, FP64) fused with the digit split of the scaled columns: U (m x n) is scaled in place
 // and *out describes its digit stack in caller buffers (n * 5 * roundup(m, 64) bf16, n ints); m <= 8192
 int scalecols_sliced(ofrr_ctx* ctx, int64_t m, int64_t n, double* U, int64_t ldu, __nv_bfloat16* stack, int* expo,
                      SlicedOperand* out);
 // C (M x N) = A_op' B with both operands already split (B.K == A.K, N = B.M)
-int sliced_gemm_tn_pre(ofrr_ctx* ctx, const SlicedOperand& A, const SlicedOperand& B, double* C, int64_t ldc);
-int sliced_gemm_scalecols_pre(ofrr_ctx* ctx, const SlicedOperand& A, const SlicedOperand& B, double* U, int64_t ldu,
+int sliced_gemm_tn_pre(ofrr_ctx* ctx, const SlicedLeft& A, const SlicedOperand& B, double* C, int64_t ldc);
+int sliced_gemm_scalecols_pre(ofrr_ctx* ctx, const SlicedLeft& A, const SlicedOperand& B, double* U, int64_t ldu,
                               bool write_u, __nv_bfloat16* stack, int* expo, SlicedOperand* out);
-int sliced_gemm_tn(ofrr_ctx* ctx, const SlicedOperand& A, int64_t N, const double* B, int64_t ldb, double* C,
+int sliced_gemm_tn(ofrr_ctx* ctx, const SlicedLeft& A, int64_t N, const double* B, int64_t ldb, double* C,
                    int64_t ldc);
 
 int residual_columns(ofrr_ctx* ctx, int64_t m, int64_t n, const double* AX, int64_t ldax,

@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <vector>
 
 namespace ofrr {
@@ -25,8 +26,8 @@ constexpr int BETA = 7;  // digit width: |leading digit| <= 128, later digits <=
 constexpr int S = 5;     // digits per operand (35 bits)
 constexpr int LMAX = 4;  // levels kept: pairs with s + t <= 4 (15 of 25), error ~ 2^-35
 
-// Digits of every column of X (K x N, column-major).  Stacked layout: column n occupies
-// stack[(n * S + s) * Kp + k] for digit s; rows k >= K are zero.  expo[n] = exponent e_n.
+// Digits of every column of X (K x N, column-major), as BF16 or packed in bytes (slice_pack, with its own layout).  BF16
+// layout: column n occupies stack[(n * S + s) * Kp + k] for digit s; rows k >= K are zero.  expo[n] = exponent e_n.
 // Integer pipes only (GB300's FP64 pipe is 1/64 rate): the column maximum is taken on the bit
 // patterns of |x|, e_n = frexp exponent of that maximum, and round(x 2^(BETA S - e_n)) is formed from
 // the significand by a right shift with round-half-even (the same value __double2ll_rn gives).
@@ -91,9 +92,9 @@ __device__ __forceinline__ int colmax_expo(unsigned long long m) {
   return (m == 0) ? 0 : (bm > 0) ? bm - 1022 : (64 - __clzll((long long)m)) - 1074;
 }
 
-// The S digits of one entry (bit pattern `bits`) of a column with exponent e, stored at col[s * Kp + k]
-__device__ __forceinline__ void slice_store(unsigned long long bits, int e, __nv_bfloat16* __restrict__ col, int64_t Kp,
-                                            int64_t k) {
+// The S digits of one entry (bit pattern `bits`) of a column with exponent e: d[0] in [-128, 128], the others in
+// [-64, 63]
+__device__ __forceinline__ void slice_digits(unsigned long long bits, int e, int (&dg)[S]) {
   // x = M 2^(be' - 1075) with M the significand (implicit bit for normal numbers, be' = max(be, 1))
   const int be = (int)((bits >> 52) & 0x7ff);
   const unsigned long long M = (bits & 0x000fffffffffffffull) | (be > 0 ? (1ull << 52) : 0ull);
@@ -114,31 +115,85 @@ __device__ __forceinline__ void slice_store(unsigned long long bits, int e, __nv
   for (int s = S - 1; s > 0; --s) {  // centred base-2^BETA digits, least significant first
     const long long d = ((r + (1 << (BETA - 1))) & ((1 << BETA) - 1)) - (1 << (BETA - 1));
     r = (r - d) >> BETA;  // exact: r - d is a multiple of 2^BETA
-    col[(size_t)s * Kp + k] = __float2bfloat16_rn((float)(int)d);  // |d| <= 64
+    dg[s] = (int)d;
   }
-  col[k] = __float2bfloat16_rn((float)(int)r);  // leading digit, |r| <= 128: exact in bf16
+  dg[0] = (int)r;
 }
 
+// The digits as BF16 at col[s * Kp + k] (the right operand of a product); |d| <= 128 is exact in BF16
+__device__ __forceinline__ void slice_store(unsigned long long bits, int e, __nv_bfloat16* __restrict__ col, int64_t Kp,
+                                            int64_t k) {
+  int dg[S];
+  slice_digits(bits, e, dg);
+#pragma unroll
+  for (int s = 0; s < S; ++s) col[(size_t)s * Kp + k] = __float2bfloat16_rn((float)dg[s]);
+}
+
+// The digits in five bytes (the left operand): plane s >= 1 holds d_s + 64 in seven bits, plane 0 the upper eight
+// bits of d_0 + 128 (0 .. 256) and plane 1's top bit its last one.  V consecutive entries, one store per plane.
+// Layout: the planes of pack_rows(N) columns x 64 entries that one CTA of the product reads at a time are adjacent,
+// stack[(((n / R) * Kp / 64 + k / 64) * S + s) * R * 64 + (n % R) * 64 + (k % 64 ^ pack_swz(n % R))] with
+// R = pack_rows(N); pack_swz permutes a row's four 16-byte chunks so that eight rows fall on different banks.
+__host__ __device__ inline int pack_rows(int64_t N) { return N < tc::BM ? (int)N : tc::BM; }
+__host__ __device__ inline int pack_swz(int row) { return ((row >> 1) & 3) << 4; }
+__device__ __forceinline__ uint8_t* pack_col(uint8_t* stack, int64_t N, int64_t Kp, int64_t n) {
+  const int R = pack_rows(N);
+  return stack + (n / R) * (size_t)R * S * Kp + (n % R) * 64;
+}
+template <int V>
+__device__ __forceinline__ void slice_pack(const unsigned long long* bits, int e, uint8_t* __restrict__ col, int R,
+                                           int swz, int64_t k) {
+  static_assert(V == 1 || V == 2 || V == 4, "entries per store");
+  unsigned pl[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) pl[s] = 0;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    int dg[S];
+    slice_digits(bits[v], e, dg);
+    const unsigned lead = (unsigned)(dg[0] + 128);
+    pl[0] |= (lead >> 1) << (8 * v);
+    pl[1] |= ((unsigned)(dg[1] + 64) | (lead & 1u) << 7) << (8 * v);
+#pragma unroll
+    for (int s = 2; s < S; ++s) pl[s] |= (unsigned)(dg[s] + 64) << (8 * v);
+  }
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    uint8_t* p = col + ((size_t)(k >> 6) * S + s) * (R * 64) + ((int)(k & 63) ^ swz);
+    if constexpr (V == 4) *reinterpret_cast<unsigned*>(p) = pl[s];
+    else if constexpr (V == 2) *reinterpret_cast<unsigned short*>(p) = (unsigned short)pl[s];
+    else *p = (uint8_t)pl[s];
+  }
+}
+
+// TD: __nv_bfloat16 (one digit each) or uint8_t (packed; a thread takes SLICE_U consecutive entries)
+template <class TD>
 __global__ void __launch_bounds__(SLICE_T) k_slice_digits(int64_t K, int64_t Kp, int64_t N, const double* __restrict__ X,
                                                           int64_t ldx, const unsigned long long* __restrict__ colmax,
-                                                          __nv_bfloat16* __restrict__ stack, int* __restrict__ expo) {
-  const int64_t k0 = (int64_t)blockIdx.x * SLICE_CHUNK + threadIdx.x;
+                                                          TD* __restrict__ stack, int* __restrict__ expo) {
+  constexpr bool PACK = std::is_same<TD, uint8_t>::value;
+  constexpr int64_t STEP = PACK ? 1 : SLICE_T;
+  const int64_t k0 = (int64_t)blockIdx.x * SLICE_CHUNK + (PACK ? SLICE_U * threadIdx.x : threadIdx.x);
   for (int64_t n = blockIdx.y; n < N; n += gridDim.y) {
     const int e = colmax_expo(colmax[n]);
     if (blockIdx.x == 0 && threadIdx.x == 0) expo[n] = e;
     const double* x = X + n * ldx;
-    __nv_bfloat16* col = stack + (size_t)n * S * Kp;
     unsigned long long v[SLICE_U];
 #pragma unroll
     for (int u = 0; u < SLICE_U; ++u) {
-      const int64_t k = k0 + (int64_t)u * SLICE_T;
+      const int64_t k = k0 + (int64_t)u * STEP;
       v[u] = (k < K) ? (unsigned long long)__double_as_longlong(x[k]) : 0ull;
     }
+    if constexpr (PACK) {
+      if (k0 < Kp) slice_pack<SLICE_U>(v, e, pack_col(stack, N, Kp, n), pack_rows(N), pack_swz((int)(n % pack_rows(N))), k0);
+    } else {
+      TD* col = stack + (size_t)n * S * Kp;
 #pragma unroll
-    for (int u = 0; u < SLICE_U; ++u) {
-      const int64_t k = k0 + (int64_t)u * SLICE_T;
-      if (k >= Kp) break;
-      slice_store(v[u], e, col, Kp, k);
+      for (int u = 0; u < SLICE_U; ++u) {
+        const int64_t k = k0 + (int64_t)u * STEP;
+        if (k >= Kp) break;
+        slice_store(v[u], e, col, Kp, k);
+      }
     }
   }
 }
@@ -147,10 +202,11 @@ __global__ void __launch_bounds__(SLICE_T) k_slice_digits(int64_t K, int64_t Kp,
 // registers, takes its maximum with a block reduction and writes the digits (no second read, no
 // atomics, no zeroed scratch).
 constexpr int SC_T = 512;
-template <int U, int T = SC_T>
+template <class TD, int U, int T = SC_T>
 __global__ void __launch_bounds__(T) k_slice_cols(int64_t K, int64_t Kp, int64_t N, const double* __restrict__ X,
-                                                  int64_t ldx, __nv_bfloat16* __restrict__ stack,
-                                                  int* __restrict__ expo) {
+                                                  int64_t ldx, TD* __restrict__ stack, int* __restrict__ expo) {
+  constexpr bool PACK = std::is_same<TD, uint8_t>::value;
+  constexpr int V = PACK ? (U < 4 ? U : 4) : 1;  // consecutive entries of a thread
   __shared__ unsigned long long red[T / 32];
   for (int64_t n = blockIdx.x; n < N; n += gridDim.x) {
     const double* x = X + n * ldx;
@@ -158,7 +214,7 @@ __global__ void __launch_bounds__(T) k_slice_cols(int64_t K, int64_t Kp, int64_t
     unsigned long long mx = 0;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int64_t k = threadIdx.x + (int64_t)u * T;
+      const int64_t k = ((int64_t)threadIdx.x + (int64_t)(u / V) * T) * V + u % V;
       v[u] = (k < K) ? (unsigned long long)__double_as_longlong(x[k]) : 0ull;
       mx = max(mx, v[u] & 0x7fffffffffffffffull);
     }
@@ -169,11 +225,16 @@ __global__ void __launch_bounds__(T) k_slice_cols(int64_t K, int64_t Kp, int64_t
     for (int w = 0; w < T / 32; ++w) mx = max(mx, red[w]);
     const int e = colmax_expo(mx);
     if (threadIdx.x == 0) expo[n] = e;
-    __nv_bfloat16* col = stack + (size_t)n * S * Kp;
+    TD* col;
+    if constexpr (PACK) col = pack_col(stack, N, Kp, n);
+    else col = stack + (size_t)n * S * Kp;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int64_t k = threadIdx.x + (int64_t)u * T;
-      if (k < Kp) slice_store(v[u], e, col, Kp, k);
+    for (int u = 0; u < U; u += V) {
+      const int64_t k = ((int64_t)threadIdx.x + (int64_t)(u / V) * T) * V;
+      if (k < Kp) {
+        if constexpr (PACK) slice_pack<V>(v + u, e, col, pack_rows(N), pack_swz((int)(n % pack_rows(N))), k);
+        else slice_store(v[u], e, col, Kp, k);
+      }
     }
     __syncthreads();  // red is reused by the next column
   }
@@ -319,45 +380,93 @@ __global__ void __launch_bounds__(SCS_T) k_scalecols_slice(int64_t m, int64_t Kp
 
 // Fused exact-slice product.  One CTA owns a 128 x SBN tile of C and a range of at most 16 k-blocks
 // (1024 entries of K, so that the level-0 and level-1 FP32 sums are exact).  Per k-block the B digits
-// d'_0..d'_4 (5 tiles) are loaded once into a B slot, and the A digits d_0..d_4 stream through an
-// A ring one tile at a time; for A digit s the MMA warp issues the pairs (s, t), t <= LMAX - s,
+// d'_0..d'_4 (5 tiles) are loaded once into a B slot and the A digits arrive packed in five bytes an entry (5 planes
+// of 128 x 64 bytes).  Groups of four warps unpack them, plane by plane, into BF16 tiles in TMEM, from where the MMA
+// reads its A operand; for A digit s the MMA warp issues the pairs (s, t), t <= LMAX - s,
 // into the TMEM accumulator of level L = s + t (5 accumulators of SBN columns), as one wide MMA.  A is therefore read
 // once per product (not once per level).  The epilogue converts each level to an integer, combines
 // acc = sum_L S_L 2^(BETA (LMAX - L)) exactly in 64 bits and writes it (one split) as
 // C = 2^(ea + eb - BETA (LMAX + 2)) acc, or as an int64 partial for k_sliced_finish.
+//
+// Unpacking costs one PRMT and one packed subtraction per two digits: the byte u becomes the low byte of the BF16
+// 0x43uu = 128 + u, and 128 + 64 is subtracted exactly; plane 0 is 2 (128 + u) - 384 plus plane 1's top bit.
+// What bounds it: the MMAs, 15 digit pairs of 128 x 64 x 64 per k-block = 1920 cycles of the ~2150 a k-block takes;
+// a launch adds ~2 us until the first tile is unpacked and ~2.5 us of epilogue.  8192 x 64 x 2048 went from 47 to
+// 26 us: with BF16 A digits (168 MB, beyond L2) by TMA and one lane building a descriptor per MMA, issue took ~4900
+// cycles per k-block; issued by an elected lane of a converged warp from running descriptors and with the digits in
+// bytes (84 MB) it took ~3300, bound by shared memory (the unpacked tiles were written there and read again); with the
+// unpacked tiles in TMEM shared memory carries only the packed planes and B.
 constexpr int SBN = 64;
-constexpr int SL_ATILE = tc::BM * tc::BK * 2;  // 16 KB: one digit of a 128-row k-block
-constexpr int SL_BTILE = SBN * tc::BK * 2;     // 8 KB
+constexpr int SL_ACOLS = tc::BK / 2;        // TMEM columns of one A digit tile (two BF16 each)
+constexpr int SL_RPLANE = tc::BM * tc::BK;  // 8 KB: one packed digit plane of a 128-row k-block
+constexpr int SL_BTILE = SBN * tc::BK * 2;  // 8 KB
 constexpr int SL_ASLOTS = 6;
+constexpr int SL_RSLOTS = 3;
 constexpr int SL_BSLOTS = 2;
-constexpr int SL_THREADS = 192;
+constexpr int SL_GROUPS = 4;  // groups of four unpacking warps (warps 2 ..), the epilogue afterwards
+constexpr int SL_THREADS = 64 + 128 * SL_GROUPS;
 constexpr int SL_KB_MAX = 16;
 constexpr int SL_SHIFT = BETA * (LMAX + 2);
-constexpr size_t SL_SMEM = (size_t)SL_ASLOTS * SL_ATILE + (size_t)SL_BSLOTS * S * SL_BTILE + 1024 + 256;
-constexpr uint32_t SL_TMEM_COLS = 512;  // LMAX + 1 accumulators of SBN columns, rounded to a power of two
-static_assert((LMAX + 1) * SBN <= (int)SL_TMEM_COLS, "TMEM columns");
+constexpr size_t SL_SMEM = (size_t)SL_BSLOTS * S * SL_BTILE + (size_t)SL_RSLOTS * S * SL_RPLANE + 1024 + 256;
+constexpr uint32_t SL_TMEM_COLS = 512;
+constexpr int SL_ABASE = (LMAX + 1) * SBN;  // LMAX + 1 accumulators of SBN columns, then the A ring
+static_assert(SL_ABASE + SL_ASLOTS * SL_ACOLS <= (int)SL_TMEM_COLS, "TMEM columns");
+static_assert(SL_GROUPS <= S && SBN == 16 * SL_GROUPS, "every group meets every k-block; epilogue columns");
 
 // instruction descriptor with its N field (bits 17-22, N >> 3) replaced
 __device__ __forceinline__ uint32_t idesc_with_n(uint32_t idesc, int n) {
   return (idesc & ~(0x3Fu << 17)) | ((uint32_t)(n >> 3) << 17);
 }
 
+// two packed bytes (selected by `sel`, top bits cleared by the caller) of a plane s >= 1 as two BF16 digits
+__device__ __forceinline__ unsigned bf2_bits(__nv_bfloat162 x) { return *reinterpret_cast<unsigned*>(&x); }
+__device__ __forceinline__ __nv_bfloat162 bf2(unsigned x) { return *reinterpret_cast<__nv_bfloat162*>(&x); }
+__device__ __forceinline__ unsigned unpack2(unsigned w, unsigned sel) {
+  return bf2_bits(__hsub2(bf2(__byte_perm(w, 0x43434343u, sel)), __floats2bfloat162_rn(192.f, 192.f)));
+}
+// the leading digits: two bytes of plane 0 and the top bits (0 or 1) of two of plane 1
+__device__ __forceinline__ unsigned unpack2_lead(unsigned w, unsigned l, unsigned sel) {
+  const __nv_bfloat162 x = __hfma2(bf2(__byte_perm(w, 0x43434343u, sel)), __floats2bfloat162_rn(2.f, 2.f),
+                                   __floats2bfloat162_rn(-384.f, -384.f));
+  return bf2_bits(__hadd2(x, bf2(__byte_perm(l, 0u, sel) * 0x3f80u)));
+}
+
+// size bytes (a multiple of 16, both addresses 16-byte aligned) into shared memory
+__device__ __forceinline__ void bulk_load(uint64_t* bar, void* dst, const void* src, int size) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   tc::smem_u32(dst)),
+               "l"(src), "r"(size), "r"(tc::smem_u32(bar))
+               : "memory");
+}
+
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+  long long d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
+}
+
 __global__ void __launch_bounds__(SL_THREADS, 1)
-    k_sliced_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
+    k_sliced_tn(const uint8_t* __restrict__ Ap, const __grid_constant__ CUtensorMap tmB, int M, int N,
                 int64_t Kp, int kb_total, int kb_per_split, uint32_t idesc, long long* __restrict__ partial,
                 double* __restrict__ C, int64_t ldc, const int* __restrict__ ea, const int* __restrict__ eb,
                 int* __restrict__ err) {
   using namespace tc;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sA = base;
-  uint8_t* sB = base + SL_ASLOTS * SL_ATILE;
-  uint64_t* bars = (uint64_t*)(sB + SL_BSLOTS * S * SL_BTILE);
-  uint64_t* a_full = bars;
-  uint64_t* a_empty = bars + SL_ASLOTS;
+  uint8_t* sB = base;
+  uint8_t* sR = sB + SL_BSLOTS * S * SL_BTILE;
+  uint64_t* bars = (uint64_t*)(sR + SL_RSLOTS * S * SL_RPLANE);
+  uint64_t* a_full = bars;                // unpacked tiles: four warps' arrivals
+  uint64_t* a_empty = bars + SL_ASLOTS;   // read by the MMA (commit)
   uint64_t* b_full = bars + 2 * SL_ASLOTS;
   uint64_t* b_empty = b_full + SL_BSLOTS;
-  uint64_t* accum = b_empty + SL_BSLOTS;
+  uint64_t* r_full = b_empty + SL_BSLOTS;  // packed planes
+  uint64_t* r_empty = r_full + SL_RSLOTS;  // unpacked: every warp's arrival
+  uint64_t* accum = r_empty + SL_RSLOTS;
   uint32_t* tmem_slot = (uint32_t*)(accum + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -365,15 +474,21 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
   const int kb0 = blockIdx.z * kb_per_split;
   const int kb1 = min(kb0 + kb_per_split, kb_total);
   const int nkb = max(kb1 - kb0, 0);
+  const int rplane = pack_rows(M) * 64;  // bytes of one packed plane of a k-block
+  const uint8_t* Ablk = Ap + (size_t)blockIdx.x * kb_total * S * rplane;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < SL_ASLOTS; ++i) {
-      mbar_init(&a_full[i], 1);
+      mbar_init(&a_full[i], 4);
       mbar_init(&a_empty[i], 1);
     }
     for (int i = 0; i < SL_BSLOTS; ++i) {
       mbar_init(&b_full[i], 1);
       mbar_init(&b_empty[i], 1);
+    }
+    for (int i = 0; i < SL_RSLOTS; ++i) {
+      mbar_init(&r_full[i], 1);
+      mbar_init(&r_empty[i], 4 * SL_GROUPS);
     }
     mbar_init(accum, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -391,113 +506,161 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmA) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmB) : "memory");
-      int a_issued = 0, b_issued = 0;
-      bool ok = true;
-      for (int i = 0; i < nkb && ok; ++i) {
-        const int bs = i % SL_BSLOTS;
-        if (i >= SL_BSLOTS && !mbar_wait(&b_empty[bs], ((i / SL_BSLOTS) + 1) & 1, err, 21)) break;
+      int r_issued = 0, b_issued = 0;
+      for (int i = 0; i < nkb; ++i) {
+        const int rs = i % SL_RSLOTS, bs = i % SL_BSLOTS;
         const int kx = (kb0 + i) * BK;
+        if (i >= SL_RSLOTS && !mbar_wait(&r_empty[rs], ((i / SL_RSLOTS) + 1) & 1, err, 22)) break;
+        mbar_expect_tx(&r_full[rs], S * rplane);
+        bulk_load(&r_full[rs], sR + rs * S * SL_RPLANE, Ablk + (size_t)(kb0 + i) * S * rplane, S * rplane);
+        r_issued = i + 1;
+        if (i >= SL_BSLOTS && !mbar_wait(&b_empty[bs], ((i / SL_BSLOTS) + 1) & 1, err, 21)) break;
         mbar_expect_tx(&b_full[bs], S * SL_BTILE);
         for (int t = 0; t < S; ++t)
           tma_load_2d(&tmB, &b_full[bs], sB + (bs * S + t) * SL_BTILE, (int)(t * Kp) + kx, n0);
         b_issued = i + 1;
-        for (int s = 0; s < S; ++s) {
-          const int as = a_issued % SL_ASLOTS;
-          if (a_issued >= SL_ASLOTS && !mbar_wait(&a_empty[as], ((a_issued / SL_ASLOTS) + 1) & 1, err, 22)) {
-            ok = false;
-            break;
-          }
-          mbar_expect_tx(&a_full[as], SL_ATILE);
-          tma_load_2d(&tmA, &a_full[as], sA + as * SL_ATILE, (int)(s * Kp) + kx, m0);
-          ++a_issued;
-        }
       }
       // drain: every issued copy must have landed before the CTA may exit
-      for (int j = max(0, a_issued - SL_ASLOTS); j < a_issued; ++j)
-        mbar_wait(&a_full[j % SL_ASLOTS], (j / SL_ASLOTS) & 1, err, 23);
+      for (int j = max(0, r_issued - SL_RSLOTS); j < r_issued; ++j)
+        mbar_wait(&r_full[j % SL_RSLOTS], (j / SL_RSLOTS) & 1, err, 23);
       for (int j = max(0, b_issued - SL_BSLOTS); j < b_issued; ++j)
         mbar_wait(&b_full[j % SL_BSLOTS], (j / SL_BSLOTS) & 1, err, 24);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int a_used = 0;
-      bool ok = true;
-      for (int i = 0; i < nkb && ok; ++i) {
-        const int bs = i % SL_BSLOTS;
-        if (!mbar_wait(&b_full[bs], (i / SL_BSLOTS) & 1, err, 25)) break;
+    // The whole warp walks the unrolled loop and one elected lane issues: addresses stay warp-uniform.  Issuing from
+    // one lane's branch with descriptors rebuilt per MMA took ~1000 cycles per A digit, the MMAs themselves 128 to 640.
+    const bool leader = elect_one();
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t b_base = smem_u32(sB) >> 4;
+    uint32_t as = 0, aph = 0, acc = 0;
+    bool ok = true;
+    for (int i = 0; i < nkb && ok; ++i) {
+      const uint32_t bs = (uint32_t)i % SL_BSLOTS;
+      if (!mbar_wait(&b_full[bs], (i / SL_BSLOTS) & 1, err, 25)) break;
+      const uint32_t b0 = b_base + bs * (S * SL_BTILE >> 4);
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        if (ok && !mbar_wait(&a_full[as], aph, err, 26)) ok = false;
         fence_after();
-        for (int s = 0; s < S; ++s) {
-          const int as = a_used % SL_ASLOTS;
-          if (!mbar_wait(&a_full[as], (a_used / SL_ASLOTS) & 1, err, 26)) {
-            ok = false;
-            break;
-          }
-          fence_after();
-          // A digit s against the B digits 0..LMAX-s at once: the slot's B tiles are adjacent rows of
-          // one K-major operand and the level accumulators s..LMAX adjacent TMEM columns, so one MMA
-          // of N = (LMAX-s+1) SBN (at most 256; the rest in a second MMA) replaces LMAX-s+1 MMAs
-          const uint32_t a0 = smem_u32(sA + as * SL_ATILE);
-          const uint32_t b0 = smem_u32(sB + (bs * S) * SL_BTILE);
-          const int nt = LMAX - s + 1;
-          const int n1 = nt < 4 ? nt : 4;
-          const uint32_t id1 = idesc_with_n(idesc, n1 * SBN), id2 = idesc_with_n(idesc, (nt - n1) * SBN);
-          const uint32_t d = tmem + (uint32_t)(s * SBN);
+        // A digit s against the B digits 0..LMAX-s at once: the slot's B tiles are adjacent rows of
+        // one K-major operand and the level accumulators s..LMAX adjacent TMEM columns, so one MMA
+        // of N = (LMAX-s+1) SBN (at most 256; the rest in a second MMA) replaces LMAX-s+1 MMAs
+        constexpr int NMAX = 4;
+        const int nt = LMAX - s + 1, n1 = nt < NMAX ? nt : NMAX;
+        const uint32_t a0 = tm + SL_ABASE + as * SL_ACOLS, d = tm + (uint32_t)(s * SBN);
+        if (leader && ok) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
-            const uint32_t acc = (i > 0 || s > 0 || k > 0) ? 1u : 0u;
-            umma_f16(d, desc_sw128(a0 + 32 * k), desc_sw128(b0 + 32 * k), id1, acc);
+            umma_f16_ts(d, a0 + 8 * k, b0 + 2 * k, idesc_with_n(idesc, n1 * SBN), acc);
             if (nt > n1)
-              umma_f16(d + (uint32_t)(n1 * SBN), desc_sw128(a0 + 32 * k), desc_sw128(b0 + n1 * SL_BTILE + 32 * k),
-                       id2, acc);
+              umma_f16_ts(d + (uint32_t)(n1 * SBN), a0 + 8 * k, b0 + (n1 * SL_BTILE >> 4) + 2 * k,
+                          idesc_with_n(idesc, (nt - n1) * SBN), acc);
+            acc = 1;
           }
           umma_commit(&a_empty[as]);
-          ++a_used;
         }
-        umma_commit(&b_empty[bs]);
+        __syncwarp();
+        if (++as == SL_ASLOTS) {
+          as = 0;
+          aph ^= 1;
+        }
+        acc = 1;
       }
-      umma_commit(accum);
+      if (leader) umma_commit(&b_empty[bs]);
+      __syncwarp();
     }
+    if (leader) umma_commit(accum);
     __syncwarp();
   } else {
-    // epilogue warps 2..5 -> TMEM lane quarter (warp % 4)
-    const int q = warp & 3;
-    const bool ok = mbar_wait(accum, 0, err, 27);
-    fence_after();
-    const int row = m0 + 32 * q + lane;
-    const int erow = (row < M) ? ea[row] : 0;
+    {
+      // unpack: groups of four warps take the digits in turn; a thread converts the 64 entries of one row
+      const int g = (warp - 2) >> 2, row = 32 * (warp & 3) + lane;
+      const int swz = pack_swz(row);
+      const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
+      int held = -1;  // k-block whose planes this warp is reading
+      const uint8_t* raw = sR;
 #pragma unroll 1
-    for (int c = 0; c < SBN; c += 16) {
-      long long acc[16];
+      for (int use = g; use < nkb * S; use += SL_GROUPS) {
+        const int i = use / S, s = use - i * S, as = use % SL_ASLOTS;
+        if (i != held) {
+          __syncwarp();
+          if (held >= 0 && lane == 0) mbar_arrive(&r_empty[held % SL_RSLOTS]);
+          held = i;
+          if (!__all_sync(0xffffffffu, mbar_wait(&r_full[i % SL_RSLOTS], (i / SL_RSLOTS) & 1, err, 28))) break;
+          raw = sR + (i % SL_RSLOTS) * S * SL_RPLANE + row * 64;
+        }
+        uint32_t o[SL_ACOLS];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) acc[j] = 0;
-#pragma unroll 1
-      for (int L = 0; L <= LMAX; ++L) {
-        float v[16];
-        tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(L * SBN + c), v);
-        // every level sum is an integer below 2^25 in magnitude (at most 1024 terms of at most 2^14.3)
+        for (int c = 0; c < 4; ++c) {
+          const uint4 w = *reinterpret_cast<const uint4*>(raw + s * rplane + ((c * 16) ^ swz));
+          const unsigned in[4] = {w.x, w.y, w.z, w.w};
+          if (s == 0) {
+            const uint4 w1 = *reinterpret_cast<const uint4*>(raw + rplane + ((c * 16) ^ swz));
+            const unsigned in1[4] = {w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[j] += (long long)__float2int_rn(v[j]) * (1ll << (BETA * (LMAX - L)));
-      }
-      if (!ok || nkb == 0) {
+            for (int j = 0; j < 4; ++j) {
+              const unsigned l = (in1[j] >> 7) & 0x01010101u;
+              o[8 * c + 2 * j] = unpack2_lead(in[j], l, 0x4140);
+              o[8 * c + 2 * j + 1] = unpack2_lead(in[j], l, 0x4342);
+            }
+          } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[j] = 0;
-      }
-      if (row < M) {
-        if (partial != nullptr) {
-          long long* P = partial + (size_t)blockIdx.z * (size_t)M * N;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int n = n0 + c + j;
-            if (n < N) P[row + (size_t)n * M] = acc[j];
+            for (int j = 0; j < 4; ++j) {
+              o[8 * c + 2 * j] = unpack2(in[j] & 0x7f7f7f7fu, 0x4140);
+              o[8 * c + 2 * j + 1] = unpack2(in[j] & 0x7f7f7f7fu, 0x4342);
+            }
           }
-        } else {
-#pragma unroll 4
-          for (int j = 0; j < 16; ++j) {
-            const int n = n0 + c + j;
-            if (n < N) C[row + (size_t)n * ldc] = i64_ldexp(acc[j], erow + eb[n] - SL_SHIFT);
-          }
+        }
+        if (use >= SL_ASLOTS &&
+            !__all_sync(0xffffffffu, mbar_wait(&a_empty[as], ((use / SL_ASLOTS) + 1) & 1, err, 29)))
+          break;
+        fence_after();
+        tmem_st32(tmem + lanes + (uint32_t)(SL_ABASE + as * SL_ACOLS), o);
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&a_full[as]);
+      }
+    }
+    {
+      // epilogue: TMEM lane quarter warp % 4, 16 columns per group of four warps
+      const int q = warp & 3, c = ((warp - 2) >> 2) * 16;
+      const int row = m0 + 32 * q + lane;
+      const int erow = (row < M) ? ea[row] : 0;
+      const int ecol = (lane < 16 && n0 + c + lane < N) ? eb[n0 + c + lane] : 0;
+      const bool ok = mbar_wait(accum, 0, err, 27);
+      fence_after();
+      float v[LMAX + 1][16];
+      __syncwarp();
+#pragma unroll
+      for (int L = 0; L <= LMAX; ++L)
+        tmem_ld16_async(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(L * SBN + c), v[L]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int L = 0; L <= LMAX; ++L) tmem_loaded(v[L]);
+      // every level sum is an integer below 2^25 in magnitude (at most 1024 terms of at most 2^14.3).  One column at
+      // a time: the conversions (a quarter of the arithmetic rate) and the stores of its neighbours overlap.
+      const bool any = ok && nkb > 0;
+      auto combined = [&](int j) {
+        long long acc = 0;
+#pragma unroll
+        for (int L = 0; L <= LMAX; ++L) acc = mad_wide(__float2int_rn(v[L][j]), 1 << (BETA * (LMAX - L)), acc);
+        return any ? acc : 0ll;
+      };
+      if (partial != nullptr) {
+        long long* P = partial + (size_t)blockIdx.z * (size_t)M * N;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int n = n0 + c + j;
+          const long long acc = combined(j);
+          if (row < M && n < N) P[row + (size_t)n * M] = acc;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int n = n0 + c + j, en = __shfl_sync(0xffffffffu, ecol, j);
+          const long long acc = combined(j);
+          if (row < M && n < N) C[row + (size_t)n * ldc] = i64_ldexp(acc, erow + en - SL_SHIFT);
         }
       }
     }
@@ -578,17 +741,19 @@ __global__ void __launch_bounds__(SCS_T) k_finish_scalecols_slice(int64_t m, int
 
 static_assert(slice::S == kSliceDigits, "digit count");
 
-// Digit stack of X (K x M, column-major FP64) into caller buffers (M * S * roundup(K, 64) bf16, M ints)
-int sliced_prepare_into(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, int64_t ldx, __nv_bfloat16* stack,
-                        int* expo, SlicedOperand* out) {
+// Digit stack of X (K x M, column-major FP64) into caller buffers (sliced_digits<TD>(M, roundup(K, 64)), M ints): BF16 for
+// the right operand of a product, packed bytes for the left one
+template <class TD>
+int sliced_prepare_into(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, int64_t ldx, TD* stack, int* expo,
+                        SlicedDigits<TD>* out) {
   out->K = K;
   out->Kp = (K + 63) / 64 * 64;
   out->M = M;
   out->stack = stack;
   out->expo = expo;
   if (out->Kp <= 128) {  // short columns (back-transform coefficients): 64 threads per column
-    slice::k_slice_cols<2, 64><<<(unsigned)std::min<int64_t>(M, 65535), 64, 0, ctx->stream>>>(K, out->Kp, M, X, ldx,
-                                                                                            stack, expo);
+    slice::k_slice_cols<TD, 2, 64><<<(unsigned)std::min<int64_t>(M, 65535), 64, 0, ctx->stream>>>(K, out->Kp, M, X,
+                                                                                                ldx, stack, expo);
     OFRR_LAUNCHED(ctx, "k_slice_cols");
     return OFRR_SUCCESS;
   }
@@ -596,13 +761,13 @@ int sliced_prepare_into(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, in
     const unsigned grid = (unsigned)std::min<int64_t>(M, 65535);
     const int64_t u = (out->Kp + slice::SC_T - 1) / slice::SC_T;
     if (u <= 2)
-      slice::k_slice_cols<2><<<grid, slice::SC_T, 0, ctx->stream>>>(K, out->Kp, M, X, ldx, stack, expo);
+      slice::k_slice_cols<TD, 2><<<grid, slice::SC_T, 0, ctx->stream>>>(K, out->Kp, M, X, ldx, stack, expo);
     else if (u <= 4)
-      slice::k_slice_cols<4><<<grid, slice::SC_T, 0, ctx->stream>>>(K, out->Kp, M, X, ldx, stack, expo);
+      slice::k_slice_cols<TD, 4><<<grid, slice::SC_T, 0, ctx->stream>>>(K, out->Kp, M, X, ldx, stack, expo);
     else if (u <= 8)
-      slice::k_slice_cols<8><<<grid, slice::SC_T, 0, ctx->stream>>>(K, out->Kp, M, X, ldx, stack, expo);
+      slice::k_slice_cols<TD, 8><<<grid, slice::SC_T, 0, ctx->stream>>>(K, out->Kp, M, X, ldx, stack, expo);
     else
-      slice::k_slice_cols<16><<<grid, slice::SC_T, 0, ctx->stream>>>(K, out->Kp, M, X, ldx, stack, expo);
+      slice::k_slice_cols<TD, 16><<<grid, slice::SC_T, 0, ctx->stream>>>(K, out->Kp, M, X, ldx, stack, expo);
     OFRR_LAUNCHED(ctx, "k_slice_cols");
     return OFRR_SUCCESS;
   }
@@ -621,17 +786,19 @@ int sliced_prepare_into(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, in
 }
 
 // Build the digit stack of X (K x M, column-major FP64) in the workspace.
-int sliced_prepare(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, int64_t ldx, SlicedOperand* out) {
+template <class TD>
+int sliced_prepare(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, int64_t ldx, SlicedDigits<TD>* out) {
   int st = OFRR_SUCCESS;
   const int64_t Kp = (K + 63) / 64 * 64;
-  __nv_bfloat16* stack = ws_get<__nv_bfloat16>(ctx, (size_t)M * slice::S * Kp, &st);
+  TD* stack = ws_get<TD>(ctx, sliced_digits<TD>(M, Kp), &st);
   if (!stack) return st;
   int* expo = ws_get<int>(ctx, (size_t)M, &st);
   if (!expo) return st;
   return sliced_prepare_into(ctx, K, M, X, ldx, stack, expo, out);
 }
+template int sliced_prepare(ofrr_ctx*, int64_t, int64_t, const double*, int64_t, SlicedLeft*);
+template int sliced_prepare_into(ofrr_ctx*, int64_t, int64_t, const double*, int64_t, uint8_t*, int*, SlicedLeft*);
 
-// C (M x N, FP64) = A_op' B with A_op the prepared stack (K x M) and B (K x N, FP64, column-major)
 // C (M x N, FP64) = A_op' B with A_op the prepared stack (K x M) and B (K x N, FP64, column-major).
 // reps > 1 (profiling) repeats the product kernel and reports its mean time per launch in *us.
 // fs != nullptr (with several K ranges): the partial sums go straight to k_finish_scalecols_slice.
@@ -641,7 +808,7 @@ struct FusedScale {
   int* expo;
   bool done = false;
 };
-static int sliced_gemm_run(ofrr_ctx* ctx, const SlicedOperand& A, int64_t N, const double* B, int64_t ldb, double* C,
+static int sliced_gemm_run(ofrr_ctx* ctx, const SlicedLeft& A, int64_t N, const double* B, int64_t ldb, double* C,
                            int64_t ldc, int reps, double* us, double* bytes, const SlicedOperand* Bpre = nullptr,
                            FusedScale* fs = nullptr) {
   using namespace slice;
@@ -657,10 +824,8 @@ static int sliced_gemm_run(ofrr_ctx* ctx, const SlicedOperand& A, int64_t N, con
   } else {
     OFRR_TRY(sliced_prepare(ctx, K, N, B, ldb, &Bs));
   }
-  CUtensorMap ma, mb;
-  if (!tc::make_map(&ma, OFRR_BF16, A.stack, S * Kp, M, S * Kp, tc::BM) ||
-      !tc::make_map(&mb, OFRR_BF16, Bs.stack, S * Kp, N, S * Kp, SBN))
-    return OFRR_ERR_INTERNAL;
+  CUtensorMap mb;
+  if (!tc::make_map(&mb, OFRR_BF16, Bs.stack, S * Kp, N, S * Kp, SBN)) return OFRR_ERR_INTERNAL;
   const int kbt = (int)(Kp / tc::BK);
   const int tiles = (int)(((M + tc::BM - 1) / tc::BM) * ((N + SBN - 1) / SBN));
   // K ranges of at most 16 k-blocks (exactness), and about one wave of CTAs
@@ -687,7 +852,7 @@ static int sliced_gemm_run(ofrr_ctx* ctx, const SlicedOperand& A, int64_t N, con
     OFRR_CUDA(cudaEventRecord(e0, ctx->stream));
   }
   for (int r = 0; r < (reps > 1 ? reps : 1); ++r) {
-    k_sliced_tn<<<grid, SL_THREADS, SL_SMEM, ctx->stream>>>(ma, mb, (int)M, (int)N, Kp, kbt, kbps,
+    k_sliced_tn<<<grid, SL_THREADS, SL_SMEM, ctx->stream>>>(A.stack, mb, (int)M, (int)N, Kp, kbt, kbps,
                                                           tc::make_idesc(OFRR_BF16, SBN), P, C, ldc, A.expo, Bs.expo,
                                                           ctx->dev_flags + kFlagTcWait);
     OFRR_LAUNCHED(ctx, "k_sliced_tn");
@@ -701,7 +866,7 @@ static int sliced_gemm_run(ofrr_ctx* ctx, const SlicedOperand& A, int64_t N, con
     cudaEventDestroy(e1);
     if (us) *us = 1e3 * (double)ms / reps;
     if (bytes)  // digit stacks read once, int64 partials (or FP64 C) written once
-      *bytes = (double)S * Kp * 2 * (double)(M + N) + (double)M * N * 8 * (splits > 1 ? splits : 1);
+      *bytes = (double)S * Kp * (M + 2.0 * N) + (double)M * N * 8 * (splits > 1 ? splits : 1);
   }
   if (splits > 1 && fs) {
     const int64_t Kpc = (M + 63) / 64 * 64;
@@ -725,12 +890,12 @@ static int sliced_gemm_run(ofrr_ctx* ctx, const SlicedOperand& A, int64_t N, con
   return OFRR_SUCCESS;
 }
 
-int sliced_gemm_tn(ofrr_ctx* ctx, const SlicedOperand& A, int64_t N, const double* B, int64_t ldb, double* C,
+int sliced_gemm_tn(ofrr_ctx* ctx, const SlicedLeft& A, int64_t N, const double* B, int64_t ldb, double* C,
                    int64_t ldc) {
   return sliced_gemm_run(ctx, A, N, B, ldb, C, ldc, 1, nullptr, nullptr);
 }
 
-int sliced_gemm_tn_pre(ofrr_ctx* ctx, const SlicedOperand& A, const SlicedOperand& B, double* C, int64_t ldc) {
+int sliced_gemm_tn_pre(ofrr_ctx* ctx, const SlicedLeft& A, const SlicedOperand& B, double* C, int64_t ldc) {
   return sliced_gemm_run(ctx, A, B.M, nullptr, 0, C, ldc, 1, nullptr, nullptr, &B);
 }
 
@@ -738,7 +903,7 @@ int sliced_gemm_tn_pre(ofrr_ctx* ctx, const SlicedOperand& A, const SlicedOperan
 // describes them), as sliced_gemm_tn_pre followed by scalecols_sliced and with the same results.  With
 // several K ranges the partial sums are combined inside the scaling kernel, and write_u = false
 // leaves U unwritten (a block that only feeds the next product through its digits).
-int sliced_gemm_scalecols_pre(ofrr_ctx* ctx, const SlicedOperand& A, const SlicedOperand& B, double* U, int64_t ldu,
+int sliced_gemm_scalecols_pre(ofrr_ctx* ctx, const SlicedLeft& A, const SlicedOperand& B, double* U, int64_t ldu,
                               bool write_u, __nv_bfloat16* stack, int* expo, SlicedOperand* out) {
   const int64_t m = A.M, n = B.M;
   if (m < 1 || m > 8192 || n < 1 || n > 65535) return OFRR_ERR_BLAS_INVALID_SIZE;
@@ -780,7 +945,7 @@ extern "C" int ofrr_gemm_f64_emulated(ofrr_ctx* ctx, int64_t M, int64_t N, int64
   if (M == 0 || N == 0) return OFRR_SUCCESS;
   if (!A || !B || !C || lda < K || ldb < K || ldc < M || K < 1) return OFRR_ERR_INVALID_ARGUMENT;
   WsScope scope(ctx);
-  SlicedOperand As;
+  SlicedLeft As;
   OFRR_TRY(sliced_prepare(ctx, K, M, A, lda, &As));
   return sliced_gemm_tn(ctx, As, N, B, ldb, C, ldc);
 }
@@ -794,7 +959,7 @@ extern "C" int ofrr_profile_gemm_f64_emulated(ofrr_ctx* ctx, int64_t M, int64_t 
     return OFRR_ERR_INVALID_ARGUMENT;
   if (!A || !B || !C || lda < K || ldb < K || ldc < M) return OFRR_ERR_INVALID_ARGUMENT;
   WsScope scope(ctx);
-  SlicedOperand As;
+  SlicedLeft As;
   OFRR_TRY(sliced_prepare(ctx, K, M, A, lda, &As));
   return sliced_gemm_run(ctx, As, N, B, ldb, C, ldc, reps, us_per_launch, bytes_per_launch);
 }
@@ -815,7 +980,8 @@ extern "C" int ofrr_debug_scale_slice(ofrr_ctx* ctx, int mode, int64_t M, int64_
   if (mode == 2) return sliced_prepare_into(ctx, M, N, X, ldx, stack, expo, &out);
   if (K < 1 || !A || !B || lda < K || ldb < K) return OFRR_ERR_INVALID_ARGUMENT;
   WsScope scope(ctx);
-  SlicedOperand As, Bs;
+  SlicedLeft As;
+  SlicedOperand Bs;
   OFRR_TRY(sliced_prepare(ctx, K, M, A, lda, &As));
   OFRR_TRY(sliced_prepare(ctx, K, N, B, ldb, &Bs));
   return sliced_gemm_scalecols_pre(ctx, As, Bs, X, ldx, true, stack, expo, &out);

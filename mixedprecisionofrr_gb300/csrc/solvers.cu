@@ -156,7 +156,7 @@ struct Op {
 
   // digit stacks of A for the FP64 emulation: sAt for A V (operand A', K = n), sA for A' U (K = m).
   // Must be called in the solve's outermost workspace scope (the stacks live as long as the solve).
-  SlicedOperand sA, sAt;
+  SlicedLeft sA, sAt;
   bool have_sA = false, have_sAt = false;
   // |A| in a 16-bit type in both K-contiguous orientations (absA[0] = |A'| for A X, absA[1] = |A| for
   // A' X), for the bounds on the emulation error; made once per solve by prepare_abs
@@ -179,7 +179,7 @@ struct Op {
     sAt.Kp = (n() + 63) / 64 * 64;
     sAt.M = m();
     int st = OFRR_SUCCESS;
-    sAt.stack = ws_get<__nv_bfloat16>(ctx, (size_t)m() * kSliceDigits * sAt.Kp, &st);
+    sAt.stack = ws_get<uint8_t>(ctx, sliced_digits<uint8_t>(m(), sAt.Kp), &st);
     if (!sAt.stack) return st;
     sAt.expo = ws_get<int>(ctx, (size_t)m(), &st);
     if (!sAt.expo) return st;
@@ -187,7 +187,7 @@ struct Op {
     double* At = ws_get<double>(ctx, (size_t)m() * n(), &st);
     if (!At) return st;
     OFRR_TRY(cast_transpose_impl(ctx, A->dtype, OFRR_F64, m(), n(), A->data, A->ld, At, n()));
-    SlicedOperand t;
+    SlicedLeft t;
     OFRR_TRY(sliced_prepare_into(ctx, n(), m(), At, n(), sAt.stack, sAt.expo, &t));
     have_sAt = true;
     return OFRR_SUCCESS;
