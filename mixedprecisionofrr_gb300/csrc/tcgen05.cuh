@@ -57,34 +57,38 @@ __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* ba
       : "memory");
 }
 
-// UMMA shared-memory descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address (16-byte units)
-  d |= (uint64_t)1 << 16;                    // leading byte offset (ignored for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset between 8-row groups
-  d |= (uint64_t)1 << 46;                    // descriptor version
-  d |= (uint64_t)2 << 61;                    // 128-byte swizzle
-  return d;
-}
+// UMMA shared-memory descriptor of a K-major operand with 128-byte swizzle: bits 0-13 the start address in 16-byte
+// units, 16-29 the leading byte offset (ignored here, 1), 32-45 the stride between 8-row groups (1024 B in 16-byte
+// units), bit 46 the version, 61-63 the swizzle (2 = 128 bytes).  Only the low word varies, by the address.
+constexpr uint32_t kDescLo = 1u << 16;
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
 
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// D (TMEM) += A B, both operands by their descriptors' low words (shared address >> 4).
+// F8: E4M3 x E4M3 -> FP32 (kind::f8f6f4), K = 32 bytes per instruction like the 16-bit form
+template <bool F8>
+__device__ __forceinline__ void umma_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                        uint32_t accumulate) {
+  if (F8)
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, p;\n}\n" ::"r"(tmem_d),
+        "r"(a_lo | kDescLo), "r"(b_lo | kDescLo), "r"(idesc), "r"(accumulate), "r"(kDescHi)
+        : "memory");
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n" ::"r"(tmem_d),
+        "r"(a_lo | kDescLo), "r"(b_lo | kDescLo), "r"(idesc), "r"(accumulate), "r"(kDescHi)
+        : "memory");
 }
 // A from TMEM (128 lanes x 8 columns of two 16-bit values per K = 16), B by its descriptor's low word (shared address
-// >> 4, as desc_sw128 sets it)
+// >> 4)
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc,
                                             uint32_t accumulate) {
-  constexpr uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
   asm volatile(
       "{\n .reg .pred p;\n .reg .b64 b;\n mov.b64 b, {%2, %5};\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}\n" ::"r"(tmem_d),
-      "r"(tmem_a), "r"(b_lo | (1u << 16)), "r"(idesc), "r"(accumulate), "r"(hi)
+      "r"(tmem_a), "r"(b_lo | kDescLo), "r"(idesc), "r"(accumulate), "r"(kDescHi)
       : "memory");
 }
 // one lane of the (converged) warp, the same one on every call
@@ -92,15 +96,6 @@ __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.b32 %0, 1, 0, q;\n}\n" : "=r"(p));
   return p != 0;
-}
-// E4M3 x E4M3 -> FP32 (kind::f8f6f4): K = 32 bytes per instruction, the same descriptors as the 16-bit form
-__device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
