@@ -550,6 +550,10 @@ int residual_columns2(ofrr_ctx* ctx, int64_t m, int64_t n, const double* AV, con
                       double* out);
 int column_norms(ofrr_ctx* ctx, ofrr_dtype t, int64_t m, int64_t n, const void* X, int64_t ldx,
                  double* out_dev);
+// matrix sign function X <- sign(X) (n <= 96; *flag = 1 on a singular step) and an orthonormal basis Q (n x p) of
+// range((I + S) / 2) (sign_function.cu)
+int sign_newton(ofrr_ctx* ctx, int n, double* X, int maxit, double tol, int* flag);
+int sign_basis(ofrr_ctx* ctx, int n, int p, const double* S, double* Q);
 // exact-slice FP64 emulation (sliced.cu): digit stacks of a fixed K x M FP64 operand and the
 // product C (M x N) = X' B with X the prepared left operand and B (K x N) FP64.  The left operand (the large one) keeps
 // its digits in one byte each, the right one in BF16.

@@ -743,179 +743,12 @@ __global__ void k_unit_cols(int n, double* __restrict__ U) {
 // separated from the others, and the matrix sign function gives it without eigenvectors:
 // S = sign(C - sigma I) (Newton, X <- (mu X + (mu X)^-1) / 2 with determinant scaling mu), P = (I + S) / 2
 // projects onto the eigenvalues with real part above sigma [N. J. Higham, Functions of Matrices,
-// SIAM 2008, ch. 5].  One CTA, FP64; Gauss-Jordan inversion with partial pivoting in shared memory.
+// SIAM 2008, ch. 5] (sign_function.cu).
 constexpr int kSignMaxN = 96;
-
-template <class T>
-__global__ void __launch_bounds__(256) k_sign_newton(int n, double* __restrict__ Xg, int maxit, double tol,
-                                                     int* __restrict__ flag) {
-  extern __shared__ __align__(16) unsigned char sgn_raw[];
-  T* X = reinterpret_cast<T*>(sgn_raw);  // n x n, column-major
-  T* Y = X + (size_t)n * n;              // its inverse (Gauss-Jordan in place)
-  __shared__ int piv[kSignMaxN];
-  __shared__ T s_col[kSignMaxN];
-  __shared__ int s_p;
-  __shared__ double s_logdet, s_num, s_den;
-  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
-  const int nn = n * n;
-  if (*flag) return;  // an earlier stage met a singular matrix
-  for (int e = tid; e < nn; e += nthr) X[e] = (T)Xg[e];
-  __syncthreads();
-  for (int it = 0; it < maxit; ++it) {
-    for (int e = tid; e < nn; e += nthr) Y[e] = X[e];
-    if (tid == 0) s_logdet = 0.0;
-    __syncthreads();
-    bool singular = false;
-    for (int k = 0; k < n; ++k) {
-      if (tid < 32) {  // pivot: first largest |Y(i, k)|, i >= k
-        T best = T(-1);
-        int bi = k;
-        for (int i = k + lane; i < n; i += 32) {
-          const T a = fabs(Y[i + (size_t)k * n]);
-          if (a > best) {
-            best = a;
-            bi = i;
-          }
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          const T ob = __shfl_down_sync(0xffffffffu, best, off);
-          const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-          if (ob > best || (ob == best && oi < bi)) {
-            best = ob;
-            bi = oi;
-          }
-        }
-        if (lane == 0) s_p = bi;
-      }
-      __syncthreads();
-      const int p = s_p;
-      if (p != k)
-        for (int j = tid; j < n; j += nthr) {
-          const T t = Y[k + (size_t)j * n];
-          Y[k + (size_t)j * n] = Y[p + (size_t)j * n];
-          Y[p + (size_t)j * n] = t;
-        }
-      if (tid == 0) piv[k] = p;
-      __syncthreads();
-      const T d = Y[k + (size_t)k * n];
-      if (!(fabs(d) > T(0))) {  // zero or NaN pivot: every thread sees the same value
-        singular = true;
-        break;
-      }
-      const T dinv = T(1) / d;
-      if (tid == 0) s_logdet += log(fabs((double)d));
-      for (int i = tid; i < n; i += nthr) s_col[i] = (i == k) ? T(0) : Y[i + (size_t)k * n];
-      __syncthreads();
-      for (int j = tid; j < n; j += nthr) Y[k + (size_t)j * n] = (j == k) ? dinv : Y[k + (size_t)j * n] * dinv;
-      for (int i = tid; i < n; i += nthr)
-        if (i != k) Y[i + (size_t)k * n] = T(0);
-      __syncthreads();
-      for (int e = tid; e < nn; e += nthr) {
-        const int i = e % n, j = e / n;
-        if (i != k) Y[e] -= s_col[i] * Y[k + (size_t)j * n];
-      }
-      __syncthreads();
-    }
-    if (singular) {
-      if (tid == 0) *flag = 1;
-      return;
-    }
-    for (int k = n - 1; k >= 0; --k) {  // undo the row interchanges as column interchanges of the inverse
-      const int p = piv[k];
-      if (p != k)
-        for (int i = tid; i < n; i += nthr) {
-          const T t = Y[i + (size_t)k * n];
-          Y[i + (size_t)k * n] = Y[i + (size_t)p * n];
-          Y[i + (size_t)p * n] = t;
-        }
-      __syncthreads();
-    }
-    const double mu = (it < 4) ? exp(-s_logdet / n) : 1.0;  // determinant scaling in the first steps
-    if (tid == 0) {
-      s_num = 0.0;
-      s_den = 0.0;
-    }
-    __syncthreads();
-    double num = 0.0, den = 0.0;
-    for (int e = tid; e < nn; e += nthr) {
-      const T xn = (T)(0.5 * (mu * (double)X[e] + (double)Y[e] / mu));
-      num += ((double)xn - (double)X[e]) * ((double)xn - (double)X[e]);
-      den += (double)xn * (double)xn;
-      X[e] = xn;
-    }
-    atomicAdd(&s_num, num);
-    atomicAdd(&s_den, den);
-    __syncthreads();
-    const bool done = s_num <= tol * tol * s_den;
-    __syncthreads();
-    if (done && it >= 1) break;
-  }
-  for (int e = tid; e < nn; e += nthr) Xg[e] = (double)X[e];
-}
 
 __global__ void k_shift_copy(int n, const double* __restrict__ C, double sigma, double* __restrict__ X) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x)
     X[e] = C[e] - ((e % n == e / n) ? sigma : 0.0);
-}
-
-// Q (n x p) = orthonormal basis of range((I + S) / 2): the projector applied to a fixed pseudo-random
-// block (splitmix64 hashes), then modified Gram-Schmidt twice (FP64, one CTA)
-__global__ void __launch_bounds__(256) k_proj_basis(int n, int p, const double* __restrict__ S, double* __restrict__ Q) {
-  extern __shared__ double pb[];  // n x p
-  __shared__ double s_red[8];
-  __shared__ double s_dot;
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  for (int e = tid; e < n * p; e += nthr) {
-    const int i = e % n, c = e / n;
-    double acc = 0.0;
-    for (int k = 0; k < n; ++k) {
-      unsigned long long h = 0x9e3779b97f4a7c15ULL * (unsigned long long)(k + 1) + 0xbf58476d1ce4e5b9ULL * (c + 1);
-      h ^= h >> 31;
-      h *= 0x94d049bb133111ebULL;
-      h ^= h >> 29;
-      const double om = (double)(h >> 11) * (1.0 / 9007199254740992.0) - 0.5;
-      const double pik = 0.5 * (S[i + (size_t)k * n] + ((i == k) ? 1.0 : 0.0));
-      acc += pik * om;
-    }
-    pb[e] = acc;
-  }
-  __syncthreads();
-  auto block_sum = [&](double v) -> double {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if ((tid & 31) == 0) s_red[tid >> 5] = v;
-    __syncthreads();
-    if (tid == 0) {
-      double t = 0.0;
-      for (int w = 0; w < (nthr + 31) / 32; ++w) t += s_red[w];
-      s_dot = t;
-    }
-    __syncthreads();
-    const double r = s_dot;
-    __syncthreads();
-    return r;
-  };
-  for (int c = 0; c < p; ++c) {
-    double* qc = pb + (size_t)c * n;
-    for (int pass = 0; pass < 2; ++pass) {
-      for (int c2 = 0; c2 < c; ++c2) {
-        const double* q2 = pb + (size_t)c2 * n;
-        double v = 0.0;
-        for (int i = tid; i < n; i += nthr) v += q2[i] * qc[i];
-        const double dt = block_sum(v);
-        for (int i = tid; i < n; i += nthr) qc[i] -= dt * q2[i];
-        __syncthreads();
-      }
-    }
-    double v = 0.0;
-    for (int i = tid; i < n; i += nthr) v += qc[i] * qc[i];
-    const double t = block_sum(v);
-    const double sc = (t > 0.0) ? 1.0 / sqrt(t) : 0.0;
-    for (int i = tid; i < n; i += nthr) qc[i] *= sc;
-    __syncthreads();
-  }
-  for (int e = tid; e < n * p; e += nthr) Q[e] = pb[e];
 }
 
 // Y (n x p, ld n) spanning the invariant subspace of the pencil (G, M) for its p eigenvalues with real
@@ -942,13 +775,8 @@ int invariant_subspace_nonsym(ofrr_ctx* ctx, int n, const double* G, const doubl
   OFRR_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), ctx->stream));
   // FP64 throughout: the iteration converges to the sign of the matrix it is given, so rounding errors of
   // a lower-precision start are not corrected by later FP64 steps (they change the matrix, not the path)
-  const size_t sm64 = 2 * (size_t)n * n * sizeof(double);
-  OFRR_TRY(allow_smem(k_sign_newton<double>));
-  k_sign_newton<double><<<1, 256, sm64, ctx->stream>>>(n, X, 80, 1e-14, flag);
-  OFRR_LAUNCHED(ctx, "k_sign_newton");
-  OFRR_TRY(allow_smem(k_proj_basis));
-  k_proj_basis<<<1, 256, (size_t)n * p * sizeof(double), ctx->stream>>>(n, p, X, Q);
-  OFRR_LAUNCHED(ctx, "k_proj_basis");
+  OFRR_TRY(sign_newton(ctx, n, X, 80, 1e-14, flag));
+  OFRR_TRY(sign_basis(ctx, n, p, X, Q));
   OFRR_TRY(trsm(ctx, n, p, L, Q, n, 0, Y, 1));  // Y = L^-T Q
   int hf = 0;
   OFRR_TRY(fetch(ctx, &hf, flag, sizeof(int)));
