@@ -38,12 +38,28 @@ __device__ __forceinline__ void cdivf(T xr, T xi, T yr, T yi, T& cr, T& ci) {
   }
 }
 
-// One warp.  C: n x n (FP64, ld ldc).  Outputs: wr, wi (n), X (n x n, FP64, ld n): eigenvectors of C
+// The chain of a QR sweep is bound by latency: in FP64 every warp instruction takes 64 cycles of the sub-partition's
+// pipe, a division ~560 and a comparison ~105.  So independent quotients of a step are formed in different lanes of one
+// division, the searches for small subdiagonal entries look at 32 candidates at a time, tests against zero are made on
+// the bit patterns, and the Schur vectors are updated by a second warp on its own sub-partition, which follows the
+// reflectors through a two-slot queue.  Values and order of operations are those of the plain loops.
+// Random matrices: FP64 with vectors, n = 25, 4.74 -> 2.12 ms; FP32 values only, n = 65, 3.22 -> 2.43 ms.
+__device__ __forceinline__ bool ns_zero(double x) {
+  return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
+}
+__device__ __forceinline__ bool ns_neg(double x) {  // x < 0 (false for -0 and NaN)
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
+}
+__device__ __forceinline__ void ns_bar_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void ns_bar_arrive(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+
+// One warp, and with VEC a second one for the Schur vectors.  C: n x n (FP64, ld ldc).  Outputs: wr, wi (n), X (n x n, FP64, ld n): eigenvectors of C
 // (real parts, unit norm), unsorted; *flag = 1 when the QR iteration did not converge.
 // VEC = false: eigenvalues only (EISPACK hqr instead of hqr2): no transformations accumulated, the QR
 // sweeps restricted to the active block, no eigenvectors (X is not written)
 template <class T, bool VEC = true>
-__global__ void __launch_bounds__(32) k_nonsym_eig(int nn, const double* __restrict__ C, int ldc,
+__global__ void __launch_bounds__(VEC ? 64 : 32) k_nonsym_eig(int nn, const double* __restrict__ C, int ldc,
                                                        double* __restrict__ wr, double* __restrict__ wi,
                                                        double* __restrict__ X, int* __restrict__ flag,
                                                        int pair_imag) {
@@ -56,10 +72,57 @@ __global__ void __launch_bounds__(32) k_nonsym_eig(int nn, const double* __restr
   T* ort = Y + nn * ld;  // n
   T* d = ort + nn;       // n
   T* e = d + nn;         // n
-  const int lane = threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  // queue to the second warp: named barriers 1, 2 (slot full) and 3, 4 (slot empty)
+  struct Op {
+    int kind, k;  // 0: reflector of columns k, k + 1; 1: and k + 2; 2: rotation of columns k, k + 1; 3: end
+    T x, y, z, q, r;
+  };
+  __shared__ Op s_op[2];
 #define HH(i, j) H[(i) + (j) * ld]
 #define VV(i, j) V[(i) + (j) * ld]
 #define YY(i, j) Y[(i) + (j) * ld]
+  if (VEC && threadIdx.x >= 32) {
+    ns_bar_arrive(3);
+    ns_bar_arrive(4);
+    for (int cnt = 0;; ++cnt) {
+      ns_bar_sync(1 + (cnt & 1));
+      const Op o = s_op[cnt & 1];
+      if (o.kind == 3) break;
+      ns_bar_arrive(3 + (cnt & 1));
+      const T x = o.x, y = o.y, z = o.z, q = o.q, r = o.r;
+      const int k = o.k;
+      const bool notlast = o.kind == 1;
+      if (o.kind == 2) {
+        for (int i = lane; i < nn; i += 32) {
+          const T zz = VV(i, k);
+          VV(i, k) = q * zz + x * VV(i, k + 1);
+          VV(i, k + 1) = q * VV(i, k + 1) - x * zz;
+        }
+      } else {
+        for (int i = lane; i < nn; i += 32) {
+          T pp = x * VV(i, k) + y * VV(i, k + 1);
+          if (notlast) {
+            pp += z * VV(i, k + 2);
+            VV(i, k + 2) -= pp * r;
+          }
+          VV(i, k) -= pp;
+          VV(i, k + 1) -= pp * q;
+        }
+      }
+      __syncwarp();
+    }
+    __syncthreads();  // V is complete
+    return;
+  }
+  int sent = 0;
+  auto send = [&](int kind, int k, T x, T y, T z, T q, T r) {
+    ns_bar_sync(3 + (sent & 1));
+    if (lane == 0) s_op[sent & 1] = Op{kind, k, x, y, z, q, r};
+    __syncwarp();
+    ns_bar_arrive(1 + (sent & 1));
+    ++sent;
+  };
   for (int idx = lane; idx < nn * nn; idx += 32) {
     const int i = idx % nn, j = idx / nn;
     HH(i, j) = (T)C[i + (size_t)j * ldc];
@@ -139,12 +202,17 @@ __global__ void __launch_bounds__(32) k_nonsym_eig(int nn, const double* __restr
   bool failed = false;
   while (n >= low) {
     int l = n;
-    while (l > low) {
-      s = fabs(HH(l - 1, l - 1)) + fabs(HH(l, l));
+    for (; l > low; l -= 32) {  // the lowest l with a negligible subdiagonal entry, 32 candidates at a time
+      const int lc = max(l - lane, low + 1);
+      s = fabs(HH(lc - 1, lc - 1)) + fabs(HH(lc, lc));
       if (s == T(0.)) s = norm;
-      if (fabs(HH(l, l - 1)) < eps * s) break;
-      --l;
+      const unsigned hit = __ballot_sync(0xffffffffu, l - lane > low && fabs(HH(lc, lc - 1)) < eps * s);
+      if (hit) {
+        l -= __ffs(hit) - 1;
+        break;
+      }
     }
+    l = max(l, low);
     if (l == n) {  // one root
       const T hn = HH(n, n) + exshift;
       __syncwarp();
@@ -198,12 +266,8 @@ __global__ void __launch_bounds__(32) k_nonsym_eig(int nn, const double* __restr
           HH(i, n - 1) = q * zz + p * HH(i, n);
           HH(i, n) = q * HH(i, n) - p * zz;
         }
-        for (int i = low + lane; VEC && i <= high; i += 32) {  // accumulate
-          const T zz = VV(i, n - 1);
-          VV(i, n - 1) = q * zz + p * VV(i, n);
-          VV(i, n) = q * VV(i, n) - p * zz;
-        }
         __syncwarp();
+        if (VEC) send(2, n - 1, p, T(0.), T(0.), q, T(0.));  // accumulate
       } else {  // complex pair
         __syncwarp();
         if (lane == 0) {
@@ -254,22 +318,31 @@ __global__ void __launch_bounds__(32) k_nonsym_eig(int nn, const double* __restr
       ++iter;
       // two consecutive small subdiagonal elements
       int m = n - 2;
-      while (m >= l) {
-        z = HH(m, m);
+      for (;; m -= 32) {  // 32 candidates at a time; m = l ends the search
+        const int mc = max(m - lane, l);
+        z = HH(mc, mc);
         r = x - z;
         s = y - z;
-        p = (r * s - w) / HH(m + 1, m) + HH(m, m + 1);
-        q = HH(m + 1, m + 1) - z - r - s;
-        r = HH(m + 2, m + 1);
+        p = (r * s - w) / HH(mc + 1, mc) + HH(mc, mc + 1);
+        q = HH(mc + 1, mc + 1) - z - r - s;
+        r = HH(mc + 2, mc + 1);
         s = fabs(p) + fabs(q) + fabs(r);
         p /= s;
         q /= s;
         r /= s;
-        if (m == l) break;
-        if (fabs(HH(m, m - 1)) * (fabs(q) + fabs(r)) <
-            eps * (fabs(p) * (fabs(HH(m - 1, m - 1)) + fabs(z) + fabs(HH(m + 1, m + 1)))))
+        bool stop = mc == l;
+        if (!stop)
+          stop = fabs(HH(mc, mc - 1)) * (fabs(q) + fabs(r)) <
+                 eps * (fabs(p) * (fabs(HH(mc - 1, mc - 1)) + fabs(z) + fabs(HH(mc + 1, mc + 1))));
+        const unsigned hit = __ballot_sync(0xffffffffu, stop);
+        if (hit) {
+          const int src = __ffs(hit) - 1;
+          m = max(m - src, l);
+          p = __shfl_sync(0xffffffffu, p, src);
+          q = __shfl_sync(0xffffffffu, q, src);
+          r = __shfl_sync(0xffffffffu, r, src);
           break;
-        --m;
+        }
       }
       __syncwarp();
       for (int i = m + 2 + lane; i <= n; i += 32) {
@@ -285,22 +358,44 @@ __global__ void __launch_bounds__(32) k_nonsym_eig(int nn, const double* __restr
           q = HH(k + 1, k - 1);
           r = notlast ? HH(k + 2, k - 1) : T(0.);
           x = fabs(p) + fabs(q) + fabs(r);
-          if (x == T(0.)) continue;
-          p /= x;
-          q /= x;
-          r /= x;
+          if constexpr (sizeof(T) == 8) {  // three quotients in three lanes
+            if (ns_zero(x)) continue;
+            const T quo = ((lane == 0) ? p : (lane == 1) ? q : r) / x;
+            p = __shfl_sync(0xffffffffu, quo, 0);
+            q = __shfl_sync(0xffffffffu, quo, 1);
+            r = __shfl_sync(0xffffffffu, quo, 2);
+          } else {
+            if (x == T(0.)) continue;
+            p /= x;
+            q /= x;
+            r /= x;
+          }
         }
         s = sqrt(p * p + q * q + r * r);
-        if (p < T(0.)) s = -s;
-        if (s == T(0.)) continue;
+        if constexpr (sizeof(T) == 8) {
+          if (ns_neg(p)) s = -s;
+          if (ns_zero(s)) continue;
+        } else {
+          if (p < T(0.)) s = -s;
+          if (s == T(0.)) continue;
+        }
         const T hk = (k != m) ? -s * x : ((l != m) ? -HH(k, k - 1) : T(0.));
         const bool set_hk = (k != m) || (l != m);
         p = p + s;
-        x = p / s;
-        y = q / s;
-        z = r / s;
-        q = q / p;
-        r = r / p;
+        if constexpr (sizeof(T) == 8) {  // five quotients in five lanes
+          const T quo = ((lane == 0) ? p : (lane == 1 || lane == 3) ? q : r) / (lane < 3 ? s : p);
+          x = __shfl_sync(0xffffffffu, quo, 0);
+          y = __shfl_sync(0xffffffffu, quo, 1);
+          z = __shfl_sync(0xffffffffu, quo, 2);
+          q = __shfl_sync(0xffffffffu, quo, 3);
+          r = __shfl_sync(0xffffffffu, quo, 4);
+        } else {
+          x = p / s;
+          y = q / s;
+          z = r / s;
+          q = q / p;
+          r = r / p;
+        }
         __syncwarp();
         if (lane == 0 && set_hk) HH(k, k - 1) = hk;
         const int jmax = VEC ? nn - 1 : n;  // values only: the active block's columns
@@ -324,18 +419,14 @@ __global__ void __launch_bounds__(32) k_nonsym_eig(int nn, const double* __restr
           HH(i, k) -= pp;
           HH(i, k + 1) -= pp * q;
         }
-        for (int i = low + lane; VEC && i <= high; i += 32) {  // accumulate
-          T pp = x * VV(i, k) + y * VV(i, k + 1);
-          if (notlast) {
-            pp += z * VV(i, k + 2);
-            VV(i, k + 2) -= pp * r;
-          }
-          VV(i, k) -= pp;
-          VV(i, k + 1) -= pp * q;
-        }
+        if (VEC) send(notlast ? 1 : 0, k, x, y, z, q, r);  // accumulate
         __syncwarp();
       }
     }
+  }
+  if (VEC) {
+    send(3, 0, T(0.), T(0.), T(0.), T(0.), T(0.));
+    __syncthreads();
   }
   if (failed) {
     if (lane == 0 && flag) *flag = 1;
@@ -648,13 +739,13 @@ int nonsym_eig_dev(ofrr_ctx* ctx, int n, const double* C, double* wr, double* wi
   const size_t smem64 = ((size_t)3 * n * (n + 1) + 3 * (size_t)n) * sizeof(double);
   if (refine && smem64 <= 227 * 1024) {
     OFRR_TRY(allow_smem(k_nonsym_eig<double>));
-    k_nonsym_eig<double><<<1, 32, smem64, ctx->stream>>>(n, C, n, wr, wi, X, ctx->dev_flags + 3, pair_imag ? 1 : 0);
+    k_nonsym_eig<double><<<1, 64, smem64, ctx->stream>>>(n, C, n, wr, wi, X, ctx->dev_flags + 3, pair_imag ? 1 : 0);
     OFRR_LAUNCHED(ctx, "k_nonsym_eig_f64");
     return OFRR_SUCCESS;
   }
   const size_t smem = ((size_t)3 * n * (n + 1) + 3 * (size_t)n) * sizeof(float);
   OFRR_TRY(allow_smem(k_nonsym_eig<float>));
-  k_nonsym_eig<float><<<1, 32, smem, ctx->stream>>>(n, C, n, wr, wi, X, ctx->dev_flags + 3, pair_imag ? 1 : 0);
+  k_nonsym_eig<float><<<1, 64, smem, ctx->stream>>>(n, C, n, wr, wi, X, ctx->dev_flags + 3, pair_imag ? 1 : 0);
   OFRR_LAUNCHED(ctx, "k_nonsym_eig_f32");
   if (!refine) return OFRR_SUCCESS;
   // ||C||_F on the host side of the acceptance test: one small reduction, read back
