@@ -105,11 +105,12 @@ __device__ __forceinline__ uint64_t be_mix(uint64_t x) {
 // The FP32 and 16-bit copies of every matrix are stored column-major with the leading dimension rounded up
 // to 8 elements (zero rows below n) at 16-byte aligned offsets, so kc consecutive columns are one
 // contiguous, aligned block: one cp.async.bulk per stage, completing on the stage's `full` mbarrier.
-// Every warp arrives on the stage's `empty` mbarrier once it has read the stage; thread 0 refills a stage
-// after its `empty` phase completes.  The chunk counter runs on across products, so the barrier parities
+// Every warp arrives on the stage's `empty` mbarrier once it has read the stage; the warps take turns to refill a
+// stage, one chunk after its release.  (Issuing a copy takes a thread several hundred cycles: with one thread issuing
+// them all, its warp was the slowest in every chunk and the stream's time added to the arithmetic's.)  The chunk counter runs on across products, so the barrier parities
 // follow from it.  Every wait is bounded (about 2 s); a wait that runs out records a status word and the
 // CTA leaves the kernel after the copies it issued have landed (again bounded).
-constexpr int BE_NS = 4;           // stages
+constexpr int BE_NS = 5;           // stages
 constexpr int BE_STAGE = 16384;    // bytes per stage
 
 struct BeRing {
@@ -117,6 +118,7 @@ struct BeRing {
   uint64_t* full;      // BE_NS (shared)
   uint64_t* empty;     // BE_NS (shared)
   uint32_t count;      // chunks consumed so far (uniform across the CTA)
+  unsigned* issued;    // chunks issued so far (shared; read only when a wait ran out)
   int* err;            // device status word
 };
 
@@ -147,94 +149,116 @@ __device__ __forceinline__ void be_layout(int n, int* G, int* R) {
   *R = br;
 }
 
+__device__ __forceinline__ float4 be_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 be_ld4(const __half* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
+  const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float4 be_ld4(const __nv_bfloat16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
 // W (n x b, row-major, shared) = A (n x n, column-major with leading dimension ld, global, type TA)
 // V (n x b, row-major, shared), FP32 accumulation.  Partial sums of the G groups are added in group order
-// (results do not depend on timing).  Returns false (uniformly) when a bounded wait ran out.
+// (results do not depend on timing).  A warp owns 32 R rows x 16 columns; lane (lr, lc) = (lane / 4, lane % 4) the
+// columns 4 lc .. 4 lc + 3 of the rows 32 u + 4 lr .. + 3, u < R, so per column of A it takes one 16-byte load of V and
+// R of A for 16 R multiply-adds (a row of all 16 columns per lane took four and R).  n = 1024, FP32 A on every SM:
+// 157 us a product against 245 us before both changes (FMA pipe 68 us, HBM 93 us); n = 447: 43 against 64.
+// Returns false (uniformly) when a bounded wait ran out.
 template <class TA, int R>
 __device__ bool be_matmul_r(int n, int ld, const TA* __restrict__ A, const float* V, float* W, BeRing& rg, int G) {
-  const int tid = threadIdx.x, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int Tg = ((BE_T / G) / 32) * 32;
   const int g = tid / Tg, t = tid % Tg;
   const bool active = g < G;
   const int kc = min(n, BE_STAGE / (ld * (int)sizeof(TA)));
   const int nck = (n + kc - 1) / kc;
   const uint32_t base = rg.count;
-  auto issue = [&](int c) {
-    const uint32_t gc = base + (uint32_t)c;
-    const int st = (int)(gc % BE_NS);
-    const int k0 = c * kc, cols = min(kc, n - k0);
-    const uint32_t bytes = (uint32_t)(cols * ld * (int)sizeof(TA));
-    tc::mbar_expect_tx(&rg.full[st], bytes);
-    be_bulk_g2s(rg.buf + (size_t)st * BE_STAGE, A + (int64_t)k0 * ld, bytes, &rg.full[st]);
-  };
   // refills wait for the stage's previous use to be released (that use belongs to an earlier chunk, or
   // to the previous product)
-  bool bad = false;
-  if (tid == 0) {
-    for (int c = 0; c < min(nck, BE_NS); ++c) {
-      const uint32_t gc = base + (uint32_t)c;
-      if (gc >= BE_NS && !tc::mbar_wait(&rg.empty[gc % BE_NS], ((gc / BE_NS) + 1) & 1, rg.err, 21)) {
-        bad = true;
-        break;
-      }
-      issue(c);
-    }
-  }
-  float acc[R][BE_B];
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int c = 0; c < BE_B; ++c) acc[r][c] = 0.f;
-  int c = 0;
-  for (; c < nck && !bad; ++c) {
+  auto refill = [&](int c) -> bool {
     const uint32_t gc = base + (uint32_t)c;
     const int st = (int)(gc % BE_NS);
-    if (!tc::mbar_wait(&rg.full[st], (gc / BE_NS) & 1, rg.err, 22)) {
+    if (gc >= BE_NS && !tc::mbar_wait(&rg.empty[st], ((gc / BE_NS) + 1) & 1, rg.err, 21)) return false;
+    const int k0 = c * kc, cols = min(kc, n - k0);
+    const uint32_t bytes = (uint32_t)(cols * ld * (int)sizeof(TA));
+    atomicMax(rg.issued, gc + 1);
+    tc::mbar_expect_tx(&rg.full[st], bytes);
+    be_bulk_g2s(rg.buf + (size_t)st * BE_STAGE, A + (int64_t)k0 * ld, bytes, &rg.full[st]);
+    return true;
+  };
+  bool bad = false;
+  if (tid == 0)
+    for (int c = 0; c < min(nck, BE_NS) && !bad; ++c) bad = !refill(c);
+  __syncwarp();
+  float acc[4 * R][4];
+#pragma unroll
+  for (int r = 0; r < 4 * R; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
+  const int lr = lane >> 2, lc = lane & 3;
+  const int rb = (t >> 5) * 32 * R + 4 * lr;
+  int off[R];  // rows past the leading dimension read its last rows (in bounds; their sums are not stored)
+#pragma unroll
+  for (int u = 0; u < R; ++u) off[u] = min(rb + 32 * u, ld - 4);
+  uint32_t st = base % BE_NS, ph = (base / BE_NS) & 1;
+  int k0 = 0;
+  for (int c = 0; c < nck && !bad; ++c) {
+    if (!tc::mbar_wait(&rg.full[st], ph, rg.err, 22)) {
       bad = true;
       break;
     }
-    const TA* sA = reinterpret_cast<const TA*>(rg.buf + (size_t)st * BE_STAGE);
-    const int k0 = c * kc, cols = min(kc, n - k0);
+    const int cols = min(kc, n - k0);
     if (active) {
+      const TA* pa = reinterpret_cast<const TA*>(rg.buf + (size_t)st * BE_STAGE) + g * ld;
+      const float* pv = V + (k0 + g) * BE_B;
+      int sw = (k0 + g) & 3;
+#pragma unroll 1
       for (int kk = g; kk < cols; kk += G) {
-        const float4* vk = reinterpret_cast<const float4*>(V + (k0 + kk) * BE_B);
-        const int sw = (k0 + kk) & 3;
-        float v[BE_B];
+        const float4 x = *reinterpret_cast<const float4*>(pv + ((lc ^ sw) << 2));
+        float4 a4[R];
 #pragma unroll
-        for (int q = 0; q < BE_B / 4; ++q) {
-          const float4 x = vk[q ^ sw];
-          v[4 * q] = x.x;
-          v[4 * q + 1] = x.y;
-          v[4 * q + 2] = x.z;
-          v[4 * q + 3] = x.w;
-        }
+        for (int u = 0; u < R; ++u) a4[u] = be_ld4(pa + off[u]);
+        pv += G * BE_B;
+        sw = (sw + G) & 3;
+        pa += G * ld;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = t + r * Tg;
-          const float a = (i < n) ? be_ld(sA + kk * ld + i) : 0.f;
+        for (int u = 0; u < R; ++u) {
+          const float a[4] = {a4[u].x, a4[u].y, a4[u].z, a4[u].w};
 #pragma unroll
-          for (int q = 0; q < BE_B; ++q) acc[r][q] = fmaf(a, v[q], acc[r][q]);
+          for (int e = 0; e < 4; ++e) {
+            acc[4 * u + e][0] = fmaf(a[e], x.x, acc[4 * u + e][0]);
+            acc[4 * u + e][1] = fmaf(a[e], x.y, acc[4 * u + e][1]);
+            acc[4 * u + e][2] = fmaf(a[e], x.z, acc[4 * u + e][2]);
+            acc[4 * u + e][3] = fmaf(a[e], x.w, acc[4 * u + e][3]);
+          }
         }
       }
     }
+    k0 += kc;
     __syncwarp();
-    if (lane == 0) be_arrive(&rg.empty[st]);
-    if (tid == 0 && c + BE_NS < nck) {
-      const uint32_t gn = base + (uint32_t)(c + BE_NS);
-      if (!tc::mbar_wait(&rg.empty[st], ((gn / BE_NS) + 1) & 1, rg.err, 23)) {
-        bad = true;
-        break;
-      }
-      issue(c + BE_NS);
+    if (lane == 0) {
+      be_arrive(&rg.empty[st]);
+      if ((c % (BE_T / 32)) == warp && c >= 1 && c - 1 + BE_NS < nck) bad = !refill(c - 1 + BE_NS);
+    }
+    __syncwarp();
+    if (++st == BE_NS) {
+      st = 0;
+      ph ^= 1;
     }
   }
   if (__syncthreads_or(bad)) {
     // leave only after every copy this CTA issued has landed (bounded)
-    if (tid == 0)
-      for (int j = 0; j < nck && j < c + BE_NS; ++j) {
-        const uint32_t gc = base + (uint32_t)j;
-        if (j >= c) tc::mbar_wait(&rg.full[gc % BE_NS], (gc / BE_NS) & 1, rg.err, 24);
-      }
+    if (tid == 0) {
+      const uint32_t end = *(volatile unsigned*)rg.issued;
+      for (uint32_t gc = end > BE_NS ? end - BE_NS : 0; gc < end; ++gc)
+        tc::mbar_wait(&rg.full[gc % BE_NS], (gc / BE_NS) & 1, rg.err, 24);
+    }
     __syncthreads();
     return false;
   }
@@ -242,23 +266,19 @@ __device__ bool be_matmul_r(int n, int ld, const TA* __restrict__ A, const float
   for (int gg = 0; gg < G; ++gg) {
     if (g == gg) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int i = t + r * Tg;
+      for (int r = 0; r < 4 * R; ++r) {
+        const int i = rb + 32 * (r >> 2) + (r & 3);
         if (i < n) {
-          float4* w = reinterpret_cast<float4*>(W + i * BE_B);
-          const int sw = i & 3;
-#pragma unroll
-          for (int q = 0; q < BE_B / 4; ++q) {
-            float4 x = make_float4(acc[r][4 * q], acc[r][4 * q + 1], acc[r][4 * q + 2], acc[r][4 * q + 3]);
-            if (gg > 0) {
-              const float4 y = w[q ^ sw];
-              x.x += y.x;
-              x.y += y.y;
-              x.z += y.z;
-              x.w += y.w;
-            }
-            w[q ^ sw] = x;
+          float4* w = reinterpret_cast<float4*>(W + i * BE_B) + (lc ^ (i & 3));
+          float4 x = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+          if (gg > 0) {
+            const float4 y = *w;
+            x.x += y.x;
+            x.y += y.y;
+            x.z += y.z;
+            x.w += y.w;
           }
+          *w = x;
         }
       }
     }
@@ -798,6 +818,7 @@ __global__ void __launch_bounds__(BE_T, 1) k_batch_si(BatchDev d) {
   float* W = V + BE_NMAX * BE_B;     // BE_NMAX x BE_B
   unsigned char* ring = reinterpret_cast<unsigned char*>(W + BE_NMAX * BE_B);  // BE_NS x BE_STAGE
   __shared__ uint64_t s_full[BE_NS], s_empty[BE_NS];
+  __shared__ unsigned s_issued;
   __shared__ float s_red[BE_T / 32 * BE_B];
   __shared__ int s_redi[BE_T / 32 * BE_B];
   __shared__ float s_c[BE_B];
@@ -814,6 +835,7 @@ __global__ void __launch_bounds__(BE_T, 1) k_batch_si(BatchDev d) {
   const int tid = threadIdx.x;
   const int b = d.b;
   if (tid == 0) {
+    s_issued = 0;
     for (int st = 0; st < BE_NS; ++st) {
       tc::mbar_init(&s_full[st], 1);
       tc::mbar_init(&s_empty[st], BE_T / 32);
@@ -821,7 +843,7 @@ __global__ void __launch_bounds__(BE_T, 1) k_batch_si(BatchDev d) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  BeRing rg{ring, s_full, s_empty, 0u, d.err};
+  BeRing rg{ring, s_full, s_empty, 0u, &s_issued, d.err};
   while (true) {
     if (tid == 0) s_job = (int)atomicAdd(d.queue, 1u);
     __syncthreads();
@@ -858,20 +880,19 @@ __global__ void __launch_bounds__(BE_T, 1) k_batch_si(BatchDev d) {
         __syncthreads();
       }
       // ---- Hessenberg basis of V (in place): MGS order, pivot on the first largest entry.  The
-      //      coefficients of column j come from a forward substitution on the pivot rows (thread 0, the
+      //      coefficients of column j come from a forward substitution on the pivot rows (a lane per row, the
       //      same fused multiply-adds in the same order as the column-by-column eliminations), then one
       //      pass updates the column and finds its pivot ----
       for (int j = 0; j < b; ++j) {
-        if (tid == 0) {
-          for (int l = 0; l < j; ++l) {
-            float cl = 0.f;
-            if (s_sel[l]) {
-              const int pr = s_perm[l];
-              cl = V[be_at(pr, j)];
-              for (int l2 = 0; l2 < l; ++l2) cl = fmaf(-s_c[l2], V[be_at(pr, l2)], cl);
-            }
-            s_c[l] = cl;
+        if (tid < 32) {  // lane l holds coefficient l
+          const bool on = tid < j && s_sel[min(tid, BE_B - 1)] != 0;
+          const int pr = on ? s_perm[tid] : 0;
+          float cl = on ? V[be_at(pr, j)] : 0.f;
+          for (int l2 = 0; l2 < j; ++l2) {
+            const float cf = __shfl_sync(0xffffffffu, cl, l2);
+            if (on && tid > l2) cl = fmaf(-cf, V[be_at(pr, l2)], cl);
           }
+          if (tid < j) s_c[tid] = cl;
         }
         __syncthreads();
         float bv = -1.f;
