@@ -512,135 +512,166 @@ __device__ double br_block_sum(double v, double* red) {
   return t;
 }
 
-// Rayleigh-Ritz of the symmetric pencil (G, M) of k2 <= 32 unit columns on one warp in FP64 (lane l owns
-// row / column l): M + tiny I = L L' with columns whose part outside the span of the earlier ones is
+// Rayleigh-Ritz of the symmetric pencil (G, M) of k2 <= 32 unit columns in FP64 by the whole CTA: M + tiny I = L L' with columns whose part outside the span of the earlier ones is
 // below 1e-4 of their norm dropped (their row and column of the pencil removed), C = L^-1 sym(G) L^-T,
 // a parallel cyclic Jacobi method (round-robin pairs, every round rotating k2 / 2 disjoint pairs), and
 // the kb largest eigenvalues' vectors Z = L^-T U (k2 x kb, row-major, into Zout).  All arrays k2 x k2
-// row-major in shared memory; G becomes U, M becomes C.
-__device__ void br_rayleigh_ritz_warp(int k2, int kb, double* G, double* M, double* L, double* T, double* Zout,
-                                      double* cs, int* pq, int* s_idx) {
-  const int lane = threadIdx.x & 31;
+// row-major with stride br_ld(k2) in shared memory; G becomes U, M becomes C.
+// An FP64 warp instruction takes 64 cycles of its SM sub-partition, so one warp (with 32-way bank conflicts in the
+// column passes) took 5.2 ms per step.  Warp 0 factors, substitutes and forms the rotations; a 2 x 2 block of C per
+// thread of 8 warps; U follows one round behind on the sub-partitions without warp 0, beside its next rotations.
+// The order of operations on each entry is unchanged: 0.9 ms for 32 columns.
+__host__ __device__ constexpr int br_ld(int k2) { return k2 + 1; }
+// c a - s b and s a + c b with one product rounded before the sum
+__device__ __forceinline__ double br_diff(double c, double a, double s, double b) {
+  return __fma_rn(c, a, -__dmul_rn(s, b));
+}
+__device__ __forceinline__ double br_sum(double s, double a, double c, double b) {
+  return __fma_rn(s, a, __dmul_rn(c, b));
+}
+
+__device__ void br_rayleigh_ritz(int k2, int kb, double* G, double* M, double* L, double* T, double* Zout, double* cs,
+                                 int* pq, int* s_idx) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ld = br_ld(k2);
   __shared__ int s_drop[BR_K2];
-  double mx = 0.0;
-  for (int i = 0; i < k2; ++i) mx = fmax(mx, M[i * k2 + i]);
-  for (int e = lane; e < k2 * k2; e += 32) L[e] = 0.0;
-  __syncwarp();
-  for (int j = 0; j < k2; ++j) {
-    // row j of L left of the diagonal is final
-    double dj = M[j * k2 + j] + 1e-14 * mx;
-    for (int q = 0; q < j; ++q) dj -= L[j * k2 + q] * L[j * k2 + q];
-    const bool drop = !(dj > 1e-8 * M[j * k2 + j]);
-    if (lane == 0) s_drop[j] = drop ? 1 : 0;
-    if (drop) {
-      __syncwarp();
-      for (int q = lane; q < k2; q += 32) {
-        L[j * k2 + q] = (q == j) ? 1.0 : 0.0;
-        G[j * k2 + q] = 0.0;
-        G[q * k2 + j] = 0.0;
+  __shared__ int s_go;
+  if (warp == 0) {
+    double mx = 0.0;
+    for (int i = 0; i < k2; ++i) mx = fmax(mx, M[i * ld + i]);
+    for (int e = lane; e < k2 * ld; e += 32) L[e] = 0.0;
+    __syncwarp();
+    for (int j = 0; j < k2; ++j) {
+      // row j of L left of the diagonal is final
+      double dj = M[j * ld + j] + 1e-14 * mx;
+      for (int q = 0; q < j; ++q) dj -= L[j * ld + q] * L[j * ld + q];
+      const bool drop = !(dj > 1e-8 * M[j * ld + j]);
+      if (lane == 0) s_drop[j] = drop ? 1 : 0;
+      if (drop) {
+        __syncwarp();
+        for (int q = lane; q < k2; q += 32) {
+          L[j * ld + q] = (q == j) ? 1.0 : 0.0;
+          G[j * ld + q] = 0.0;
+          G[q * ld + j] = 0.0;
+        }
+        __syncwarp();
+        continue;
+      }
+      dj = sqrt(dj);
+      const int i = lane;
+      double lij = 0.0;
+      if (i > j && i < k2) {
+        double v = M[i * ld + j];
+        for (int q = 0; q < j; ++q) v -= L[i * ld + q] * L[j * ld + q];
+        lij = v / dj;
       }
       __syncwarp();
-      continue;
+      if (i > j && i < k2) L[i * ld + j] = lij;
+      if (lane == 0) L[j * ld + j] = dj;
+      __syncwarp();
     }
-    dj = sqrt(dj);
-    const int i = lane;
-    double lij = 0.0;
-    if (i > j && i < k2) {
-      double v = M[i * k2 + j];
-      for (int q = 0; q < j; ++q) v -= L[i * k2 + q] * L[j * k2 + q];
-      lij = v / dj;
-    }
+    // T = L^-1 sym(G): lane c solves column c
+    for (int c = lane; c < k2; c += 32)
+      for (int i = 0; i < k2; ++i) {
+        double v = 0.5 * (G[i * ld + c] + G[c * ld + i]);
+        for (int q = 0; q < i; ++q) v -= L[i * ld + q] * T[q * ld + c];
+        T[i * ld + c] = v / L[i * ld + i];
+      }
     __syncwarp();
-    if (i > j && i < k2) L[i * k2 + j] = lij;
-    if (lane == 0) L[j * k2 + j] = dj;
+    // C = T L^-T: lane r solves row r (into M)
+    for (int r = lane; r < k2; r += 32)
+      for (int i = 0; i < k2; ++i) {
+        double v = T[r * ld + i];
+        for (int q = 0; q < i; ++q) v -= L[i * ld + q] * M[r * ld + q];
+        M[r * ld + i] = v / L[i * ld + i];
+      }
     __syncwarp();
   }
-  // T = L^-1 sym(G): lane c solves column c
-  for (int c = lane; c < k2; c += 32)
-    for (int i = 0; i < k2; ++i) {
-      double v = 0.5 * (G[i * k2 + c] + G[c * k2 + i]);
-      for (int q = 0; q < i; ++q) v -= L[i * k2 + q] * T[q * k2 + c];
-      T[i * k2 + c] = v / L[i * k2 + i];
-    }
-  __syncwarp();
-  // C = T L^-T: lane r solves row r (into M)
-  for (int r = lane; r < k2; r += 32)
-    for (int i = 0; i < k2; ++i) {
-      double v = T[r * k2 + i];
-      for (int q = 0; q < i; ++q) v -= L[i * k2 + q] * M[r * k2 + q];
-      M[r * k2 + i] = v / L[i * k2 + i];
-    }
-  __syncwarp();
   double* Cm = M;
   double* U = G;
-  for (int e = lane; e < k2 * k2; e += 32) {
-    const int i = e / k2, j = e % k2;
-    U[e] = (i == j) ? 1.0 : 0.0;
-    if (i < j) {
-      const double a = 0.5 * (Cm[i * k2 + j] + Cm[j * k2 + i]);
-      Cm[i * k2 + j] = a;
-      Cm[j * k2 + i] = a;
+  __syncthreads();
+  if (warp == 0) {
+    for (int e = lane; e < k2 * k2; e += 32) {
+      const int i = e / k2, j = e % k2;
+      U[i * ld + j] = (i == j) ? 1.0 : 0.0;
+      if (i < j) {
+        const double a = 0.5 * (Cm[i * ld + j] + Cm[j * ld + i]);
+        Cm[i * ld + j] = a;
+        Cm[j * ld + i] = a;
+      }
     }
   }
-  __syncwarp();
+  __syncthreads();
   const int np = k2 / 2;
+  auto rotate_u = [&](const double* c2, const int* p2, int m) {  // U = U J, pair m (row `lane`)
+    if (lane < k2) {
+      const int p = p2[2 * m], q = p2[2 * m + 1];
+      const double c = c2[2 * m], sn = c2[2 * m + 1];
+      const double up = U[lane * ld + p], uq = U[lane * ld + q];
+      U[lane * ld + p] = br_diff(c, up, sn, uq);
+      U[lane * ld + q] = br_sum(sn, up, c, uq);
+    }
+  };
   for (int sweep = 0; sweep < 20; ++sweep) {
-    double off = 0.0, dn = 0.0;
-    for (int e = lane; e < k2 * k2; e += 32) {
-      const double v = Cm[e] * Cm[e];
-      if (e / k2 != e % k2) off += v;
-      else dn += v;
-    }
+    if (warp == 0) {
+      double off = 0.0, dn = 0.0;
+      for (int e = lane; e < k2 * k2; e += 32) {
+        const double x = Cm[(e / k2) * ld + e % k2], v = x * x;
+        if (e / k2 != e % k2) off += v;
+        else dn += v;
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_xor_sync(0xffffffffu, off, o);
-      dn += __shfl_xor_sync(0xffffffffu, dn, o);
+      for (int o = 16; o > 0; o >>= 1) {
+        off += __shfl_xor_sync(0xffffffffu, off, o);
+        dn += __shfl_xor_sync(0xffffffffu, dn, o);
+      }
+      if (lane == 0) s_go = (off <= 1e-28 * dn) ? 0 : 1;
     }
-    if (off <= 1e-28 * dn) break;
+    __syncthreads();
+    if (!s_go) break;
     for (int round = 0; round < k2 - 1; ++round) {
-      if (lane < np) {  // round-robin pairs: position 0 fixed, the others rotate
+      double* c2 = cs + (round & 1) * BR_K2;
+      int* p2 = pq + (round & 1) * BR_K2;
+      if (tid < np) {  // round-robin pairs: position 0 fixed, the others rotate
         const int a = (lane == 0) ? 0 : 1 + (lane - 1 + round) % (k2 - 1);
         const int b = 1 + (k2 - 2 - lane + round) % (k2 - 1);
         const int p = min(a, b), q = max(a, b);
-        const double apq = Cm[p * k2 + q];
+        const double apq = Cm[p * ld + q];
         double c = 1.0, sn = 0.0;
         if (fabs(apq) > 1e-300) {
-          const double theta = (Cm[q * k2 + q] - Cm[p * k2 + p]) / (2.0 * apq);
-          const double tt = copysign(1.0, theta) / (fabs(theta) + sqrt(fma(theta, theta, 1.0)));
-          c = 1.0 / sqrt(fma(tt, tt, 1.0));
+          const double theta = (Cm[q * ld + q] - Cm[p * ld + p]) / (2.0 * apq);
+          const double tt = copysign(__drcp_rn(fabs(theta) + sqrt(fma(theta, theta, 1.0))), theta);
+          c = __drcp_rn(sqrt(fma(tt, tt, 1.0)));
           sn = tt * c;
         }
-        cs[2 * lane] = c;
-        cs[2 * lane + 1] = sn;
-        pq[2 * lane] = p;
-        pq[2 * lane + 1] = q;
+        c2[2 * lane] = c;
+        c2[2 * lane + 1] = sn;
+        p2[2 * lane] = p;
+        p2[2 * lane + 1] = q;
+      } else if ((warp & 3) != 0 && round > 0) {  // the previous round's rotations of U
+        for (int m = warp - (warp >> 2) - 1; m < np; m += BE_T / 32 - BE_T / 128)
+          rotate_u(cs + ((round & 1) ^ 1) * BR_K2, pq + ((round & 1) ^ 1) * BR_K2, m);
       }
-      __syncwarp();
-      if (lane < k2) {  // columns: C = C J, U = U J (row `lane`)
-        for (int m = 0; m < np; ++m) {
-          const int p = pq[2 * m], q = pq[2 * m + 1];
-          const double c = cs[2 * m], sn = cs[2 * m + 1];
-          const double sp = Cm[lane * k2 + p], sq = Cm[lane * k2 + q];
-          Cm[lane * k2 + p] = c * sp - sn * sq;
-          Cm[lane * k2 + q] = sn * sp + c * sq;
-          const double up = U[lane * k2 + p], uq = U[lane * k2 + q];
-          U[lane * k2 + p] = c * up - sn * uq;
-          U[lane * k2 + q] = sn * up + c * uq;
-        }
+      __syncthreads();
+      for (int e = tid; e < np * np; e += BE_T) {  // C = J' C J, block (pair m, pair m2): columns, then rows
+        const int m = e % np, m2 = e / np;
+        const int p = p2[2 * m], q = p2[2 * m + 1], p1 = p2[2 * m2], q1 = p2[2 * m2 + 1];
+        const double c = c2[2 * m], sn = c2[2 * m + 1], c1 = c2[2 * m2], s1 = c2[2 * m2 + 1];
+        const double a = Cm[p * ld + p1], b = Cm[p * ld + q1], x = Cm[q * ld + p1], y = Cm[q * ld + q1];
+        const double ap = br_diff(c1, a, s1, b), aq = br_sum(s1, a, c1, b);
+        const double xp = br_diff(c1, x, s1, y), xq = br_sum(s1, x, c1, y);
+        Cm[p * ld + p1] = br_diff(c, ap, sn, xp);
+        Cm[q * ld + p1] = br_sum(sn, ap, c, xp);
+        Cm[p * ld + q1] = br_diff(c, aq, sn, xq);
+        Cm[q * ld + q1] = br_sum(sn, aq, c, xq);
       }
-      __syncwarp();
-      if (lane < k2) {  // rows: C = J' C (column `lane`)
-        for (int m = 0; m < np; ++m) {
-          const int p = pq[2 * m], q = pq[2 * m + 1];
-          const double c = cs[2 * m], sn = cs[2 * m + 1];
-          const double sp = Cm[p * k2 + lane], sq = Cm[q * k2 + lane];
-          Cm[p * k2 + lane] = c * sp - sn * sq;
-          Cm[q * k2 + lane] = sn * sp + c * sq;
-        }
-      }
-      __syncwarp();
+      __syncthreads();
     }
+    for (int m = warp; m < np; m += BE_T / 32)
+      rotate_u(cs + ((k2 - 2) & 1) * BR_K2, pq + ((k2 - 2) & 1) * BR_K2, m);
+    __syncthreads();
   }
+  if (warp != 0) return;
   // the kb largest eigenvalues among the kept directions (a dropped index keeps U = e_j, C_jj = 0)
   if (lane == 0) {
     int nk = 0;
@@ -649,7 +680,7 @@ __device__ void br_rayleigh_ritz_warp(int k2, int kb, double* G, double* M, doub
     for (int i = 1; i < nk; ++i) {
       const int v = s_idx[i];
       int j = i - 1;
-      while (j >= 0 && Cm[s_idx[j] * k2 + s_idx[j]] < Cm[v * k2 + v]) {
+      while (j >= 0 && Cm[s_idx[j] * ld + s_idx[j]] < Cm[v * ld + v]) {
         s_idx[j + 1] = s_idx[j];
         --j;
       }
@@ -662,13 +693,13 @@ __device__ void br_rayleigh_ritz_warp(int k2, int kb, double* G, double* M, doub
   for (int c = lane; c < kb; c += 32) {
     const int src = s_idx[c];
     for (int i = k2 - 1; i >= 0; --i) {
-      double v = U[i * k2 + src];
-      for (int q = i + 1; q < k2; ++q) v -= L[q * k2 + i] * T[q * k2 + c];
-      T[i * k2 + c] = v / L[i * k2 + i];
+      double v = U[i * ld + src];
+      for (int q = i + 1; q < k2; ++q) v -= L[q * ld + i] * T[q * ld + c];
+      T[i * ld + c] = v / L[i * ld + i];
     }
   }
   __syncwarp();
-  for (int e = lane; e < k2 * kb; e += 32) Zout[e] = T[(e / kb) * k2 + (e % kb)];
+  for (int e = lane; e < k2 * kb; e += 32) Zout[e] = T[(e / kb) * ld + (e % kb)];
   __syncwarp();
 }
 
@@ -677,17 +708,19 @@ __device__ void br_rayleigh_ritz_warp(int k2, int kb, double* G, double* M, doub
 // the nev leading pairs meet tol (or `steps` steps).  The guard columns keep the nearby part of the
 // spectrum inside the search space, so each step removes the error along it instead of only damping it.
 // One matrix (index mi, order n) from its FP32 block in d.X32.  Xs: BE_NMAX x BE_B doubles of shared memory
-// (the right-hand block of a product); arena: 4 BR_K2^2 + BR_K2 BE_B doubles of shared memory (the pencil).
+// (the right-hand block of a product); arena: 4 BR_K2 br_ld(BR_K2) + BR_K2 BE_B doubles of shared memory
+// (the pencil).
 __device__ void be_refine_one(const RefineDev& d, int mi, int n, double* Xs, double* arena) {
   __shared__ double s_red[BE_T / 32];
   __shared__ double s_lam[2 * BE_B];
-  __shared__ double s_cs[BR_K2];
-  __shared__ int s_pq[BR_K2], s_idx[BR_K2];
+  __shared__ double s_cs[2 * BR_K2];
+  __shared__ int s_pq[2 * BR_K2], s_idx[BR_K2];
   double* s_G = arena;
-  double* s_M = s_G + BR_K2 * BR_K2;
-  double* s_L = s_M + BR_K2 * BR_K2;
-  double* s_T = s_L + BR_K2 * BR_K2;
-  double* s_Z = s_T + BR_K2 * BR_K2;
+  constexpr int kArr = BR_K2 * br_ld(BR_K2);
+  double* s_M = s_G + kArr;
+  double* s_L = s_M + kArr;
+  double* s_T = s_L + kArr;
+  double* s_Z = s_T + kArr;
   double* br_sm = Xs;
   const int tid = threadIdx.x;
   const int kb = d.b, k2 = 2 * d.b, nev = d.nev;
@@ -768,13 +801,13 @@ __device__ void be_refine_one(const RefineDev& d, int mi, int n, double* Xs, dou
           for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
           if (lane == 0) {
             double* D = which ? s_M : s_G;
-            D[r * k2 + c] = acc;
-            D[c * k2 + r] = acc;
+            D[r * br_ld(k2) + c] = acc;
+            D[c * br_ld(k2) + r] = acc;
           }
         }
       }
       __syncthreads();
-      if (tid < 32) br_rayleigh_ritz_warp(k2, kb, s_G, s_M, s_L, s_T, s_Z, s_cs, s_pq, s_idx);
+      br_rayleigh_ritz(k2, kb, s_G, s_M, s_L, s_T, s_Z, s_cs, s_pq, s_idx);
       __syncthreads();
       // X <- [X R] Z, A X <- [AX AR] Z
       for (int e = tid; e < 2 * n; e += BE_T) {
