@@ -633,6 +633,9 @@ int kry_sum_unit_cols(ofrr_ctx* ctx, ofrr_dtype tw, int64_t n, int k, const void
 // partial sums): the exact-arithmetic Gram products of a Rayleigh-Ritz step
 int gram_f64(ofrr_ctx* ctx, int64_t M, int64_t N, int64_t K, const double* A, int64_t lda, const double* B,
              int64_t ldb, double* C, int64_t ldc);
+// G = V' W and M = V' V (b x b, ld b) for FP64 V, W of K rows, b <= 128, one pass over both (gram_pair.cu)
+int gram_pair_f64(ofrr_ctx* ctx, int64_t K, int b, const double* V, int64_t ldv, const double* W, int64_t ldw, double* G,
+                  double* M);
 // C (M x N) = A (M x K) B (K x N), FP64 on the CUDA cores (K <= 256): exact-arithmetic back-transforms
 int tsmm_f64(ofrr_ctx* ctx, int64_t M, int64_t N, int64_t K, const double* A, int64_t lda, const double* B,
              int64_t ldb, double* C, int64_t ldc);

@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(128) k_backtransform16(int64_t m, int b, const
 // Out (type tq) = tq(gemm(Q, Cf, pmc) rounded to pmo): the fused kernel for 16-bit bases with FP32
 // compute and output, the general product and cast otherwise
 int back_transform(ofrr_ctx* ctx, ofrr_dtype tq, ofrr_dtype pmc, ofrr_dtype pmo, int64_t m, int b, const void* Q,
-                   int64_t ldq, const double* Cf, void* Out, int64_t ldo) {
+                   int64_t ldq, const double* Cf, void* Out, int64_t ldo, bool exact = false) {
   if ((tq == OFRR_F16 || tq == OFRR_BF16) && pmc == OFRR_F32 && pmo == OFRR_F32 && b <= 128 && Out != Q) {
     const dim3 grid((unsigned)((m + 127) / 128), (unsigned)((b + 31) / 32));
     if (tq == OFRR_F16)
@@ -388,7 +388,8 @@ int back_transform(ofrr_ctx* ctx, ofrr_dtype tq, ofrr_dtype pmc, ofrr_dtype pmo,
     if (!Vn) return st;
     ldvn = m;
   }
-  OFRR_TRY(gemm_impl(ctx, 0, 0, tq, OFRR_F64, pmc, pmo, m, b, b, 1.0, Q, ldq, Cf, b, 0.0, Vn, ldvn));
+  if (exact) OFRR_TRY(tsmm_f64(ctx, m, b, b, (const double*)Q, ldq, Cf, b, (double*)Vn, ldvn));
+  else OFRR_TRY(gemm_impl(ctx, 0, 0, tq, OFRR_F64, pmc, pmo, m, b, b, 1.0, Q, ldq, Cf, b, 0.0, Vn, ldvn));
   if (Vn != Out) OFRR_TRY(cast_impl(ctx, pmo, tq, m, b, Vn, ldvn, Out, ldo));
   return OFRR_SUCCESS;
 }
@@ -431,13 +432,27 @@ int rr_eig_dev(ofrr_ctx* ctx, Op& op, ofrr_dtype ta, const void* Q, ofrr_dtype t
   OFRR_TRY(dmalloc(ctx, &U, (size_t)b * b));
   void* tmp = ws_alloc(ctx, (size_t)b * b * dtype_size(pmo), &st);
   if (!tmp) return st;
-  // VAV = peig(gemm(V, 'T', AV, pmc, pmo))
-  OFRR_TRY(gemm_impl(ctx, 1, 0, tq, tav, pmc, pmo, b, b, n, 1.0, Q, ldq, AV, n, 0.0, tmp, b));
-  OFRR_TRY(cast_impl(ctx, pmo, OFRR_F64, b, b, tmp, b, G, b));
+  // VAV = peig(gemm(V, 'T', AV, pmc, pmo)), VV = gemm(V, 'T', V, pmc, pmo).  The reference's FP64 step on a
+  // symmetric operator takes both from one pass over V and AV (if its partial sums fit in the workspace); the
+  // 16-bit, emulated and single-precision steps and the nonsymmetric solver keep a product each.
+  if (use_gen) OFRR_TRY(dmalloc(ctx, &M, (size_t)b * b));
+  const bool f64 = tq == OFRR_F64 && tav == OFRR_F64 && pmc == OFRR_F64 && pmo == OFRR_F64;
+  const bool own = f64 && use_gen && symmetric && !fast && b <= 128 && !ctx->emulate_f64;
+  bool paired = false;
+  if (own) {
+    const int gst = gram_pair_f64(ctx, n, b, (const double*)Q, ldq, (const double*)AV, n, G, M);
+    if (gst != OFRR_SUCCESS && gst != OFRR_ERR_OUT_OF_MEMORY) return gst;
+    paired = gst == OFRR_SUCCESS;
+  }
+  if (!paired) {
+    OFRR_TRY(gemm_impl(ctx, 1, 0, tq, tav, pmc, pmo, b, b, n, 1.0, Q, ldq, AV, n, 0.0, tmp, b));
+    OFRR_TRY(cast_impl(ctx, pmo, OFRR_F64, b, b, tmp, b, G, b));
+  }
   if (use_gen) {
-    OFRR_TRY(dmalloc(ctx, &M, (size_t)b * b));
-    OFRR_TRY(gemm_impl(ctx, 1, 0, tq, tq, pmc, pmo, b, b, n, 1.0, Q, ldq, Q, ldq, 0.0, tmp, b));
-    OFRR_TRY(cast_impl(ctx, pmo, OFRR_F64, b, b, tmp, b, M, b));
+    if (!paired) {
+      OFRR_TRY(gemm_impl(ctx, 1, 0, tq, tq, pmc, pmo, b, b, n, 1.0, Q, ldq, Q, ldq, 0.0, tmp, b));
+      OFRR_TRY(cast_impl(ctx, pmo, OFRR_F64, b, b, tmp, b, M, b));
+    }
     if (gtol != 0.0 && !(fast && symmetric && b <= 128)) {
       k_add_diag<<<(b + 255) / 256, 256, 0, ctx->stream>>>(b, M, b, gtol);
       OFRR_LAUNCHED(ctx, "k_add_diag");
@@ -452,7 +467,7 @@ int rr_eig_dev(ofrr_ctx* ctx, Op& op, ofrr_dtype ta, const void* Q, ofrr_dtype t
     OFRR_TRY(geig_dev(ctx, b, G, b, M, b, symmetric ? 1 : 0, d, U, b));
   }
   // V = gemm(V, 'N', U, pmc, pmo) then back to V's precision
-  return back_transform(ctx, tq, pmc, pmo, n, b, Q, ldq, U, Vout, ldvo);
+  return back_transform(ctx, tq, pmc, pmo, n, b, Q, ldq, U, Vout, ldvo, own);
 }
 
 // at most 4 CTAs per column: each thread handles several rows of one column
