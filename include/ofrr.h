@@ -487,6 +487,9 @@ int ofrr_ctx_trim(ofrr_ctx* ctx);
  * usable.  No fault, trap or unbounded wait is involved. */
 int ofrr_debug_bounded_wait(ofrr_ctx* ctx, int64_t timeout_ns);
 
+/* Self-test of the short FP64 operations of the latency-bound kernels: out[i] = 1 / a[i] (op 0), a[i] / b[i] (1),
+ * sqrt(a[i]) (2); device arrays of n. */
+int ofrr_debug_f64_ops(ofrr_ctx* ctx, int op, int64_t n, const double* a, const double* b, double* out);
 /* Self-test of the fused scale-and-split kernels of the emulated FP64 power iteration (no reference
  * counterpart; the power loop of subspace_iter_svd.m:63-69, scalecols.m after each product).
  * mode 0: X (M x N, M <= 8192) is scaled in place as ofrr_scalecols does (FP64, reciprocal multiply);

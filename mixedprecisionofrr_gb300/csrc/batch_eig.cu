@@ -23,6 +23,7 @@
 //    input until the FP64 residuals of the nev leading pairs meet tol (usually one step; at most 12).
 // Bounded waits only: the queue is one atomic counter; the copy ring's mbarrier waits give up after ~2 s
 // (status word, then the CTA leaves).
+#include "f64_ops.cuh"
 #include "ofrr_internal.cuh"
 #include "tcgen05.cuh"
 
@@ -639,9 +640,9 @@ __device__ void br_rayleigh_ritz(int k2, int kb, double* G, double* M, double* L
         const double apq = Cm[p * ld + q];
         double c = 1.0, sn = 0.0;
         if (fabs(apq) > 1e-300) {
-          const double theta = (Cm[q * ld + q] - Cm[p * ld + p]) / (2.0 * apq);
-          const double tt = copysign(__drcp_rn(fabs(theta) + sqrt(fma(theta, theta, 1.0))), theta);
-          c = __drcp_rn(sqrt(fma(tt, tt, 1.0)));
+          const double theta = f64::div(Cm[q * ld + q] - Cm[p * ld + p], 2.0 * apq);
+          const double tt = copysign(f64::rcp(fabs(theta) + f64::sqrt(fma(theta, theta, 1.0))), theta);
+          c = f64::rcp(f64::sqrt(fma(tt, tt, 1.0)));
           sn = tt * c;
         }
         c2[2 * lane] = c;

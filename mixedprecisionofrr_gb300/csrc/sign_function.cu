@@ -17,6 +17,7 @@
 // logarithm and block barriers in every step's chain).
 #include <algorithm>
 
+#include "f64_ops.cuh"
 #include "ofrr_internal.cuh"
 #include "tcgen05.cuh"
 
@@ -157,7 +158,7 @@ __global__ void __launch_bounds__(32 * kSignWarps, 1) k_sign_cluster(int n, doub
           for (int t = 0; t < kSignCtas - 1; ++t) push_f64(base[t] + (kSignHead + i) * 8, rbar[t], s);
         }
       }
-      const double dinv = __drcp_rn(d);
+      const double dinv = f64::rcp(d);
       if (lane < kSignHead) {
         const double h = (lane == 0) ? __longlong_as_double((long long)p) : (lane == 1) ? d : dinv;
         mine[lane] = h;

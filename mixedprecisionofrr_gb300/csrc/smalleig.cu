@@ -11,6 +11,7 @@
 // algorithm on one CTA in a global workspace (k_geig_sym).
 #include <atomic>
 
+#include "f64_ops.cuh"
 #include "ofrr_internal.cuh"
 
 namespace ofrr {
@@ -21,7 +22,7 @@ namespace ofrr {
 // GB300 runs FP64 at 1/64 of its FP32 rate (a warp instruction occupies an SM sub-partition for about 64
 // cycles), so the sweeps are bound by the FP64 pipe of the SMs they run on and, between two barriers, by
 // the dependent chain that turns (a_pp, a_qq, a_pq) into a rotation (measured on 16 CTAs at n = 64, cycles
-// per round: rotations 3260, C 1100, handing over 100, barrier 1180).  The rotations of a round are
+// per round: rotations ~1700, C 1100, handing over 100, barrier 1180).  The rotations of a round are
 // independent, so they are spread over a cluster: CTA c owns the seats of PP = ceil(N / 2 / NC) pairs of
 // the round-robin schedule, i.e. 2 PP columns of C and of W.  Rows and columns of a 2 x 2 block only
 // depend on that block, so a round is one pass over the CTA's columns; the new columns go straight to the
@@ -33,8 +34,9 @@ constexpr int kJacT = 512;
 constexpr int kGeigClusterMaxN = 144;  // Cholesky, substitutions and L beside 32 columns in one CTA's 227 KB
 
 // The rotation of sym.Schur2 (t the root of smaller magnitude of t^2 + 2 tau t - 1 = 0, t = 1 for tau = 0).
-// Divisions and square roots are FP64 sequences of about 430 cycles each, so the chain takes ~2000 cycles, the
-// largest part of a round.  Taking the angle in FP32 and normalising (c, s) in FP64 halves it, but on the SVD
+// The chain's divisions and square roots (560 and 630 cycles each as plain operations) were the largest part of a
+// round, 3260 cycles; in their short forms (f64_ops.cuh, the same values) it takes half of that.  Taking the angle in
+// FP32 and normalising (c, s) in FP64 would shorten it as much, but on the SVD
 // pencil [[0, K], [K', 0]] of a block U ~ A V the matrix K is triangular up to rounding, equal diagonal entries
 // meet entries of rounding size, and which of the two roots is taken (the sign of the vectors) then hangs on the
 // last bits: the quotients keep every result what the one-CTA form gives, bit for bit.
@@ -45,9 +47,9 @@ __device__ __forceinline__ void jac_rotation(double app, double aqq, double apq,
   *c = 1.0;
   *s = 0.0;
   if (!jac_nonzero(apq)) return;
-  const double tau = (aqq - app) / (2.0 * apq);
-  const double t = __drcp_rn(fabs(tau) + sqrt(1.0 + tau * tau));
-  *c = __drcp_rn(sqrt(1.0 + t * t));
+  const double tau = f64::div(aqq - app, 2.0 * apq);
+  const double t = f64::rcp(fabs(tau) + f64::sqrt(__fma_rn(tau, tau, 1.0)));
+  *c = f64::rcp(f64::sqrt(__fma_rn(t, t, 1.0)));
   const double sa = t * *c;
   *s = (__double2hiint(tau) < 0 && jac_nonzero(tau)) ? -sa : sa;
 }
@@ -886,4 +888,22 @@ extern "C" int ofrr_syev(ofrr_ctx* ctx, int n, double* A, int lda, double* w) {
 extern "C" int ofrr_sygv(ofrr_ctx* ctx, int n, double* A, int lda, double* B, int ldb, double* w) {
   if (!ctx || n < 0 || (n > 0 && (!A || !B || !w || lda < n || ldb < n))) return OFRR_ERR_INVALID_ARGUMENT;
   return sygv_dev(ctx, n, A, lda, B, ldb, w);
+}
+
+namespace ofrr {
+namespace {
+__global__ void k_f64_ops(int op, int64_t n, const double* __restrict__ a, const double* __restrict__ b,
+                          double* __restrict__ out) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = op == 0 ? f64::rcp(a[i]) : op == 1 ? f64::div(a[i], b[i]) : f64::sqrt(a[i]);
+}
+}  // namespace
+}  // namespace ofrr
+
+// Self-test of the short FP64 operations (f64_ops.cuh): out[i] = 1 / a[i] (op 0), a[i] / b[i] (1), sqrt(a[i]) (2)
+extern "C" int ofrr_debug_f64_ops(ofrr_ctx* ctx, int op, int64_t n, const double* a, const double* b, double* out) {
+  if (!ctx || op < 0 || op > 2 || n < 1 || !a || !out || (op == 1 && !b)) return OFRR_ERR_INVALID_ARGUMENT;
+  k_f64_ops<<<grid_for(n, 256, 152 * 8), 256, 0, ctx->stream>>>(op, n, a, b, out);
+  OFRR_LAUNCHED(ctx, "k_f64_ops");
+  return sync_and_check(ctx);
 }

@@ -16,6 +16,7 @@
 // eigenvector of a complex pair is the real part of the complex eigenvector, every vector has unit
 // 2-norm, and pairs are sorted by descending real part (stable).  Accuracy is FP32 relative to
 // ||C||; the callers are the 16-bit/32-bit Krylov bases of the mixed schedule.
+#include "f64_ops.cuh"
 #include "ofrr_internal.cuh"
 
 namespace ofrr {
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(VEC ? 64 : 32) k_nonsym_eig(int nn, const doub
           x = fabs(p) + fabs(q) + fabs(r);
           if constexpr (sizeof(T) == 8) {  // three quotients in three lanes
             if (ns_zero(x)) continue;
-            const T quo = ((lane == 0) ? p : (lane == 1) ? q : r) / x;
+            const T quo = f64::div((lane == 0) ? p : (lane == 1) ? q : r, x);
             p = __shfl_sync(0xffffffffu, quo, 0);
             q = __shfl_sync(0xffffffffu, quo, 1);
             r = __shfl_sync(0xffffffffu, quo, 2);
@@ -371,11 +372,13 @@ __global__ void __launch_bounds__(VEC ? 64 : 32) k_nonsym_eig(int nn, const doub
             r /= x;
           }
         }
-        s = sqrt(p * p + q * q + r * r);
+        s = p * p + q * q + r * r;
         if constexpr (sizeof(T) == 8) {
+          s = f64::sqrt(s);
           if (ns_neg(p)) s = -s;
           if (ns_zero(s)) continue;
         } else {
+          s = sqrt(s);
           if (p < T(0.)) s = -s;
           if (s == T(0.)) continue;
         }
@@ -383,7 +386,7 @@ __global__ void __launch_bounds__(VEC ? 64 : 32) k_nonsym_eig(int nn, const doub
         const bool set_hk = (k != m) || (l != m);
         p = p + s;
         if constexpr (sizeof(T) == 8) {  // five quotients in five lanes
-          const T quo = ((lane == 0) ? p : (lane == 1 || lane == 3) ? q : r) / (lane < 3 ? s : p);
+          const T quo = f64::div((lane == 0) ? p : (lane == 1 || lane == 3) ? q : r, lane < 3 ? s : p);
           x = __shfl_sync(0xffffffffu, quo, 0);
           y = __shfl_sync(0xffffffffu, quo, 1);
           z = __shfl_sync(0xffffffffu, quo, 2);
