@@ -23,6 +23,7 @@
 //    stop[0] and turns the remaining launches of the cycle into no-ops.
 // HBM traffic of step i: CSR (nnz (4 + s_a) + 4 n) + staging read and write (2 n s_e) + the column
 // write (n s) + i - 1 earlier columns (n s each) + the pivot marks (n), s = sizeof(T).
+#include "f64_ops.cuh"
 #include "ofrr_internal.cuh"
 
 namespace ofrr {
@@ -493,41 +494,71 @@ __global__ void k_kry_addcol(int64_t n, TW* __restrict__ w, const TA* __restrict
     w[i] = from_c<TW, double>(to_c<double, TW>(w[i]) + to_c<double, TA>(a[i]));
 }
 
-// x = M^-1 g for the SPD Gram matrix M (nc x nc, FP64): Cholesky in shared memory, one CTA
+// x = M^-1 g for the SPD Gram matrix M (nc x nc, FP64): Cholesky in shared memory, one CTA.  The last warp forms the
+// next pivot's root beside the trailing update of the others, the forward substitution takes a row per thread; the
+// backward one adds its products in ascending order, so each sum waits for the solution before it.
 __global__ void __launch_bounds__(256) k_kry_spd_solve(int nc, const double* __restrict__ M,
                                                        const double* __restrict__ g, double* __restrict__ x) {
   extern __shared__ double sl[];  // nc x nc (column-major), then nc
-  __shared__ double s_d;
+  __shared__ double s_d[2];
   double* y = sl + (size_t)nc * nc;
   const int tid = threadIdx.x;
   for (int e = tid; e < nc * nc; e += blockDim.x) sl[e] = M[e];
   for (int e = tid; e < nc; e += blockDim.x) y[e] = g[e];
   __syncthreads();
+  const int lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  auto root = [&](int j) {
+    const double v = sl[j + (size_t)j * nc];
+    s_d[j & 1] = f64::sqrt(v > 0.0 ? v : 0.0);
+  };
+  if (tid == 0) root(0);
+  __syncthreads();
   for (int j = 0; j < nc; ++j) {  // right-looking: column j, then the trailing update
-    if (tid == 0) s_d = sqrt(fmax(sl[j + (size_t)j * nc], 0.0));
-    __syncthreads();
-    const double d = s_d;
+    const double d = s_d[j & 1];
     for (int i = j + 1 + tid; i < nc; i += blockDim.x)
-      sl[i + (size_t)j * nc] = (d > 0.0) ? sl[i + (size_t)j * nc] / d : 0.0;
+      sl[i + (size_t)j * nc] = (d > 0.0) ? f64::div(sl[i + (size_t)j * nc], d) : 0.0;
     if (tid == 0) sl[j + (size_t)j * nc] = d;
     __syncthreads();
-    const int w = nc - j - 1;
-    for (int e = tid; e < w * w; e += blockDim.x) {
-      const int c = j + 1 + e / w, r = j + 1 + e % w;
-      if (r >= c) sl[r + (size_t)c * nc] -= sl[r + (size_t)j * nc] * sl[c + (size_t)j * nc];
+    if (warp == nw - 1) {
+      if (lane == 0 && j + 1 < nc) {
+        const double l = sl[j + 1 + (size_t)j * nc];
+        sl[j + 1 + (size_t)(j + 1) * nc] = fma(-l, l, sl[j + 1 + (size_t)(j + 1) * nc]);
+        root(j + 1);
+      }
+    } else {
+      for (int c = j + 1 + warp; c < nc; c += nw - 1) {
+        const double lc = sl[c + (size_t)j * nc];
+        for (int r = (c == j + 1 ? c + 1 : c) + lane; r < nc; r += 32)
+          sl[r + (size_t)c * nc] = fma(-sl[r + (size_t)j * nc], lc, sl[r + (size_t)c * nc]);
+      }
     }
     __syncthreads();
   }
-  if (tid == 0) {  // L y = g, then L' x = y
-    for (int i = 0; i < nc; ++i) {
-      double t = y[i];
-      for (int k = 0; k < i; ++k) t -= sl[i + (size_t)k * nc] * y[k];
-      y[i] = (sl[i + (size_t)i * nc] > 0.0) ? t / sl[i + (size_t)i * nc] : 0.0;
-    }
+  for (int k = 0; k < nc; ++k) {  // L y = g: y_k, then its products out of every later row
+    const double dk = sl[k + (size_t)k * nc];
+    if (tid == 0) y[k] = (dk > 0.0) ? f64::div(y[k], dk) : 0.0;
+    __syncthreads();
+    const double yk = y[k];
+    for (int i = k + 1 + tid; i < nc; i += blockDim.x) y[i] = fma(-sl[i + (size_t)k * nc], yk, y[i]);
+    __syncthreads();
+  }
+  if (tid == 0) {  // L' x = y
     for (int i = nc - 1; i >= 0; --i) {
+      const double* l = sl + (size_t)i * nc;
       double t = y[i];
-      for (int k = i + 1; k < nc; ++k) t -= sl[k + (size_t)i * nc] * y[k];
-      y[i] = (sl[i + (size_t)i * nc] > 0.0) ? t / sl[i + (size_t)i * nc] : 0.0;
+      int k = i + 1;
+      for (; k + 8 <= nc; k += 8) {
+        double a[8], c[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          a[u] = l[k + u];
+          c[u] = y[k + u];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t = fma(-a[u], c[u], t);
+      }
+      for (; k < nc; ++k) t = fma(-l[k], y[k], t);
+      y[i] = (l[i] > 0.0) ? f64::div(t, l[i]) : 0.0;
     }
     for (int i = 0; i < nc; ++i) x[i] = y[i];
   }

@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(32) k_back_subst(int n, const double* __restri
       for (int u = 0; u < 8; ++u) s = __fma_rn(-a[u], b[u], s);
     }
     for (; k < n; ++k) s = __fma_rn(-l[k], sU[k * 32 + lane], s);
-    s = s / l[r];
+    s = f64::div(s, l[r]);
     sU[r * 32 + lane] = s;
     if (store) U[r + (size_t)j * ldu] = s;
   }

@@ -17,6 +17,7 @@
 // The SVD form (svd_rr.m's pencil [[0,B],[B',0]] vs blkdiag(U'U, V'V) + tau I) reduces with two
 // Cholesky factors to the SVD of C = Lu^-1 B Lv^-T; its right singular vectors are the eigenvectors
 // of C'C (refined as above), the left ones Y = C W diag(1/sigma).
+#include "f64_ops.cuh"
 #include "ofrr_internal.cuh"
 
 #include <algorithm>
@@ -73,7 +74,7 @@ __global__ void __launch_bounds__(256) k_chol_f64(int n, const double* const* Ms
       if (flag) *flag = 1;
     }
     if constexpr (EXACT) {
-      s_rinv2[k & 1] = S[k + k * n] = sqrt(d);
+      s_rinv2[k & 1] = S[k + k * n] = f64::sqrt(d);
     } else {
       const double r = rsqrt(d);
       S[k + k * n] = d * r;
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(256) k_chol_f64(int n, const double* const* Ms
   __syncthreads();
   for (int k = 0; k < n; ++k) {
     const double rinv = s_rinv2[k & 1];
-    for (int i = k + 1 + tid; i < n; i += nt) S[i + k * n] = EXACT ? S[i + k * n] / rinv : S[i + k * n] * rinv;
+    for (int i = k + 1 + tid; i < n; i += nt) S[i + k * n] = EXACT ? f64::div(S[i + k * n], rinv) : S[i + k * n] * rinv;
     __syncthreads();
     if (warp == nw - 1) {
       if (lane == 0 && k + 1 < n) {
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(128) k_trsm_f64(int n, int nrhs, const double*
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) rd[i] = 1.0 / Ls[i + i * ld];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) rd[i] = f64::rcp(Ls[i + i * ld]);
   __syncthreads();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 4 + w;
