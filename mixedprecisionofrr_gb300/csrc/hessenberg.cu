@@ -23,7 +23,7 @@ template <class TO, class TC>
 __global__ void __launch_bounds__(256) k_hess_col(int64_t m, int n, int i, TO* __restrict__ Q, int64_t ldq,
                                                    int* __restrict__ select, int* __restrict__ perm,
                                                    TO* __restrict__ pivrows, TO* __restrict__ pvals,
-                                                   double* __restrict__ R, ArgMax* __restrict__ partial,
+                                                   double* __restrict__ R, ArgMaxK* __restrict__ partial,
                                                    unsigned int* __restrict__ counter, double select_tol,
                                                    int scale_prev, int* __restrict__ stop, int stage_L,
                                                    TO* __restrict__ snap = nullptr) {
@@ -32,9 +32,10 @@ __global__ void __launch_bounds__(256) k_hess_col(int64_t m, int n, int i, TO* _
   // n entries (aligned: FP32 arithmetic with FP64 storage leaves an odd n at a multiple of four bytes)
   TO* s_x = reinterpret_cast<TO*>(((uintptr_t)(s_r + n) + 15) & ~(uintptr_t)15);
   int* s_sel = reinterpret_cast<int*>(((uintptr_t)(s_x + n) + 15) & ~(uintptr_t)15);  // n entries
-  __shared__ ArgMax red[32];
+  __shared__ ArgMaxK red[32];
   __shared__ bool s_last;
-  __shared__ TC s_pprev;
+  __shared__ TC s_pprev, s_yprev;  // pivot of column i - 1, its reciprocal
+  __shared__ bool s_pf;
 
   const int tid = threadIdx.x;
   // Krylov mode: a breakdown earlier in this cycle turns the rest of the cycle into no-ops
@@ -47,7 +48,12 @@ __global__ void __launch_bounds__(256) k_hess_col(int64_t m, int n, int i, TO* _
     s_sel[j] = sj;
     s_x[j] = sj ? (snap ? snap[j] : Q[(int64_t)perm[j] + (int64_t)i * ldq]) : TO(0);
   }
-  if (tid == 0) s_pprev = (i > 0) ? to_c<TC, TO>(pvals[i - 1]) : TC(0);
+  if (tid == 0) {
+    const TC p = (i > 0) ? to_c<TC, TO>(pvals[i - 1]) : TC(0);
+    s_pprev = p;
+    s_pf = pivot_fast(p);
+    s_yprev = s_pf ? pivot_recip(p) : TC(0);
+  }
   // stage the strictly lower i x i block of pivot rows in shared memory when it fits, so that the
   // sequential substitution below never waits on global memory
   TO* s_L = stage_L ? reinterpret_cast<TO*>(((uintptr_t)(s_sel + n) + 15) & ~(uintptr_t)15) : nullptr;
@@ -81,14 +87,17 @@ __global__ void __launch_bounds__(256) k_hess_col(int64_t m, int n, int i, TO* _
 
   // eliminations on this thread's rows (MGS order), fused scaling of column i-1
   const int prev_sel = (i > 0) ? s_sel[i - 1] : 0;
-  ArgMax a{-1.0, 0x7fffffffffffffffLL};
+  const TC pprev = s_pprev, yprev = s_yprev;
+  const bool pf = s_pf;
+  // (integer keys: an FP64 comparison takes longer than an elimination)
+  ArgMaxK a{-1, 0x7fffffffffffffffLL};
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t row = blockIdx.x * (int64_t)blockDim.x + tid; row < m; row += stride) {
     TO qprev = TO(0);
     if (i > 0) {
       qprev = Q[row + (int64_t)(i - 1) * ldq];
       if (scale_prev) {
-        qprev = prev_sel ? from_c<TO, TC>(div_rn(to_c<TC, TO>(qprev), s_pprev)) : TO(0);
+        qprev = prev_sel ? from_c<TO, TC>(pivot_div(to_c<TC, TO>(qprev), pprev, yprev, pf)) : TO(0);
         Q[row + (int64_t)(i - 1) * ldq] = qprev;
       }
     }
@@ -113,10 +122,10 @@ __global__ void __launch_bounds__(256) k_hess_col(int64_t m, int n, int i, TO* _
       }
     }
     Q[row + (int64_t)i * ldq] = vo;
-    const double av = absd(vo);
-    if (av > a.v) a = ArgMax{av, row};
+    const long long key = amax_key(vo);
+    if (key > a.key) a = ArgMaxK{key, row};
   }
-  ArgMax r = block_argmax(a, red);
+  ArgMaxK r = block_argmaxk(a, red);
   if (tid == 0) {
     partial[blockIdx.x] = r;
     __threadfence();
@@ -128,16 +137,16 @@ __global__ void __launch_bounds__(256) k_hess_col(int64_t m, int n, int i, TO* _
   __threadfence();
 
   // last CTA: global pivot, R(:,i), selection and pivot row
-  ArgMax b{-1.0, 0x7fffffffffffffffLL};
-  const volatile ArgMax* vp = partial;
+  ArgMaxK b{-1, 0x7fffffffffffffffLL};
+  const volatile ArgMaxK* vp = partial;
   for (int t = tid; t < (int)gridDim.x; t += blockDim.x) {
-    ArgMax p;
-    p.v = vp[t].v;
+    ArgMaxK p;
+    p.key = vp[t].key;
     p.i = vp[t].i;
-    b = argmax_pick(b, p);
+    b = argmaxk_pick(b, p);
   }
-  ArgMax f = block_argmax(b, red);
-  const int64_t k = (f.v < 0.0) ? 0 : f.i;
+  ArgMaxK f = block_argmaxk(b, red);
+  const int64_t k = (f.key < 0) ? 0 : f.i;
   const TO pv = __ldcg(reinterpret_cast<const TO*>(Q + k + (int64_t)i * ldq));
   const double tol_o = to_c<double, TO>(from_c<TO, double>(select_tol));
   // kept unless |pivot| < select_tol: a column that is NaN throughout (no row wins the search, row 0
@@ -191,7 +200,7 @@ static int hess_run(ofrr_ctx* ctx, int64_t m, int n, TO* Q, int64_t ldq, double 
   // rows -- a thread's rows are a chain of dependent loads of the earlier columns.  The launches read
   // the next column's pivot-row values from a snapshot, so the grid need not be resident at once.
   int grid = grid_for(m, block, 152 * 16);
-  ArgMax* partial = ws_get<ArgMax>(ctx, grid, &st);
+  ArgMaxK* partial = ws_get<ArgMaxK>(ctx, grid, &st);
   TO* snap = ws_get<TO>(ctx, (size_t)n, &st);
   if (!partial || !snap) return st;
   OFRR_TRY(fill_zero(ctx, R, sizeof(double) * (size_t)n * n));
@@ -248,7 +257,7 @@ static int kry_col(ofrr_ctx* ctx, int64_t m, int nb, int i, TO* V, int64_t ldv, 
   const int grid = grid_for(m, block, 152 * 4);  // resident at once: column i is read from V itself
   int st = OFRR_SUCCESS;
   WsScope scope(ctx);
-  ArgMax* partial = ws_get<ArgMax>(ctx, grid, &st);
+  ArgMaxK* partial = ws_get<ArgMaxK>(ctx, grid, &st);
   if (!partial) return st;
   const int stage = ((size_t)nb * nb * sizeof(TO) <= 96 * 1024) ? 1 : 0;
   size_t smem = (size_t)nb * (sizeof(TC) + sizeof(TO)) + 32 + (size_t)nb * sizeof(int);
@@ -358,7 +367,7 @@ size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 // bytes of scratch for an n-column basis of element size es
 size_t noalloc_bytes(int64_t n, size_t es) {
-  return align256(sizeof(unsigned int)) + align256(sizeof(ArgMax) * kNoAllocGrid) + align256((size_t)n * es) +
+  return align256(sizeof(unsigned int)) + align256(sizeof(ArgMaxK) * kNoAllocGrid) + align256((size_t)n * es) +
          align256((size_t)n * n * es);
 }
 
@@ -366,8 +375,8 @@ template <class TO, class TC>
 int hess_run_noalloc(ofrr_ctx* sctx, unsigned char* scratch, int64_t m, int n, TO* Q, int64_t ldq, double select_tol,
                      double* R, int* select, int* perm) {
   unsigned int* counter = (unsigned int*)scratch;
-  ArgMax* partial = (ArgMax*)(scratch + align256(sizeof(unsigned int)));
-  TO* pvals = (TO*)((unsigned char*)partial + align256(sizeof(ArgMax) * kNoAllocGrid));
+  ArgMaxK* partial = (ArgMaxK*)(scratch + align256(sizeof(unsigned int)));
+  TO* pvals = (TO*)((unsigned char*)partial + align256(sizeof(ArgMaxK) * kNoAllocGrid));
   TO* pivrows = (TO*)((unsigned char*)pvals + align256((size_t)n * sizeof(TO)));
   const int block = 256;
   const int grid = grid_for(m, block, kNoAllocGrid);

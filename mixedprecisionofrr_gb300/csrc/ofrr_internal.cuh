@@ -238,8 +238,8 @@ __device__ __forceinline__ bool pivot_fast(double p) {
 }
 __device__ __forceinline__ bool pivot_fast(float) { return false; }
 __device__ __forceinline__ double pivot_div(double x, double p, double y, bool fast) {
-  const double ax = fabs(x);
-  if (fast && ax >= 0x1p-900 && ax <= 0x1p+900) {
+  // 2^-900 <= |x| < 2^900 by the exponent field: an FP64 comparison takes longer than the products below
+  if (fast && ((unsigned)__double2hiint(x) >> 20 & 0x7ffu) - 123u < 1800u) {
     const double q0 = __dmul_rn(x, y);
     const double r0 = __fma_rn(-p, q0, x);
     const double q1 = __fma_rn(r0, y, q0);

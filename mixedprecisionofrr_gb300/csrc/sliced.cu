@@ -240,6 +240,41 @@ __global__ void __launch_bounds__(T) k_slice_cols(int64_t K, int64_t Kp, int64_t
   }
 }
 
+// Packed digits of short columns (Kp <= 128), one warp per column: the transposed block of a Ritz update has hundreds of
+// thousands of columns of a few dozen entries, where a CTA per column spends its time in barriers (262144 columns of 65:
+// 178 us; this form 141 us).  Lane l takes entries l, l + 32, ..; the zero tail of the column is one byte pattern.
+__global__ void __launch_bounds__(256) k_slice_short(int64_t K, int Kp, int64_t N, const double* __restrict__ X,
+                                                     int64_t ldx, uint8_t* __restrict__ stack, int* __restrict__ expo) {
+  const int lane = threadIdx.x & 31, R = pack_rows(N);
+  for (int64_t n = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); n < N; n += (int64_t)gridDim.x * 8) {
+    const double* x = X + n * ldx;
+    unsigned long long v[4], mx = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = lane + 32 * u;
+      v[u] = (k < K) ? (unsigned long long)__double_as_longlong(x[k]) : 0ull;
+      mx = max(mx, v[u] & 0x7fffffffffffffffull);
+    }
+    for (int o = 16; o > 0; o >>= 1) mx = max(mx, (unsigned long long)__shfl_xor_sync(0xffffffffu, mx, o));
+    const int e = colmax_expo(mx);
+    if (lane == 0) expo[n] = e;
+    uint8_t* col = pack_col(stack, N, Kp, n);
+    const int swz = pack_swz((int)(n % R));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = lane + 32 * u;
+      if (32 * u < K) {
+        if (k < Kp) slice_pack<1>(v + u, e, col, R, swz, k);
+      } else if (32 * u < Kp && lane < 8) {  // four zero entries: digit 0 in every plane
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+          *reinterpret_cast<unsigned*>(col + (size_t)((32 * u >> 6) * S + s) * (R * 64) +
+                                       (((32 * u + 4 * lane) & 63) ^ swz)) = 0x40404040u;
+      }
+    }
+  }
+}
+
 // scalecols (FP64, FAST: reciprocal multiply, pivot exactly 1) fused with the digit split of the
 // scaled column, for columns of at most SCS_T U CL rows: a cluster of CL CTAs per column keeps the
 // column in registers (CTA r holds rows [r SCS_T U, (r + 1) SCS_T U)), finds the pivot (integer
@@ -751,6 +786,14 @@ int sliced_prepare_into(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, in
   out->M = M;
   out->stack = stack;
   out->expo = expo;
+  if constexpr (std::is_same<TD, uint8_t>::value) {
+    if (out->Kp <= 128) {
+      const unsigned grid = (unsigned)std::min<int64_t>((M + 7) / 8, 152 * 32);
+      slice::k_slice_short<<<grid, 256, 0, ctx->stream>>>(K, (int)out->Kp, M, X, ldx, stack, expo);
+      OFRR_LAUNCHED(ctx, "k_slice_short");
+      return OFRR_SUCCESS;
+    }
+  }
   if (out->Kp <= 128) {  // short columns (back-transform coefficients): 64 threads per column
     slice::k_slice_cols<TD, 2, 64><<<(unsigned)std::min<int64_t>(M, 65535), 64, 0, ctx->stream>>>(K, out->Kp, M, X,
                                                                                                 ldx, stack, expo);
