@@ -356,20 +356,24 @@ __device__ void be_colmax(int n, int b, const float* X, float* out, float* redv,
   __syncthreads();
 }
 
+// S and U of the Jacobi method: 16 x 16, row-major, rows 17 apart (a column's 16 lanes on different banks)
+constexpr int BE_LD = BE_B + 1;
+__device__ __forceinline__ int be_jat(int e) { return (e / BE_B) * BE_LD + e % BE_B; }
+
 // Symmetric 16 x 16 Jacobi eigensolver in FP32 on one warp, parallel (round-robin) ordering: every round
 // rotates 8 disjoint pairs at once, lane m < 8 computing pair m's rotation, lane k < 16 applying all 8 to
 // row / column k.  S (ld BE_B) is overwritten, U holds the eigenvectors (columns), w the eigenvalues.
 // Rows and columns past b must be zero off the diagonal (their diagonal sorts them last).
 __device__ void be_jacobi(float* S, float* U, float* w, float* cs, int* pq) {
   const int lane = threadIdx.x & 31;
-  for (int e = lane; e < BE_B * BE_B; e += 32) U[e] = ((e / BE_B) == (e % BE_B)) ? 1.f : 0.f;
+  for (int e = lane; e < BE_B * BE_B; e += 32) U[be_jat(e)] = ((e / BE_B) == (e % BE_B)) ? 1.f : 0.f;
   __syncwarp();
   for (int sweep = 0; sweep < 20; ++sweep) {
     float off = 0.f, dn = 0.f;
     for (int e = lane; e < BE_B * BE_B; e += 32) {
-      const float v = S[e] * S[e];
+      const float x = S[be_jat(e)], v = x * x;
       if (e / BE_B != e % BE_B) off += v;
-      else dn += (fabsf(S[e]) < 1e29f) ? v : 0.f;
+      else dn += (fabsf(x) < 1e29f) ? v : 0.f;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -383,10 +387,10 @@ __device__ void be_jacobi(float* S, float* U, float* w, float* cs, int* pq) {
         const int a = (lane == 0) ? 0 : 1 + (lane - 1 + round) % (BE_B - 1);
         const int bb = 1 + (BE_B - 2 - lane + round) % (BE_B - 1);
         const int p = min(a, bb), q = max(a, bb);
-        const float apq = S[p * BE_B + q];
+        const float apq = S[p * BE_LD + q];
         float c = 1.f, sn = 0.f;
         if (fabsf(apq) > 1e-30f) {
-          const float theta = (S[q * BE_B + q] - S[p * BE_B + p]) / (2.f * apq);
+          const float theta = (S[q * BE_LD + q] - S[p * BE_LD + p]) / (2.f * apq);
           const float t = copysignf(1.f, theta) / (fabsf(theta) + sqrtf(fmaf(theta, theta, 1.f)));
           c = rsqrtf(fmaf(t, t, 1.f));
           sn = t * c;
@@ -397,32 +401,42 @@ __device__ void be_jacobi(float* S, float* U, float* w, float* cs, int* pq) {
         pq[2 * lane + 1] = q;
       }
       __syncwarp();
-      if (lane < BE_B) {  // columns: S = S J, U = U J (row `lane`)
+      {  // columns: S = S J (row `lane`, lanes 0 .. 15) beside U = U J (lanes 16 .. 31)
+        float* X = ((lane & 16) ? U : S) + (lane & 15) * BE_LD;
+        float xp[BE_B / 2], xq[BE_B / 2];
+#pragma unroll
         for (int m = 0; m < BE_B / 2; ++m) {
-          const int p = pq[2 * m], q = pq[2 * m + 1];
+          xp[m] = X[pq[2 * m]];
+          xq[m] = X[pq[2 * m + 1]];
+        }
+#pragma unroll
+        for (int m = 0; m < BE_B / 2; ++m) {
           const float c = cs[2 * m], sn = cs[2 * m + 1];
-          const float sp = S[lane * BE_B + p], sq = S[lane * BE_B + q];
-          S[lane * BE_B + p] = c * sp - sn * sq;
-          S[lane * BE_B + q] = sn * sp + c * sq;
-          const float up = U[lane * BE_B + p], uq = U[lane * BE_B + q];
-          U[lane * BE_B + p] = c * up - sn * uq;
-          U[lane * BE_B + q] = sn * up + c * uq;
+          const float sp = xp[m], sq = xq[m];
+          X[pq[2 * m]] = c * sp - sn * sq;
+          X[pq[2 * m + 1]] = sn * sp + c * sq;
         }
       }
       __syncwarp();
       if (lane < BE_B) {  // rows: S = J' S (column `lane`)
+        float xp[BE_B / 2], xq[BE_B / 2];
+#pragma unroll
         for (int m = 0; m < BE_B / 2; ++m) {
-          const int p = pq[2 * m], q = pq[2 * m + 1];
+          xp[m] = S[pq[2 * m] * BE_LD + lane];
+          xq[m] = S[pq[2 * m + 1] * BE_LD + lane];
+        }
+#pragma unroll
+        for (int m = 0; m < BE_B / 2; ++m) {
           const float c = cs[2 * m], sn = cs[2 * m + 1];
-          const float sp = S[p * BE_B + lane], sq = S[q * BE_B + lane];
-          S[p * BE_B + lane] = c * sp - sn * sq;
-          S[q * BE_B + lane] = sn * sp + c * sq;
+          const float sp = xp[m], sq = xq[m];
+          S[pq[2 * m] * BE_LD + lane] = c * sp - sn * sq;
+          S[pq[2 * m + 1] * BE_LD + lane] = sn * sp + c * sq;
         }
       }
       __syncwarp();
     }
   }
-  if (lane < BE_B) w[lane] = S[lane * BE_B + lane];
+  if (lane < BE_B) w[lane] = S[lane * BE_LD + lane];
   __syncwarp();
 }
 
@@ -860,7 +874,7 @@ __global__ void __launch_bounds__(BE_T, 1) k_batch_si(BatchDev d) {
   __shared__ int s_perm[BE_B];
   __shared__ int s_sel[BE_B];
   __shared__ double s_G[BE_B * BE_B], s_M[BE_B * BE_B], s_L[BE_B * BE_B], s_T[BE_B * BE_B];
-  __shared__ float s_S[BE_B * BE_B], s_U[BE_B * BE_B], s_w[BE_B];
+  __shared__ float s_S[BE_B * BE_LD], s_U[BE_B * BE_LD], s_w[BE_B];
   __shared__ float s_Z[BE_B * BE_B];
   __shared__ float s_lam[BE_B];
   __shared__ float s_cs[BE_B];
@@ -1037,17 +1051,17 @@ __global__ void __launch_bounds__(BE_T, 1) k_batch_si(BatchDev d) {
             for (int k = 0; k < i; ++k) v -= s_L[i * BE_B + k] * y[k];
             y[i] = v / s_L[i * BE_B + i];
           }
-          for (int i = 0; i < b; ++i) s_S[r * BE_B + i] = (float)y[i];
+          for (int i = 0; i < b; ++i) s_S[r * BE_LD + i] = (float)y[i];
         }
         __syncwarp();
         for (int e = lane; e < BE_B * BE_B; e += 32) {  // symmetrise; pad rows / columns past b
           const int i = e / BE_B, j = e % BE_B;
           if (i >= b || j >= b) {
-            s_S[e] = (i == j) ? -1e30f : 0.f;
+            s_S[be_jat(e)] = (i == j) ? -1e30f : 0.f;
           } else if (i < j) {
-            const float a = 0.5f * (s_S[i * BE_B + j] + s_S[j * BE_B + i]);
-            s_S[i * BE_B + j] = a;
-            s_S[j * BE_B + i] = a;
+            const float a = 0.5f * (s_S[i * BE_LD + j] + s_S[j * BE_LD + i]);
+            s_S[i * BE_LD + j] = a;
+            s_S[j * BE_LD + i] = a;
           }
         }
         __syncwarp();
@@ -1074,7 +1088,7 @@ __global__ void __launch_bounds__(BE_T, 1) k_batch_si(BatchDev d) {
           const int src = s_redi[c];
           double y[BE_B];
           for (int i = b - 1; i >= 0; --i) {
-            double v = (double)s_U[i * BE_B + src];
+            double v = (double)s_U[i * BE_LD + src];
             for (int k = i + 1; k < b; ++k) v -= s_L[k * BE_B + i] * y[k];
             y[i] = v / s_L[i * BE_B + i];
           }
