@@ -71,83 +71,23 @@ __device__ void kry_extend(int64_t k, int i, int nb, const T* V, int64_t ldv, co
     Lrows[(int64_t)i * nb + j] = l;
   }
   if (tid == 0) Lrows[(int64_t)i * nb + i] = TE(1);
-  // Row i of L^-1 (the first half of the warps) beside w_{i+1} at the pivot rows (the second half).  Both are chains
-  // of dependent loads or FP64 operations, so loads run ahead in batches; the whole chip waits for this CTA.  Step 60
-  // of the FP64 solver on a 7-point grid: 10 us, against 37 us with one pivot row per warp at a time (four dependent
-  // loads each) and loads issued as the sums consumed them.
-  const int lane = tid & 31, wid = tid >> 5, half = nthr >> 1;
-  const bool more = i + 1 < nb;
-  if (tid == 0) s_long = 0;
-  __syncthreads();
-  if (tid < half) {
-    for (int j = tid; j - lane < i; j += half) {
-      const int m0 = j - lane;  // the warp walks its rows together; rows above j do not count
-      TE s = TE(0), a[8], nx[8];
-      auto load = [&](int m, TE* v) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = (m + u >= j && m + u < i) ? Linv[(int64_t)(m + u) * nb + j] : TE(0);
-      };
-      load(m0, a);
-      for (int m = m0; m < i; m += 8) {
-        load(m + 8, nx);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          if (m + u >= j && m + u < i) s = fma(s_L[m + u], a[u], s);
-          a[u] = nx[u];
-        }
-      }
-      if (j < i) Linv[(int64_t)i * nb + j] = -s;
+  if constexpr (sizeof(TE) == 4) {
+    // FP32 chains are short, and the batches below would take the step's loads their registers (FP16 basis, step 40 of
+    // 2 million rows: 122 us, 131 us with them)
+    __syncthreads();
+    for (int j = tid; j < i; j += nthr) {
+      TE s = TE(0);
+      for (int m = j; m < i; ++m) s = fma(s_L[m], Linv[(int64_t)m * nb + j], s);
+      Linv[(int64_t)i * nb + j] = -s;
     }
     if (tid == 0) Linv[(int64_t)i * nb + i] = TE(1);
-  } else if (more) {
-    // rows of at most 8 nonzeros: 8 lanes per row, RB rows in flight; the sum is kry_warp_sum's tree without its zeros
-    constexpr int RB = 4;
-    const int groups = half >> 3, g = (tid - half) >> 3, sub = lane & 7;
-    for (int base = 0; base <= i; base += groups * RB) {
-      int64_t r[RB];
-      int32_t p0[RB], len[RB], col[RB];
-      TE v[RB], acc[RB];
-#pragma unroll
-      for (int u = 0; u < RB; ++u) {
-        const int j = base + g + groups * u;
-        r[u] = (j < i) ? (int64_t)perm[j] : k;
-      }
-#pragma unroll
-      for (int u = 0; u < RB; ++u) {
-        p0[u] = indptr[r[u]];
-        len[u] = indptr[r[u] + 1] - p0[u];
-      }
-#pragma unroll
-      for (int u = 0; u < RB; ++u) {
-        const bool in = sub < len[u] && len[u] <= 8;
-        col[u] = in ? indices[p0[u] + sub] : -1;
-        v[u] = in ? vals[p0[u] + sub] : TE(0);
-      }
-#pragma unroll
-      for (int u = 0; u < RB; ++u) acc[u] = (col[u] >= 0) ? __ldcg(S + col[u]) : TE(0);
-#pragma unroll
-      for (int u = 0; u < RB; ++u) acc[u] = (col[u] >= 0) ? fma(v[u], to_c<TE, T>(kry_q<T, TE>(acc[u], pinv)), TE(0)) : TE(0);
-#pragma unroll
-      for (int off = 4; off > 0; off >>= 1)
-#pragma unroll
-        for (int u = 0; u < RB; ++u) acc[u] += __shfl_down_sync(0xffffffffu, acc[u], off, 8);
-#pragma unroll
-      for (int u = 0; u < RB; ++u) {
-        const int j = base + g + groups * u;
-        if (sub == 0 && j <= i) {
-          if (len[u] <= 8) s_w[j] = acc[u];
-          else s_long = 1;
-        }
-      }
-    }
-  }
-  if (!more) return;
-  __syncthreads();
-  if (s_long) {  // longer rows: one warp per row, lanes over its nonzeros
-    for (int j = wid; j <= i; j += nthr >> 5) {
+    if (i + 1 >= nb) return;
+    __syncthreads();
+    // w_{i+1} at the pivot rows: one warp per row, lanes over its nonzeros
+    const int lane = tid & 31, wid = tid >> 5, nw = nthr >> 5;
+    for (int j = wid; j <= i; j += nw) {
       const int64_t r = (j == i) ? k : (int64_t)perm[j];
       const int32_t p0 = indptr[r], p1 = indptr[r + 1];
-      if (p1 - p0 <= 8) continue;
       TE acc = TE(0);
       for (int32_t p = p0 + lane; p < p1; p += 32) {
         const int32_t col = indices[p];
@@ -157,24 +97,117 @@ __device__ void kry_extend(int64_t k, int i, int nb, const T* V, int64_t ldv, co
       if (lane == 0) s_w[j] = acc;
     }
     __syncthreads();
-  }
-  for (int j = tid; j <= i; j += nthr) {
-    const TE* row = Linv + (int64_t)j * nb;
-    TE c = TE(0), a[8], nx[8];
-    auto load = [&](int m, TE* v) {
+    for (int j = tid; j <= i; j += nthr) {
+      TE c = TE(0);
+      for (int m = 0; m <= j; ++m) c = fma(Linv[(int64_t)j * nb + m], s_w[m], c);
+      coef[j] = c;
+    }
+  } else {
+    // Row i of L^-1 (the first half of the warps) beside w_{i+1} at the pivot rows (the second half).  Both are chains
+    // of dependent loads or FP64 operations, so loads run ahead in batches; the whole chip waits for this CTA.  Step 60
+    // of the FP64 solver on a 7-point grid: 10 us, against 37 us with one pivot row per warp at a time (four dependent
+    // loads each) and loads issued as the sums consumed them.
+    const int lane = tid & 31, wid = tid >> 5, half = nthr >> 1;
+    const bool more = i + 1 < nb;
+    if (tid == 0) s_long = 0;
+    __syncthreads();
+    if (tid < half) {
+      for (int j = tid; j - lane < i; j += half) {
+        const int m0 = j - lane;  // the warp walks its rows together; rows above j do not count
+        TE s = TE(0), a[8], nx[8];
+        auto load = [&](int m, TE* v) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = (m + u <= j) ? row[m + u] : TE(0);
-    };
-    load(0, a);
-    for (int m = 0; m <= j; m += 8) {
-      load(m + 8, nx);
+          for (int u = 0; u < 8; ++u) v[u] = (m + u >= j && m + u < i) ? Linv[(int64_t)(m + u) * nb + j] : TE(0);
+        };
+        load(m0, a);
+        for (int m = m0; m < i; m += 8) {
+          load(m + 8, nx);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (m + u <= j) c = fma(a[u], s_w[m + u], c);
-        a[u] = nx[u];
+          for (int u = 0; u < 8; ++u) {
+            if (m + u >= j && m + u < i) s = fma(s_L[m + u], a[u], s);
+            a[u] = nx[u];
+          }
+        }
+        if (j < i) Linv[(int64_t)i * nb + j] = -s;
+      }
+      if (tid == 0) Linv[(int64_t)i * nb + i] = TE(1);
+    } else if (more) {
+      // rows of at most 8 nonzeros: 8 lanes per row, RB rows in flight; the sum is kry_warp_sum's tree without its zeros
+      constexpr int RB = 4;
+      const int groups = half >> 3, g = (tid - half) >> 3, sub = lane & 7;
+      for (int base = 0; base <= i; base += groups * RB) {
+        int64_t r[RB];
+        int32_t p0[RB], len[RB], col[RB];
+        TE v[RB], acc[RB];
+#pragma unroll
+        for (int u = 0; u < RB; ++u) {
+          const int j = base + g + groups * u;
+          r[u] = (j < i) ? (int64_t)perm[j] : k;
+        }
+#pragma unroll
+        for (int u = 0; u < RB; ++u) {
+          p0[u] = indptr[r[u]];
+          len[u] = indptr[r[u] + 1] - p0[u];
+        }
+#pragma unroll
+        for (int u = 0; u < RB; ++u) {
+          const bool in = sub < len[u] && len[u] <= 8;
+          col[u] = in ? indices[p0[u] + sub] : -1;
+          v[u] = in ? vals[p0[u] + sub] : TE(0);
+        }
+#pragma unroll
+        for (int u = 0; u < RB; ++u) acc[u] = (col[u] >= 0) ? __ldcg(S + col[u]) : TE(0);
+#pragma unroll
+        for (int u = 0; u < RB; ++u) acc[u] = (col[u] >= 0) ? fma(v[u], to_c<TE, T>(kry_q<T, TE>(acc[u], pinv)), TE(0)) : TE(0);
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1)
+#pragma unroll
+          for (int u = 0; u < RB; ++u) acc[u] += __shfl_down_sync(0xffffffffu, acc[u], off, 8);
+#pragma unroll
+        for (int u = 0; u < RB; ++u) {
+          const int j = base + g + groups * u;
+          if (sub == 0 && j <= i) {
+            if (len[u] <= 8) s_w[j] = acc[u];
+            else s_long = 1;
+          }
+        }
       }
     }
-    coef[j] = c;
+    if (!more) return;
+    __syncthreads();
+    if (s_long) {  // longer rows: one warp per row, lanes over its nonzeros
+      for (int j = wid; j <= i; j += nthr >> 5) {
+        const int64_t r = (j == i) ? k : (int64_t)perm[j];
+        const int32_t p0 = indptr[r], p1 = indptr[r + 1];
+        if (p1 - p0 <= 8) continue;
+        TE acc = TE(0);
+        for (int32_t p = p0 + lane; p < p1; p += 32) {
+          const int32_t col = indices[p];
+          acc = fma(vals[p], to_c<TE, T>(kry_q<T, TE>(__ldcg(S + col), pinv)), acc);
+        }
+        acc = kry_warp_sum(acc);
+        if (lane == 0) s_w[j] = acc;
+      }
+      __syncthreads();
+    }
+    for (int j = tid; j <= i; j += nthr) {
+      const TE* row = Linv + (int64_t)j * nb;
+      TE c = TE(0), a[8], nx[8];
+      auto load = [&](int m, TE* v) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = (m + u <= j) ? row[m + u] : TE(0);
+      };
+      load(0, a);
+      for (int m = 0; m <= j; m += 8) {
+        load(m + 8, nx);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (m + u <= j) c = fma(a[u], s_w[m + u], c);
+          a[u] = nx[u];
+        }
+      }
+      coef[j] = c;
+    }
   }
 }
 
