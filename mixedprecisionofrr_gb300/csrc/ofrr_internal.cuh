@@ -233,9 +233,8 @@ __device__ __forceinline__ double div_rn(double a, double b) { return f64::div(a
 // [2^-900, 2^900] (where an intermediate could underflow or overflow) use the division itself.
 __device__ __forceinline__ double pivot_recip(double p) { return f64::rcp(p); }
 __device__ __forceinline__ float pivot_recip(float p) { return __frcp_rn(p); }
-__device__ __forceinline__ bool pivot_fast(double p) {
-  const double a = fabs(p);
-  return a >= 0x1p-450 && a <= 0x1p+450;
+__device__ __forceinline__ bool pivot_fast(double p) {  // 2^-450 <= |p| < 2^450, by the exponent field
+  return ((unsigned)__double2hiint(p) >> 20 & 0x7ffu) - 573u < 900u;
 }
 __device__ __forceinline__ bool pivot_fast(float) { return false; }
 __device__ __forceinline__ double pivot_div(double x, double p, double y, bool fast) {
