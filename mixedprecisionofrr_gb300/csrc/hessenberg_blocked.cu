@@ -414,10 +414,10 @@ __global__ void __launch_bounds__(HB_T) k_hess_inblock(int64_t m, int n, int c0,
 
 // ---- panels of FP32-compute bases: one row per thread in registers ---------------------------------
 // For at most HR_T rows per CTA (8192 rows on sixteen) and FP32 arithmetic a thread keeps its row's values of up to
-// NV = 16 or 32 panel columns in registers.  The values shift down by one with every column (column t is always v[0]; the shift is part of the
-// elimination), so the loop over columns stays rolled with constant register indices, and a finished column goes
-// straight to Q.  The exchange is k_hess_inblock's: candidates pushed by st.async into every CTA's receive slots, two
-// buffers, completing on the receiver's mbarrier; the warp that owns the CTA's candidate sends it.
+// NV = 16 or 32 panel columns in registers.  The values shift down by one with every column (column t is always v[0];
+// the shift is part of the elimination), so the loop over columns stays rolled with constant register indices, and a
+// finished column goes straight to Q.  The exchange is k_hess_inblock's: candidates pushed by st.async into every CTA's
+// receive slots, two buffers, completing on the receiver's mbarrier; the warp that owns the CTA's candidate sends it.
 // What bounds it: the chain of a column, about 3,200 cycles at 8192 rows and 32 columns (waiting for the candidates
 // 940, choosing 330, dividing 440, eliminating 860, argmax and sending 600).  The shared-memory form above takes 3,500
 // with blocks of 16 columns, each with two further launches.  Measured, half storage, 8192 rows: 16 columns 31 -> 25
@@ -460,7 +460,9 @@ __global__ void __launch_bounds__(HR_T) k_hess_reg(int64_t m, int n, int c0, int
   __shared__ Cand s_recv[2][HB_CL_MAX];
   __shared__ Cand s_send;
   __shared__ __align__(8) uint64_t s_bar[2];
-  __shared__ uint2 s_red[HR_T / 32];  // per warp: key, thread
+  // per warp: key, thread.  Two buffers: warps read column t's entries after its barrier, and nothing holds a fast warp
+  // from storing column t + 1's before a slow one has read; column t + 2's come after t + 1's barrier, so after the reads.
+  __shared__ uint2 s_red[2][HR_T / 32];
   __shared__ int s_abort;
   const bool have = tid < nr;
   const int nwarps = (nr + 31) / 32;  // warps with rows (warp 0 always takes part)
@@ -491,9 +493,9 @@ __global__ void __launch_bounds__(HR_T) k_hess_reg(int64_t m, int n, int c0, int
     const unsigned key = !have ? 0u : bits > 0x7f800000u ? 1u : bits + 2u;
     const unsigned mk = __reduce_max_sync(0xffffffffu, key);
     const unsigned who = __ballot_sync(0xffffffffu, key == mk);
-    if (lane == 0) s_red[wid] = make_uint2(mk, wid * 32 + __ffs(who) - 1);  // lowest row of the warp's maxima
+    if (lane == 0) s_red[t & 1][wid] = make_uint2(mk, wid * 32 + __ffs(who) - 1);  // lowest row of the warp's maxima
     __syncthreads();
-    const uint2 e = (lane < HR_T / 32) ? s_red[lane] : make_uint2(0u, 0u);
+    const uint2 e = (lane < HR_T / 32) ? s_red[t & 1][lane] : make_uint2(0u, 0u);
     const unsigned bk = __reduce_max_sync(0xffffffffu, e.x);
     const unsigned bw = __ballot_sync(0xffffffffu, lane < HR_T / 32 && e.x == bk);
     const int win = __shfl_sync(0xffffffffu, (int)e.y, __ffs(bw) - 1);  // the lowest warp's
