@@ -196,7 +196,7 @@ __device__ bool be_matmul_r(int n, int ld, const TA* __restrict__ A, const float
   bool bad = false;
   if (tid == 0)
     for (int c = 0; c < min(nck, BE_NS) && !bad; ++c) bad = !refill(c);
-  __syncwarp();
+  bad = __any_sync(0xffffffffu, bad);  // a warp leaves the loop below as a whole
   float acc[4 * R][4];
 #pragma unroll
   for (int r = 0; r < 4 * R; ++r)
@@ -210,7 +210,7 @@ __device__ bool be_matmul_r(int n, int ld, const TA* __restrict__ A, const float
   uint32_t st = base % BE_NS, ph = (base / BE_NS) & 1;
   int k0 = 0;
   for (int c = 0; c < nck && !bad; ++c) {
-    if (!tc::mbar_wait(&rg.full[st], ph, rg.err, 22)) {
+    if (!tc::mbar_wait_warp(&rg.full[st], ph, rg.err, 22)) {
       bad = true;
       break;
     }
@@ -247,7 +247,7 @@ __device__ bool be_matmul_r(int n, int ld, const TA* __restrict__ A, const float
       be_arrive(&rg.empty[st]);
       if ((c % (BE_T / 32)) == warp && c >= 1 && c - 1 + BE_NS < nck) bad = !refill(c - 1 + BE_NS);
     }
-    __syncwarp();
+    bad = __any_sync(0xffffffffu, bad);
     if (++st == BE_NS) {
       st = 0;
       ph ^= 1;

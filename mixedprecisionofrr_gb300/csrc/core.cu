@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "ofrr_internal.cuh"
+#include "tcgen05.cuh"
 
 #include <cmath>
 #include <cstdlib>
@@ -587,29 +588,23 @@ int residual_columns(ofrr_ctx* ctx, int64_t m, int64_t n, const double* AX, int6
   return OFRR_SUCCESS;
 }
 
-// One CTA waits on an mbarrier that nothing arrives on; the bounded wait gives up after timeout_ns,
-// records the timeout in the status word of the tcgen05 pipelines and returns.
-__global__ void k_bounded_wait_probe(unsigned long long timeout_ns, int* err) {
-  __shared__ __align__(8) unsigned long long bar;
-  const unsigned baddr = (unsigned)__cvta_generic_to_shared(&bar);
-  if (threadIdx.x == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(baddr) : "memory");
+// One CTA waits on an mbarrier that nothing arrives on; the bounded wait gives up after timeout_ns, records the timeout
+// in the status word of the tcgen05 pipelines and returns.  The two warps wait as the pipelines' warps do, in a loop with
+// warp-wide and CTA-wide operations behind the wait.  Their lanes have limits of timeout_ns to twice that, and one lane of
+// each sees its phase complete: all lanes of a warp must leave together all the same.
+__global__ void __launch_bounds__(64) k_bounded_wait_probe(unsigned long long timeout_ns, int* err) {
+  __shared__ __align__(8) uint64_t bar;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) tc::mbar_init(&bar, 1);
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  unsigned long long t0, t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  while (true) {
-    unsigned ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok)
-                 : "r"(baddr)
-                 : "memory");
-    if (ok) return;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    if (t - t0 > timeout_ns) {
-      atomicCAS(err, 0, 99);
-      return;
-    }
+  bool bad = false;
+  for (int i = 0; i < 2 && !bad; ++i) {
+    // one lane of each warp looks at the phase before the first, which is complete: it does not time out
+    const uint32_t parity = (lane == 5) ? 1u : 0u;
+    if (!tc::mbar_wait_warp(&bar, parity, err, 99, timeout_ns + timeout_ns * lane / 32)) bad = true;
+    __syncwarp();
   }
+  __syncthreads_or(bad);
 }
 
 }  // namespace ofrr
@@ -738,7 +733,7 @@ void* ofrr_ctx_get_stream(ofrr_ctx* ctx) { return ctx ? (void*)ctx->stream : nul
 int ofrr_debug_bounded_wait(ofrr_ctx* ctx, int64_t timeout_ns) {
   if (!ctx) return OFRR_ERR_INVALID_ARGUMENT;
   const long long t = timeout_ns < 1000 ? 1000 : (timeout_ns > 1000000000LL ? 1000000000LL : timeout_ns);
-  ofrr::k_bounded_wait_probe<<<1, 32, 0, ctx->stream>>>((unsigned long long)t, ctx->dev_flags + kFlagTcWait);
+  ofrr::k_bounded_wait_probe<<<1, 64, 0, ctx->stream>>>((unsigned long long)t, ctx->dev_flags + kFlagTcWait);
   OFRR_LAUNCHED(ctx, "k_bounded_wait_probe");
   return OFRR_SUCCESS;
 }

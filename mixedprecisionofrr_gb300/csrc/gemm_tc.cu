@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const uint32_t a_base = smem_u32(sA) >> 4, b_base = smem_u32(sB) >> 4;
     uint32_t st = 0, ph = 0;
     for (int i = 0; i < nkb; ++i) {
-      if (!mbar_wait(&full[st], ph, err, 13)) break;
+      if (!mbar_wait_warp(&full[st], ph, err, 13)) break;
       fence_after();
       const uint32_t a0 = a_base + st * (Smem<BN>::A_BYTES >> 4), b0 = b_base + st * (Smem<BN>::B_BYTES >> 4);
       if (leader) {
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   } else {
     // epilogue warps 2..5 -> TMEM lane quarter (warp % 4)
     const int q = warp & 3;
-    const bool ok = mbar_wait(accum, 0, err, 14);
+    const bool ok = mbar_wait_warp(accum, 0, err, 14);
     fence_after();
     const int row = m0 + 32 * q + lane;
     const bool split = (partial != nullptr);

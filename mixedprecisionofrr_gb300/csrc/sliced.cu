@@ -572,11 +572,11 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
     bool ok = true;
     for (int i = 0; i < nkb && ok; ++i) {
       const uint32_t bs = (uint32_t)i % SL_BSLOTS;
-      if (!mbar_wait(&b_full[bs], (i / SL_BSLOTS) & 1, err, 25)) break;
+      if (!mbar_wait_warp(&b_full[bs], (i / SL_BSLOTS) & 1, err, 25)) break;
       const uint32_t b0 = b_base + bs * (S * SL_BTILE >> 4);
 #pragma unroll
       for (int s = 0; s < S; ++s) {
-        if (ok && !mbar_wait(&a_full[as], aph, err, 26)) ok = false;
+        if (ok && !mbar_wait_warp(&a_full[as], aph, err, 26)) ok = false;
         fence_after();
         // A digit s against the B digits 0..LMAX-s at once: the slot's B tiles are adjacent rows of
         // one K-major operand and the level accumulators s..LMAX adjacent TMEM columns, so one MMA
@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
           __syncwarp();
           if (held >= 0 && lane == 0) mbar_arrive(&r_empty[held % SL_RSLOTS]);
           held = i;
-          if (!__all_sync(0xffffffffu, mbar_wait(&r_full[i % SL_RSLOTS], (i / SL_RSLOTS) & 1, err, 28))) break;
+          if (!mbar_wait_warp(&r_full[i % SL_RSLOTS], (i / SL_RSLOTS) & 1, err, 28)) break;
           raw = sR + (i % SL_RSLOTS) * S * SL_RPLANE + row * 64;
         }
         uint32_t o[SL_ACOLS];
@@ -647,9 +647,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
             }
           }
         }
-        if (use >= SL_ASLOTS &&
-            !__all_sync(0xffffffffu, mbar_wait(&a_empty[as], ((use / SL_ASLOTS) + 1) & 1, err, 29)))
-          break;
+        if (use >= SL_ASLOTS && !mbar_wait_warp(&a_empty[as], ((use / SL_ASLOTS) + 1) & 1, err, 29)) break;
         fence_after();
         tmem_st32(tmem + lanes + (uint32_t)(SL_ABASE + as * SL_ACOLS), o);
         fence_before();
@@ -663,10 +661,9 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
       const int row = m0 + 32 * q + lane;
       const int erow = (row < M) ? ea[row] : 0;
       const int ecol = (lane < 16 && n0 + c + lane < N) ? eb[n0 + c + lane] : 0;
-      const bool ok = mbar_wait(accum, 0, err, 27);
+      const bool ok = mbar_wait_warp(accum, 0, err, 27);
       fence_after();
       float v[LMAX + 1][16];
-      __syncwarp();
 #pragma unroll
       for (int L = 0; L <= LMAX; ++L)
         tmem_ld16_async(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(L * SBN + c), v[L]);

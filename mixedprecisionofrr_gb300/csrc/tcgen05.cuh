@@ -37,16 +37,24 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 // bounded wait (about 2 s); records code in *err and returns false on timeout
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, int code) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, int code,
+                                          uint64_t limit_ns = 2000000000ull) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer();
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (globaltimer() - t0 > 2000000000ull) {
+    if (globaltimer() - t0 > limit_ns) {
       atomicCAS(err, 0, code);
       return false;
     }
   }
+}
+// mbar_wait by a whole warp, with one answer for its lanes, which leave it converged.  (Every lane polls and reads the
+// timer by itself: near the limit one may give up while another sees the phase complete, and lanes that part there would
+// wait for each other at the next warp-wide operation and at the CTA's barrier, for ever.)
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* err, int code,
+                                               uint64_t limit_ns = 2000000000ull) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code, limit_ns));
 }
 
 __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* bar, void* dst, int x, int y) {
