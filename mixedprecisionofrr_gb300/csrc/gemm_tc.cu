@@ -204,13 +204,11 @@ __global__ void __launch_bounds__(THREADS, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
   if (csize > 1) {
-    __syncwarp();
     cluster_arrive();
     cluster_wait();
     if (csize == 2) cluster_reduce<BN, 2>(base, m0, n0, M, N, D, ldd);
     else if (csize == 4) cluster_reduce<BN, 4>(base, m0, n0, M, N, D, ldd);
     else cluster_reduce<BN, 8>(base, m0, n0, M, N, D, ldd);
-    __syncwarp();
     cluster_arrive();  // no CTA leaves while its tile may still be read
     cluster_wait();
   }

@@ -291,6 +291,7 @@ __global__ void __launch_bounds__(HB_T) k_hess_inblock(int64_t m, int n, int c0,
 #pragma unroll
     for (int t = 0; t < HB_B; ++t) s_blk[(size_t)t * RR + lr] = v[t];
   }
+  __syncwarp();
   cluster.sync();  // every CTA's barriers are armed before the first push
 
   // Warp argmax `a` of every warp -> this CTA's candidate for column t, sent to all CTAs.  Called by
@@ -409,6 +410,7 @@ __global__ void __launch_bounds__(HB_T) k_hess_inblock(int64_t m, int n, int c0,
     for (int t = 0; t < HB_B; ++t)
       if (t < nb) Q[r0 + lr + (int64_t)(c0 + t) * ldq] = s_blk[(size_t)t * RR + lr];
   }
+  __syncwarp();
   cluster.sync();  // every push into this CTA has landed before any CTA leaves
 }
 
@@ -485,6 +487,7 @@ __global__ void __launch_bounds__(HR_T) k_hess_reg(int64_t m, int n, int c0, int
   const int dst = lane & (HB_CL_MAX - 1);
   const uint32_t d_recv = cluster_addr(&s_recv[0][rank], dst < ncl ? dst : 0);
   const uint32_t d_bar = cluster_addr(&s_bar[0], dst < ncl ? dst : 0);
+  __syncwarp();
   cluster.sync();  // every CTA's barriers are armed before the first push
 
   // the CTA's candidate for column t (v[0]) to every CTA
@@ -579,6 +582,7 @@ __global__ void __launch_bounds__(HR_T) k_hess_reg(int64_t m, int n, int c0, int
     publish(t + 1, nrem - 1);  // its barrier also makes s_abort visible to every thread
     if (s_abort) break;        // a peer stopped answering: leave (the status word is set)
   }
+  __syncwarp();
   cluster.sync();  // every push into this CTA has landed before any CTA leaves
 }
 

@@ -370,11 +370,20 @@ __device__ __forceinline__ ArgMaxK block_argmaxk(ArgMaxK a, ArgMaxK* smem) {
 // Per-column kernels over a cluster of CL CTAs of SCS_T threads (scale and split, split-K combine and
 // scale): CTA r of a column's cluster holds rows [r SCS_T U, (r + 1) SCS_T U), U per thread.
 constexpr int SCS_T = 1024;
+// The cluster barrier, by whole warps: the aligned forms need every lane at the same instruction, and lanes come here from
+// loops of uneven length and stores that only some of them make.
 __device__ __forceinline__ void cluster_arrive_relaxed() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ unsigned cluster_rank() {
   unsigned r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

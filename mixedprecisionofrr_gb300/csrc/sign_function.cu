@@ -234,7 +234,6 @@ __global__ void __launch_bounds__(32 * kSignWarps, 1) k_sign_cluster(int n, doub
         s_mu = exp(-ld / n);
       }
     }
-    __syncwarp();
     cluster_arrive();
     cluster_wait();
     const double mu = (it < 4) ? s_mu : 1.0;
@@ -272,7 +271,6 @@ __global__ void __launch_bounds__(32 * kSignWarps, 1) k_sign_cluster(int n, doub
       asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster_map(&s_all[w][me], (unsigned)(tid >> 1))), "d"(t)
                    : "memory");
     }
-    __syncwarp();
     cluster_arrive();
     cluster_wait();
     double sn = 0.0, sd = 0.0;

@@ -52,8 +52,15 @@ __device__ __forceinline__ bool ns_neg(double x) {  // x < 0 (false for -0 and N
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
 }
-__device__ __forceinline__ void ns_bar_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
-__device__ __forceinline__ void ns_bar_arrive(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+// (by whole warps, which come here from loops of uneven length)
+__device__ __forceinline__ void ns_bar_sync(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+}
+__device__ __forceinline__ void ns_bar_arrive(int id) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
+}
 
 // One warp, and with VEC a second one for the Schur vectors.  C: n x n (FP64, ld ldc).  Outputs: wr, wi (n), X (n x n, FP64, ld n): eigenvectors of C
 // (real parts, unit norm), unsorted; *flag = 1 when the QR iteration did not converge.
@@ -120,7 +127,6 @@ __global__ void __launch_bounds__(VEC ? 64 : 32) k_nonsym_eig(int nn, const doub
   auto send = [&](int kind, int k, T x, T y, T z, T q, T r) {
     ns_bar_sync(3 + (sent & 1));
     if (lane == 0) s_op[sent & 1] = Op{kind, k, x, y, z, q, r};
-    __syncwarp();
     ns_bar_arrive(1 + (sent & 1));
     ++sent;
   };
