@@ -29,12 +29,18 @@ namespace ofrr {
 // triangle of the trailing block updated with one warp per column (no index division).
 // EXACT: square root and divisions instead of the reciprocal square root (the reference-semantics solver,
 // whose results depend on the last bits of its operands: see smalleig.cu).
+// The pointers travel with the launch: a table copied from the host's stack would be read again, long gone, each time a
+// captured graph runs.
+struct CholBatch {
+  const double* M[2];
+  double* L[2];
+};
 template <bool EXACT>
-__global__ void __launch_bounds__(256) k_chol_f64(int n, const double* const* Ms, int ldm, double tau,
-                                                  double* const* Ls, int* flag) {
+__global__ void __launch_bounds__(256) k_chol_f64(int n, const __grid_constant__ CholBatch batch, int ldm, double tau,
+                                                  int* flag) {
   extern __shared__ double S[];
-  const double* M = Ms[blockIdx.x];
-  double* L = Ls[blockIdx.x];
+  const double* M = batch.M[blockIdx.x];
+  double* L = batch.L[blockIdx.x];
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   __shared__ double s_maxd, s_rinv2[2];
   // stage M + tau I (lower triangle) with 16 loads per thread in flight (the kernel is latency-bound)
@@ -658,15 +664,11 @@ static int trsm(ofrr_ctx* ctx, int n, int nrhs, const double* L, const double* B
 template <bool EXACT = false>
 static int chol(ofrr_ctx* ctx, int n, int count, const double* const* Ms_host, int ldm, double tau,
                 double* const* Ls_host) {
-  int st = OFRR_SUCCESS;
-  const double** Md = ws_get<const double*>(ctx, 4, &st);
-  if (!Md) return st;
-  double** Ld = (double**)(Md + 2);
-  const void* hp[4] = {Ms_host[0], count > 1 ? Ms_host[1] : Ms_host[0], Ls_host[0], count > 1 ? Ls_host[1] : Ls_host[0]};
-  OFRR_CUDA(cudaMemcpyAsync(Md, hp, sizeof(hp), cudaMemcpyHostToDevice, ctx->stream));
+  if (count < 1 || count > 2) return OFRR_ERR_INTERNAL;
+  const CholBatch batch{{Ms_host[0], Ms_host[count - 1]}, {Ls_host[0], Ls_host[count - 1]}};
   const size_t smem = (size_t)n * n * sizeof(double);
   OFRR_TRY(allow_smem(k_chol_f64<EXACT>));
-  k_chol_f64<EXACT><<<count, 256, smem, ctx->stream>>>(n, Md, ldm, tau, Ld, ctx->dev_flags + 1);
+  k_chol_f64<EXACT><<<count, 256, smem, ctx->stream>>>(n, batch, ldm, tau, ctx->dev_flags + 1);
   OFRR_LAUNCHED(ctx, "k_chol_f64");
   return OFRR_SUCCESS;
 }
