@@ -654,9 +654,10 @@ __device__ void br_rayleigh_ritz(int k2, int kb, double* G, double* M, double* L
         const double apq = Cm[p * ld + q];
         double c = 1.0, sn = 0.0;
         if (fabs(apq) > 1e-300) {
-          const double theta = f64::div(Cm[q * ld + q] - Cm[p * ld + p], 2.0 * apq);
-          const double tt = copysign(f64::rcp(fabs(theta) + f64::sqrt(fma(theta, theta, 1.0))), theta);
-          c = f64::rcp(f64::sqrt(fma(tt, tt, 1.0)));
+          // (short forms undecided between neighbours: a rotation needs c^2 + sn^2 = 1 to a few units)
+          const double theta = f64::div<false>(Cm[q * ld + q] - Cm[p * ld + p], 2.0 * apq);
+          const double tt = copysign(f64::rcp<false>(fabs(theta) + f64::sqrt<false>(fma(theta, theta, 1.0))), theta);
+          c = f64::rcp<false>(f64::sqrt<false>(fma(tt, tt, 1.0)));
           sn = tt * c;
         }
         c2[2 * lane] = c;

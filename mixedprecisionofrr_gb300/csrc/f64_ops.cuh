@@ -1,16 +1,20 @@
-// Short FP64 reciprocal, quotient and square root for latency-bound chains.
+// Short FP64 reciprocal, quotient and square root for latency-bound chains: the correctly rounded values.
 //
-// An FP64 instruction takes this part's pipe 64 cycles, whatever it computes, so a division (~560 cycles) or square root
-// (~630) is mostly its own refinement steps.  Here the reciprocal (or reciprocal root) of the 53-bit significand is
+// An FP64 instruction takes this part's pipe 64 cycles, whatever it computes, so a division (~565 cycles) or square root
+// (~600) is mostly its own refinement steps.  Here the reciprocal (or reciprocal root) of the 53-bit significand is
 // formed to about 45 bits with FP32 pairs and integer operations alone, which run beside the FP64 pipe at full rate, and
-// only the last step is FP64: Newton's for the reciprocal (two instructions), the exact-residual correction for
+// only the last step is FP64: Newton's for the reciprocal (two instructions), the residual correction for
 // quotient and root (three) [P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor,
 // IBM J. Res. Dev. 34 (1990)].  Before its rounding a result is within 2^-86 of the exact one, so it is the correctly
-// rounded value unless that lies within 2^-86 of a rounding boundary.  Whole families of operands do: divisors just
-// below a power of two (1 / (2 - j 2^-52) is a boundary plus j^2 2^-107), and roots of operands beside a power of four.
-// These, operands outside a wide exponent range, and zero, subnormal, infinite and NaN ones take the plain operation;
-// roots of 1 + d for d < 2^-36, which a converging rotation asks for, the series 1 + (d / 2 - d^2 / 8).
-// About 240, 310 and 310 cycles.
+// rounded value or its neighbour: exact values come as close as 2^-107 to a rounding boundary (1.5 / (1 + 2^-52), or any
+// a 2^54 = b m + r with m odd and r small; one random operand in 2^33).  The remainder, formed exactly in 64-bit integers
+// (it is below 2^55, so the low words of the products suffice), decides between the two; no quotient or root lies on a
+// boundary itself.  Without that decision (RN = false) the error is below 1/2 + 2^-33 units in the last place.
+// Operands outside a wide exponent range, and zero, subnormal, infinite and NaN ones take the plain operation; so do
+// divisors and radicands just below a power of two (the seed's binade, and the root's, change there); roots of 1 + d for
+// d < 2^-36, which a converging rotation asks for, the series 1 + (d / 2 - d^2 / 8).
+// In a lone warp, cycles: reciprocal 310, quotient 400, root 455 (240, 325 and 380 with RN = false) against 350, 565 and
+// 600 of the plain operations.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -64,16 +68,39 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
   return join(y0, y0 * (r * fmaf(0.375f, r, 0.5f)), 1022 - ((e - (odd ? 1 : 0)) >> 1), 0u);
 }
 
+// the significand as an integer in [2^52, 2^53)
+__device__ __forceinline__ unsigned long long sig(double x) {
+  return ((unsigned long long)__double_as_longlong(x) & 0xfffffffffffffull) | (1ull << 52);
+}
+// the low 64 bits of s 2^k, 32 <= k < 64
+__device__ __forceinline__ unsigned long long shl_low(unsigned long long s, int k) {
+  return (unsigned long long)((unsigned)s << (k - 32)) << 32;
+}
+// x for 0 <= u <= top; else its neighbour nearer zero (u < 0) or further from it
+__device__ __forceinline__ double settle(double x, unsigned long long u, unsigned long long top) {
+  const int n = (int)((long long)u >> 63) | 1;  // -1 or 1
+  return __longlong_as_double(__double_as_longlong(x) + (u > top ? n : 0));
+}
+
+template <bool RN = true>
 __device__ __forceinline__ double rcp(double x) {
   if (plain(x) || below_pow2(x)) return __drcp_rn(x);
-  const double y = rcp_seed(x);
-  return __fma_rn(y, __fma_rn(-y, x, 1.0), y);
+  const double s = rcp_seed(x), y = __fma_rn(s, __fma_rn(-s, x, 1.0), s);
+  if (!RN) return y;
+  // the remainder 2^104 (or 2^105) - X Y in [-X / 2, X / 2]
+  const unsigned long long X = sig(x);
+  return settle(y, X + (0ull - 2 * X) * sig(y), 2 * X);
 }
+template <bool RN = true>
 __device__ __forceinline__ double div(double a, double b) {
   if (plain(a) || plain(b) || below_pow2(b) || (unsigned)(expo(a) - expo(b) + 800) > 1600u) return __ddiv_rn(a, b);
-  const double y = rcp_seed(b), q = __dmul_rn(a, y);
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
+  const double y = rcp_seed(b), q0 = __dmul_rn(a, y), q = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+  if (!RN) return q;
+  // the remainder A 2^k - B Q in [-B / 2, B / 2]; Q has 53 bits with k = 52 for A >= B, else with k = 53
+  const unsigned long long A = sig(a), B = sig(b);
+  return settle(q, (shl_low(A, A < B ? 54 : 53) + B) + (0ull - 2 * B) * sig(q), 2 * B);
 }
+template <bool RN = true>
 __device__ __forceinline__ double sqrt(double x) {
   if (plain(x) || below_pow2(x) || __double2hiint(x) < 0) return __dsqrt_rn(x);
   if ((__double2hiint(x) & 0x1fffff) == 0x100000 && (unsigned)__double2loint(x) < 65536u) {  // 4^k (1 + d), d < 2^-36
@@ -84,7 +111,11 @@ __device__ __forceinline__ double sqrt(double x) {
   }
   const double y = rsqrt_seed(x), g = __dmul_rn(x, y);
   const double hy = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));  // y / 2
-  return __fma_rn(__fma_rn(-g, g, x), hy, g);
+  const double r = __fma_rn(__fma_rn(-g, g, x), hy, g);
+  if (!RN) return r;
+  // the remainder X 2^k - G^2 (k = 52, or 53 for an odd exponent) in [1 - G, G], as (G +- 1/2)^2 - G^2 = +-G + 1/4
+  const unsigned long long G = sig(r), K = shl_low(sig(x), 53 - (expo(x) & 1)) - 1;
+  return settle(r, K + (1 - G) * G, 2 * G - 1);
 }
 
 }  // namespace f64

@@ -225,11 +225,11 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ double div_rn(double a, double b) { return f64::div(a, b); }
 
-// x / p, correctly rounded, for many x and one p (a pivot, a column maximum), given y = RN(1/p).  In FP64 (a 1/64-rate pipe on GB300) the
-// correctly rounded quotient comes from one multiply and four FMAs: q0 = RN(x y), one correction
-// q1 = RN(q0 + RN(x - p q0) y) makes q1 faithful, and by Markstein's theorem (P. Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990) the
-// second correction RN(q1 + (x - p q1) y), with x - p q1 exact, is RN(x / p).  Operands outside
+// x / p, correctly rounded, for many x and one p (a pivot, a column maximum), given y = RN(1/p) from pivot_recip.  In FP64
+// (a 1/64-rate pipe on GB300) the correctly rounded quotient comes from one multiply and four FMAs: q0 = RN(x y), one
+// correction q1 = RN(q0 + RN(x - p q0) y) makes q1 faithful, and by Markstein's theorem (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), which needs the rounded
+// reciprocal, the second correction RN(q1 + (x - p q1) y), with x - p q1 exact, is RN(x / p).  Operands outside
 // [2^-900, 2^900] (where an intermediate could underflow or overflow) use the division itself.
 __device__ __forceinline__ double pivot_recip(double p) { return f64::rcp(p); }
 __device__ __forceinline__ float pivot_recip(float p) { return __frcp_rn(p); }

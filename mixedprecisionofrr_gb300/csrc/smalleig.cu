@@ -35,11 +35,13 @@ constexpr int kGeigClusterMaxN = 144;  // Cholesky, substitutions and L beside 3
 
 // The rotation of sym.Schur2 (t the root of smaller magnitude of t^2 + 2 tau t - 1 = 0, t = 1 for tau = 0).
 // The chain's divisions and square roots (560 and 630 cycles each as plain operations) were the largest part of a
-// round, 3260 cycles; in their short forms (f64_ops.cuh, the same values) it takes half of that.  Taking the angle in
-// FP32 and normalising (c, s) in FP64 would shorten it as much, but on the SVD
-// pencil [[0, K], [K', 0]] of a block U ~ A V the matrix K is triangular up to rounding, equal diagonal entries
+// round, 3260 cycles; in their short forms (f64_ops.cuh) it takes half of that.  They stay undecided between neighbours
+// (1/2 + 2^-33 units in the last place instead of 1/2; another value than the plain operation's once in 2^33 random ones):
+// a rotation needs c^2 + s^2 = 1 to a few units, and the five decisions take 400 cycles of a round's 6,000 (4 % of a
+// 64-order solve).  Taking the angle in FP32 and normalising (c, s) in FP64 would shorten the chain as much, but on the
+// SVD pencil [[0, K], [K', 0]] of a block U ~ A V the matrix K is triangular up to rounding, equal diagonal entries
 // meet entries of rounding size, and which of the two roots is taken (the sign of the vectors) then hangs on the
-// last bits: the quotients keep every result what the one-CTA form gives, bit for bit.
+// last bits: the quotients keep results what the one-CTA form gives.
 __device__ __forceinline__ bool jac_nonzero(double x) {  // an FP64 compare costs ~100 cycles
   return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) != 0;
 }
@@ -47,9 +49,9 @@ __device__ __forceinline__ void jac_rotation(double app, double aqq, double apq,
   *c = 1.0;
   *s = 0.0;
   if (!jac_nonzero(apq)) return;
-  const double tau = f64::div(aqq - app, 2.0 * apq);
-  const double t = f64::rcp(fabs(tau) + f64::sqrt(__fma_rn(tau, tau, 1.0)));
-  *c = f64::rcp(f64::sqrt(__fma_rn(t, t, 1.0)));
+  const double tau = f64::div<false>(aqq - app, 2.0 * apq);
+  const double t = f64::rcp<false>(fabs(tau) + f64::sqrt<false>(__fma_rn(tau, tau, 1.0)));
+  *c = f64::rcp<false>(f64::sqrt<false>(__fma_rn(t, t, 1.0)));
   const double sa = t * *c;
   *s = (__double2hiint(tau) < 0 && jac_nonzero(tau)) ? -sa : sa;
 }
