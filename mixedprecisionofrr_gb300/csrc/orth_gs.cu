@@ -9,11 +9,11 @@
 //   t = norm2(v); while t >= orth_tol and t < reorth_tol normv: normv = t, another pass with
 //   R(j,i) = po(pc(R(j,i)) + pc(r_j)), t = norm2(v)
 //   t < select_tol -> dropped; else q_i = po(pc(v) / pc(t)), R(i,i) = t.
-// Bases in FP64 throughout are built in one cooperative launch (k_gs_coop).  With a narrower storage type the
-// column loop runs: dots and norms are grid reductions in the compute type (per-CTA partial sums, the last CTA
-// adds them in a fixed order: deterministic); the updates are row-parallel and apply the j terms in order with
-// one rounding to the output type per term, as the MATLAB code does; the while-loop decisions need t on the
-// host, one synchronisation per column and pass.
+// Bases in FP64 throughout are built in one cooperative launch (k_gs_coop).  With a narrower storage type, and for
+// MGS without effective re-orthogonalisation, the column loop runs: dots and norms are grid reductions in the
+// compute type (per-CTA partial sums, the last CTA adds them in a fixed order: deterministic); the updates are
+// row-parallel and apply the j terms in order with one rounding to the output type per term, as the MATLAB code
+// does; the while-loop decisions need t on the host, one synchronisation per column and pass.
 // Q keeps the input's column positions (dropped columns zero) with select flags, like the Hessenberg
 // basis, so the solvers compact both the same way.
 #include <cmath>
@@ -578,8 +578,14 @@ int gs_basis_impl(ofrr_ctx* ctx, bool classical, ofrr_dtype tin, ofrr_dtype tout
   const double s_t = round_to(tout, stol), o_t = round_to(tout, std::isnan(orth_tol) ? e : orth_tol),
                r_t = round_to(tout, std::isnan(reorth_tol) ? 1.0 / std::sqrt(2.0) : reorth_tol);
   // FP64 throughout: one cooperative launch.  With a narrower storage type every term of an update is rounded
-  // to it and the next dot sees that rounding, so those bases keep the column loop's order of operations.
-  if (tout == OFRR_F64 && tc == OFRR_F64) {
+  // to it and the next dot sees that rounding, so those bases keep the column loop's order of operations.  So does
+  // MGS without re-orthogonalisation: its one pass takes out what a dot against the already updated vector sees, the
+  // inverse compact form only what the first dots saw, and of columns dependent to working precision (a Hilbert block
+  // of 1000 x 64) 62 stay above select_tol = eps where the sequential pass leaves 47.  With re-orthogonalisation both
+  // end at the same residuals, up to rounding: it is effective when a column that loses half its norm is projected
+  // again, down to the norms that are dropped.
+  const bool again = r_t >= 0.5 && o_t <= std::max(s_t, e);
+  if (tout == OFRR_F64 && tc == OFRR_F64 && (classical || again)) {
     bool done = false;
     OFRR_TRY(gs_coop(ctx, classical, m, n, (const double*)Ain, ldin, (double*)Q, ldq, s_t, o_t, r_t, R_dev,
                      select_dev, &done));
