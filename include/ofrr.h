@@ -487,6 +487,10 @@ int ofrr_ctx_trim(ofrr_ctx* ctx);
  * usable.  No fault, trap or unbounded wait is involved. */
 int ofrr_debug_bounded_wait(ofrr_ctx* ctx, int64_t timeout_ns);
 
+/* Tests what calls do when their workspace runs out: an allocation that would take the context's workspace in use above
+ * `bytes` fails with OFRR_ERR_OUT_OF_MEMORY, as one that the device refuses does; negative: no limit. */
+int ofrr_debug_ws_limit(ofrr_ctx* ctx, int64_t bytes);
+
 /* Self-test of the short FP64 operations of the latency-bound kernels: out[i] = 1 / a[i] (op 0), a[i] / b[i] (1),
  * sqrt(a[i]) (2); device arrays of n. */
 int ofrr_debug_f64_ops(ofrr_ctx* ctx, int op, int64_t n, const double* a, const double* b, double* out);

@@ -142,6 +142,7 @@ SIGNATURES = {
                                     C.POINTER(_I64), C.POINTER(_DP), C.POINTER(_DP), C.POINTER(ofrr_info), _IP]),
     "ofrr_ctx_trim": (C.c_int, [_P]),
     "ofrr_debug_bounded_wait": (C.c_int, [_P, _I64]),
+    "ofrr_debug_ws_limit": (C.c_int, [_P, _I64]),
     "ofrr_debug_f64_ops": (C.c_int, [_P, C.c_int, _I64, _P, _P, _P]),
     "ofrr_debug_scale_slice": (C.c_int, [_P, C.c_int, _I64, _I64, _I64, _P, _I64, _P, _I64, _P, _I64, _P, _P]),
     "ofrr_gs_basis": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, C.c_int, _I64, _I64, _P, _I64, _P, _I64, _D, _D, _D,

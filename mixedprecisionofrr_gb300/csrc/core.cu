@@ -73,6 +73,14 @@ void* ws_alloc(ofrr_ctx* ctx, size_t bytes, int* status) {
   const size_t align = 256;
   bytes = (bytes + align - 1) / align * align;
   if (bytes == 0) bytes = align;
+  if (ctx->ws_limit != SIZE_MAX) {
+    size_t used = ctx->cur_off + bytes;
+    for (size_t i = 0; i < ctx->cur_chunk && i < ctx->chunks.size(); ++i) used += ctx->chunks[i].size;
+    if (used > ctx->ws_limit) {
+      *status = OFRR_ERR_OUT_OF_MEMORY;
+      return nullptr;
+    }
+  }
   while (true) {
     if (ctx->cur_chunk < ctx->chunks.size()) {
       Chunk& c = ctx->chunks[ctx->cur_chunk];
@@ -735,6 +743,12 @@ int ofrr_debug_bounded_wait(ofrr_ctx* ctx, int64_t timeout_ns) {
   const long long t = timeout_ns < 1000 ? 1000 : (timeout_ns > 1000000000LL ? 1000000000LL : timeout_ns);
   ofrr::k_bounded_wait_probe<<<1, 64, 0, ctx->stream>>>((unsigned long long)t, ctx->dev_flags + kFlagTcWait);
   OFRR_LAUNCHED(ctx, "k_bounded_wait_probe");
+  return OFRR_SUCCESS;
+}
+
+int ofrr_debug_ws_limit(ofrr_ctx* ctx, int64_t bytes) {
+  if (!ctx) return OFRR_ERR_INVALID_ARGUMENT;
+  ctx->ws_limit = bytes < 0 ? SIZE_MAX : (size_t)bytes;
   return OFRR_SUCCESS;
 }
 

@@ -84,6 +84,7 @@ struct ofrr_ctx {
   bool emulate_f64 = false;        // FP64 TN products through exact BF16 slices on the tensor cores
   bool power_f8 = false;           // 16-bit power steps through E4M3 copies (the FP8 variant)
   size_t pinned_size = 0;
+  size_t ws_limit = SIZE_MAX;      // workspace bytes in use at most (ofrr_debug_ws_limit)
   ofrr_ctx* aux = nullptr;         // second stream + workspace for independent work run beside this one
   ofrr::Tracer* tracer = nullptr;  // per-solve phase events and the JSON-lines sink (trace.cu), or null
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

@@ -443,7 +443,7 @@ int gs_coop(ofrr_ctx* ctx, bool classical, int64_t m, int64_t n, const double* A
   P.partial = ws_get<double>(ctx, (size_t)G * (n + 1), &st);
   P.total = ws_get<double>(ctx, (size_t)n + 1, &st);
   P.ctr = ws_get<unsigned>(ctx, 2, &st);
-  if (!P.partial || !P.total || !P.ctr) return st;
+  if (!P.partial || !P.total || !P.ctr) return st;  // the column loop needs more (152 n sums and a column of m)
   P.m = m;
   P.n = (int)n;
   P.lda = lda;
