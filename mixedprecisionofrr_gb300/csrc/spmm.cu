@@ -205,7 +205,10 @@ __global__ void k_csrt_fill(int64_t nrows, const int32_t* __restrict__ indptr, c
   }
 }
 
-// every nonzero to its rank in its column, with the value copies present (null: absent)
+// every nonzero to its rank in its column, with the value copies present (null: absent).  A column of k nonzeros costs
+// k^2 reads, all its nonzeros at once and each warp the same addresses: with one dense column in a sparse matrix the whole
+// transposed product takes 0.80 ms at k = 2000, 5.9 ms at 16,000 and 453 ms at 10^6 (17.1 and 1025 ms at the first two
+// with one thread's insertion sort per column), most of it the product's own serial row.
 __global__ void k_csrt_place(int64_t nrows, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
                              const int32_t* __restrict__ colptr, const int32_t* __restrict__ rows,
                              int32_t* __restrict__ rowidx, const double* __restrict__ vd, double* __restrict__ td,
