@@ -649,7 +649,7 @@ static int hess_reg_launch(ofrr_ctx* ctx, int ncl, int64_t m, int n, int c0, int
   return OFRR_SUCCESS;
 }
 
-// FP32-compute bases of at most HR_T rows per CTA of the cluster: panels of up to 64 columns
+// FP32-compute bases of at most HR_T rows per CTA of the cluster: panels of up to 32 columns
 template <class TO>
 static int hess_run_reg(ofrr_ctx* ctx, int ncl, int64_t m, int n, TO* Q, int64_t ldq, double select_tol, double* R,
                         int* select, int* perm) {

@@ -783,18 +783,16 @@ int sliced_prepare_into(ofrr_ctx* ctx, int64_t K, int64_t M, const double* X, in
   out->M = M;
   out->stack = stack;
   out->expo = expo;
-  if constexpr (std::is_same<TD, uint8_t>::value) {
-    if (out->Kp <= 128) {
+  if (out->Kp <= 128) {
+    if constexpr (std::is_same<TD, uint8_t>::value) {
       const unsigned grid = (unsigned)std::min<int64_t>((M + 7) / 8, 152 * 32);
       slice::k_slice_short<<<grid, 256, 0, ctx->stream>>>(K, (int)out->Kp, M, X, ldx, stack, expo);
       OFRR_LAUNCHED(ctx, "k_slice_short");
-      return OFRR_SUCCESS;
+    } else {  // short columns (back-transform coefficients): 64 threads per column
+      slice::k_slice_cols<TD, 2, 64><<<(unsigned)std::min<int64_t>(M, 65535), 64, 0, ctx->stream>>>(K, out->Kp, M, X,
+                                                                                                  ldx, stack, expo);
+      OFRR_LAUNCHED(ctx, "k_slice_cols");
     }
-  }
-  if (out->Kp <= 128) {  // short columns (back-transform coefficients): 64 threads per column
-    slice::k_slice_cols<TD, 2, 64><<<(unsigned)std::min<int64_t>(M, 65535), 64, 0, ctx->stream>>>(K, out->Kp, M, X,
-                                                                                                ldx, stack, expo);
-    OFRR_LAUNCHED(ctx, "k_slice_cols");
     return OFRR_SUCCESS;
   }
   if (out->Kp <= slice::SC_T * 16) {
