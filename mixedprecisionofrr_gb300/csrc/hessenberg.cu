@@ -236,8 +236,8 @@ int hessenberg_impl(ofrr_ctx* ctx, ofrr_dtype tin, ofrr_dtype tout, ofrr_dtype t
   if (A == Q && (tin != tout || lda != ldq)) return OFRR_ERR_INVALID_ARGUMENT;
   if (A != Q) OFRR_TRY(cast_impl(ctx, tin, tout, m, n, A, lda, Q, ldq));
   WsScope scope(ctx);
-  // one cooperative launch (hessenberg_coop.cu) when the whole basis fits the SMs' shared memory, the blocked
-  // cluster schedule (hessenberg_blocked.cu) when a block of columns does, else per column
+  // one cooperative launch (hessenberg_coop.cu) when the whole basis fits the SMs' shared memory and is large enough for
+  // it, the blocked cluster schedule (hessenberg_blocked.cu) when a block of columns fits, else per column
   bool done = false;
   OFRR_TRY(hess_run_coop(ctx, tout, tc, m, n, Q, ldq, select_tol, R_dev, select_dev, perm_dev, fast, &done));
   if (done) return OFRR_SUCCESS;

@@ -32,12 +32,7 @@ constexpr int HC_MAXN = 256;
 constexpr int HC_REP = 4;  // copies of a candidate's values: the whole grid reads the winner's at once
 constexpr size_t HC_SMEM_MAX = 200 * 1024;
 
-template <bool FAST> __device__ __forceinline__ double hc_elim(double v, double r, double q) {
-  return FAST ? __fma_rn(-r, q, v) : __dsub_rn(v, __dmul_rn(r, q));
-}
-template <bool FAST> __device__ __forceinline__ float hc_elim(float v, float r, float q) {
-  return __fsub_rn(v, __fmul_rn(r, q));
-}
+template <class TC> __device__ __forceinline__ TC hc_elim(TC v, TC r, TC q) { return sub_rn(v, mul_rn(r, q)); }
 
 struct HcPair {
   unsigned long long a, b;
@@ -100,7 +95,7 @@ struct HcWait {
 };
 
 // words: [2][G][2] keys and rows; vals: [2][HC_REP][G][n] tagged values (copies: the whole grid reads one row)
-template <class TO, class TC, bool FAST>
+template <class TO, class TC>
 __global__ void __launch_bounds__(HC_T) k_hess_coop(int64_t m, int n, int rows, TO* __restrict__ Q, int64_t ldq,
                                                     int* __restrict__ select, int* __restrict__ perm,
                                                     double* __restrict__ R, double select_tol,
@@ -148,7 +143,7 @@ __global__ void __launch_bounds__(HC_T) k_hess_coop(int64_t m, int n, int rows, 
       for (int u = t + lane; u < n; u += 32) {
         TO v = X[(size_t)u * RR + lr];
         if (elim_prev && u > t) {
-          v = from_c<TO, TC>(hc_elim<FAST>(to_c<TC, TO>(v), s_pr[u], q));
+          v = from_c<TO, TC>(hc_elim(to_c<TC, TO>(v), s_pr[u], q));
           X[(size_t)u * RR + lr] = v;
         }
 #pragma unroll
@@ -253,14 +248,12 @@ __global__ void __launch_bounds__(HC_T) k_hess_coop(int64_t m, int n, int rows, 
       TO nv = has_next ? X[(size_t)(t + 1) * RR + r] : TO(0);
       if (keep) {
         const TC q = to_c<TC, TO>(X[(size_t)t * RR + r]);
-        // FAST: x * RN(1/p) (within an ulp of x / p), the pivot itself exactly 1
-        const TC sq = (FAST && pf) ? ((row0 + r == k) ? TC(1) : mul_rn(q, y)) : pivot_div(q, pc, y, pf);
-        const TO so = from_c<TO, TC>(sq);
+        const TO so = from_c<TO, TC>(pivot_div(q, pc, y, pf));
         X[(size_t)t * RR + r] = so;
         const TC qs = to_c<TC, TO>(so);
         s_q[r] = qs;
         if (has_next) {
-          nv = from_c<TO, TC>(hc_elim<FAST>(to_c<TC, TO>(nv), s_pr[t + 1], qs));
+          nv = from_c<TO, TC>(hc_elim(to_c<TC, TO>(nv), s_pr[t + 1], qs));
           X[(size_t)(t + 1) * RR + r] = nv;
         }
       } else {
@@ -283,7 +276,7 @@ __global__ void __launch_bounds__(HC_T) k_hess_coop(int64_t m, int n, int rows, 
         const int u = t + 2 + it / rg, r = (it % rg) * 32 + lane;
         if (r < nr && r != lc) {
           TO* e = X + (size_t)u * RR + r;
-          *e = from_c<TO, TC>(hc_elim<FAST>(to_c<TC, TO>(*e), s_pr[u], s_q[r]));
+          *e = from_c<TO, TC>(hc_elim(to_c<TC, TO>(*e), s_pr[u], s_q[r]));
         }
       }
     }
@@ -295,7 +288,7 @@ __global__ void __launch_bounds__(HC_T) k_hess_coop(int64_t m, int n, int rows, 
 
 bool hess_blocked_fits(int64_t m, int64_t n, size_t es);
 
-template <class TO, class TC, bool FAST>
+template <class TO, class TC>
 static int hess_coop_t(ofrr_ctx* ctx, int64_t m, int n, int rows, int G, size_t smem, TO* Q, int64_t ldq,
                        double select_tol, double* R, int* select, int* perm, bool* done) {
   WsScope scope(ctx);
@@ -309,7 +302,7 @@ static int hess_coop_t(ofrr_ctx* ctx, int64_t m, int n, int rows, int G, size_t 
   OFRR_TRY(fill_zero(ctx, R, sizeof(double) * (size_t)n * n));
   int* err = ctx->dev_flags + kFlagHessWait;
   void* args[] = {&m, &n, &rows, &Q, &ldq, &select, &perm, &R, &select_tol, &words, &vals, &err};
-  const void* f = (const void*)k_hess_coop<TO, TC, FAST>;
+  const void* f = (const void*)k_hess_coop<TO, TC>;
   OFRR_TRY(allow_dynamic_smem(f));
   const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3((unsigned)G), dim3(HC_T), args, smem, ctx->stream);
   if (e == cudaErrorCooperativeLaunchTooLarge) {  // the grid cannot be resident at once on this device
@@ -322,38 +315,44 @@ static int hess_coop_t(ofrr_ctx* ctx, int64_t m, int n, int rows, int G, size_t 
   return OFRR_SUCCESS;
 }
 
-// One cooperative launch when the CTAs' rows of all columns fit their shared memory and the cluster schedules
-// are not the better ones; *done = false otherwise.  Measured, whole ofrr_hessenberg calls, us (this / blocked cluster
-// or panel / per column):
-//   FP64 exact:  8192 x 64 466 / 665, 600 x 64 408 / 444, 30000 x 64 697 / - / 1988, 4160 x 16 222 / 194 (one block: no
-//     coefficients, no block update)
-//   FP32 compute: half 8192 x 64 358 / 262, 20000 x 96 572 / 581, 100000 x 40 378 / - / 518
-//   FP64 with FMA (fast), 8192 x 64 and 2048 x 64 side by side inside a solve: 317 / 312
-// Hence: FP64 exact beyond one block of columns; FP32 arithmetic and the fast form beyond 8192 rows.  Heights that
-// the blocked schedule does not hold have always been built in the exact arithmetic, whatever `fast`: it stays so.
+// One cooperative launch when the CTAs' rows of all columns fit their shared memory and the blocked schedules (cluster
+// blocks, register panels) are not the better ones; *done = false otherwise.  Measured, whole ofrr_hessenberg calls, us,
+// this / blocked:
+//   FP64            n = 16     32         64         96         128
+//     600 rows      176 / 158  244 / 236  383 / 416  559 / 671  762 / 1017
+//     2048          188 / 160  244 / 233  401 / 429  570 / 684  787 / 1028
+//     4160          199 / 172  260 / 270  403 / 500  592 / 824  811 / 1228
+//     8192          202 / 196  257 / 321  433 / 619  657 / 1016 940 / 1542
+//     12000         193 / 223  256 / 375  459 / 756  725 / 1270 1057 / 1882
+//     25000         197 / 312  288 / 571  574 / 1240 984 / 2002 1515 / 2972
+//   FP32 arithmetic, half storage (single: within 5 %)
+//     8192          198 / 140  218 / 170  328 / 248  460 / 353  625 / 475
+//     16384         179 / 147  215 / 211  352 / 355  526 / 513  735 / 716
+//     20000         172 / 156  221 / 227  363 / 382  551 / 579  791 / 795
+//     40000         171 / 176  231 / 268  425 / 469  700 / 706  1069 / 988
+//     80000         179 / 220  271 / 359  574 / 670  1023 / 1036 1632 / 1441
+// Hence: FP64 but for few columns (16 up to 8192 rows, 32 up to 4096); FP32 arithmetic above 32768 rows and up to 80
+// columns (between 16384 and 32768 the two are within 5 %, and in a solve, where two bases are built side by side, the
+// blocked one is ahead).  Heights that the blocked schedules do not hold: 30000 x 64 in FP64 697 against 1988 us per
+// column, 100000 x 40 half 378 against 518.
+// The FMA arithmetic of the refinement phases (`fast`) stays with the blocked schedule: it runs two bases side by side,
+// and a grid over all SMs waits for the other's cluster (mixed SVD 16384 x 4000, 40 columns: 36.4 ms with this schedule,
+// 35.0 ms blocked).  Heights that the blocked schedule does not hold are built in the exact arithmetic, whatever `fast`.
 int hess_run_coop(ofrr_ctx* ctx, ofrr_dtype tout, ofrr_dtype tc, int64_t m, int64_t n, void* Q, int64_t ldq,
                   double select_tol, double* R, int* select, int* perm, bool fast, bool* done) {
   *done = false;
   if (n > HC_MAXN || m < 1 || m >= 0xffffffffLL || getenv("OFRR_HESS_PER_COLUMN")) return OFRR_SUCCESS;
-  fast = fast && tc == OFRR_F64;
-  const bool blocked = hess_blocked_fits(m, n, dtype_size(tout));
-  if (fast && !blocked) fast = false;
-  if (blocked && ((tc == OFRR_F32 || fast) ? m <= 8192 : n <= 16)) return OFRR_SUCCESS;
+  if (hess_blocked_fits(m, n, dtype_size(tout))) {
+    const bool here = (tc == OFRR_F32) ? m > 32768 && n <= 80 : !fast && n > (m <= 4096 ? 32 : m <= 8192 ? 16 : 0);
+    if (!here) return OFRR_SUCCESS;
+  }
   const int G = (int)std::min<int64_t>(HC_MAXG, (m + 31) / 32);
   const int64_t rows = (m + G - 1) / G;
   const size_t es = dtype_size(tout), cs = dtype_size(tc);
   const size_t smem = (((size_t)n * (rows | 1) * es + 15) & ~(size_t)15) + ((rows | 1) + n) * cs;
   if (smem > HC_SMEM_MAX) return OFRR_SUCCESS;
-  if (fast) {
-    OFRR_DISPATCH_STORAGE(tout, TO, {
-      OFRR_TRY((hess_coop_t<TO, double, true>(ctx, m, (int)n, (int)rows, G, smem, (TO*)Q, ldq, select_tol, R, select,
-                                              perm, done)));
-    });
-    return OFRR_SUCCESS;
-  }
   OFRR_DISPATCH_STORAGE(tout, TO, OFRR_DISPATCH_COMPUTE(tc, TC, {
-    OFRR_TRY((hess_coop_t<TO, TC, false>(ctx, m, (int)n, (int)rows, G, smem, (TO*)Q, ldq, select_tol, R, select, perm,
-                                         done)));
+    OFRR_TRY((hess_coop_t<TO, TC>(ctx, m, (int)n, (int)rows, G, smem, (TO*)Q, ldq, select_tol, R, select, perm, done)));
   }));
   return OFRR_SUCCESS;
 }
