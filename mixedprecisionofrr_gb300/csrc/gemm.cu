@@ -122,30 +122,33 @@ int gram_f64(ofrr_ctx* ctx, int64_t M, int64_t N, int64_t K, const double* A, in
 // Rayleigh-Ritz step.  Q is a non-orthogonal basis and Z's columns cancel across it (|Q||z| is 10^3 ..
 // 10^4 times |Qz|), so the emulation's error is relative to a much larger number than the result; small
 // products (and every back-transform once a solve meets the emulation floor) run in FP64.  B in shared
-// memory, a thread per row and 16 columns, A read with coalesced loads.
-template <int CW>
+// memory, a thread per row and 8 columns, A read with coalesced loads.  A warp is a chain of K x columns FP64 instructions
+// of 64 cycles each: with 16 columns a thread a block of few rows leaves sub-partitions without a warp, and one of many
+// ends in a longer last wave (us, 16 / 8 columns: 4160 x 32 x 32 25.1 / 15.0, 5000 x 64 x 64 74.0 / 55.6, 40000 x 24 x 24
+// 68.1 / 49.5, 160000 x 64 x 64 1109 / 1121, where the FP64 pipe is full either way).
+constexpr int TSMM_CW = 8;
 __global__ void __launch_bounds__(128) k_tsmm_f64(int64_t M, int N, int K, const double* __restrict__ A, int64_t lda,
                                                   const double* __restrict__ B, int64_t ldb, double* __restrict__ C,
                                                   int64_t ldc) {
-  extern __shared__ double sBm[];  // K x CW slice of B (row-major)
-  const int c0 = blockIdx.y * CW, nc = min(CW, N - c0);
-  for (int e = threadIdx.x; e < K * CW; e += blockDim.x) {
-    const int k = e / CW, c = e % CW;
+  extern __shared__ double sBm[];  // K x TSMM_CW slice of B (row-major)
+  const int c0 = blockIdx.y * TSMM_CW, nc = min(TSMM_CW, N - c0);
+  for (int e = threadIdx.x; e < K * TSMM_CW; e += blockDim.x) {
+    const int k = e / TSMM_CW, c = e % TSMM_CW;
     sBm[e] = (c < nc) ? B[k + (int64_t)(c0 + c) * ldb] : 0.0;
   }
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (int64_t)gridDim.x * blockDim.x) {
-    double acc[CW];
+    double acc[TSMM_CW];
 #pragma unroll
-    for (int c = 0; c < CW; ++c) acc[c] = 0.0;
+    for (int c = 0; c < TSMM_CW; ++c) acc[c] = 0.0;
     for (int k = 0; k < K; ++k) {
       const double a = A[i + (int64_t)k * lda];
-      const double* b = sBm + k * CW;
+      const double* b = sBm + k * TSMM_CW;
 #pragma unroll
-      for (int c = 0; c < CW; ++c) acc[c] = fma(a, b[c], acc[c]);
+      for (int c = 0; c < TSMM_CW; ++c) acc[c] = fma(a, b[c], acc[c]);
     }
 #pragma unroll
-    for (int c = 0; c < CW; ++c)
+    for (int c = 0; c < TSMM_CW; ++c)
       if (c < nc) C[i + (int64_t)(c0 + c) * ldc] = acc[c];
   }
 }
@@ -153,15 +156,9 @@ __global__ void __launch_bounds__(128) k_tsmm_f64(int64_t M, int N, int K, const
 int tsmm_f64(ofrr_ctx* ctx, int64_t M, int64_t N, int64_t K, const double* A, int64_t lda, const double* B,
              int64_t ldb, double* C, int64_t ldc) {
   if (K > 256 || K < 1) return OFRR_ERR_BLAS_INVALID_SIZE;
-  // 16 columns a thread, 8 where that leaves sub-partitions without a warp: a warp is a chain of K x columns FP64
-  // instructions of 64 cycles each (4160 x 32 x 32: 15.9 us with 16, 10.3 us with 8)
-  const int64_t warps16 = ((M + 31) / 32) * ((N + 15) / 16);
-  const int cw = warps16 < 152 * 4 ? 8 : 16;
-  const dim3 grid((unsigned)std::min<int64_t>((M + 127) / 128, 152 * 8), (unsigned)((N + cw - 1) / cw));
-  const size_t smem = (size_t)K * cw * sizeof(double);
-  auto kernel = cw == 8 ? k_tsmm_f64<8> : k_tsmm_f64<16>;
-  if (smem > 48 * 1024) OFRR_TRY(allow_smem(kernel));
-  kernel<<<grid, 128, smem, ctx->stream>>>(M, (int)N, (int)K, A, lda, B, ldb, C, ldc);
+  const dim3 grid((unsigned)std::min<int64_t>((M + 127) / 128, 152 * 8), (unsigned)((N + TSMM_CW - 1) / TSMM_CW));
+  const size_t smem = (size_t)K * TSMM_CW * sizeof(double);  // at most 16 KB
+  k_tsmm_f64<<<grid, 128, smem, ctx->stream>>>(M, (int)N, (int)K, A, lda, B, ldb, C, ldc);
   OFRR_LAUNCHED(ctx, "k_tsmm_f64");
   return OFRR_SUCCESS;
 }
